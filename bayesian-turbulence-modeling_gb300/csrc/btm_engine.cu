@@ -304,6 +304,14 @@ template <class T> struct AmgDriver {
     }
 };
 
+// What the CG solvers take from the first squared residual norm: the norm,
+// whether there is nothing to solve, and the limit of their stopping test.
+__device__ __forceinline__ double cg_start(int lane, double rr, double tol) {
+    const double r0 = sqrt(rr);
+    const double limit = residual_limit(r0, tol);
+    return pick(lane, r0, flag64(r0 < 1e-30), limit);
+}
+
 // AMGSolver::solve (LinearSolver.hpp:602-653) with the reference's own
 // hierarchy rebuilt from this system (btm_ramg.cuh); one CTA.  r = I.r,
 // z = I.s (the V-cycle's level-0 x), p = I.pv, Ap = I.v, level-0 residual I.t.
@@ -321,10 +329,11 @@ __device__ __noinline__ SolveResult team_ramg_pcg(BlockTeamRef &tm, const DevMes
         I.s[c] = 0.0;
         a0[0] = fma(rc, rc, a0[0]);
     }
-    tm.template sum<1>(a0);
-    const double r0 = sqrt(a0[0]);
+    double o[3];
+    tm.template sum_then<1, 3>(a0, o, [tol](int lane, double rr, double) { return cg_start(lane, rr, tol); });
+    const double r0 = o[0], limit = o[2];
     res.initialRes = r0;
-    if (r0 < 1e-30) { res.converged = 1; return res; }
+    if (is_set(o[1])) { res.converged = 1; return res; }
     ramg_precondition(tm, M, I, nLev);
     double a1[1] = {0.0};
     for (int c = tm.rank(); c < nC; c += tm.size()) {
@@ -341,10 +350,11 @@ __device__ __noinline__ SolveResult team_ramg_pcg(BlockTeamRef &tm, const DevMes
             I.v[c] = ap;
             a2[0] = fma(I.pv[c], ap, a2[0]);
         }
-        tm.template sum<1>(a2);
-        const double pAp = a2[0];
-        if (fabs(pAp) < 1e-30) break;
-        const double alpha = rz / pAp;
+        tm.template sum_then<1, 2>(a2, o, [rz](int lane, double pAp, double) {
+            return pick(lane, flag64(fabs(pAp) < 1e-30), rz / pAp);
+        });
+        if (is_set(o[0])) break;
+        const double alpha = o[1];
         double a3[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             x[c] = x[c] + alpha * I.pv[c];
@@ -353,17 +363,17 @@ __device__ __noinline__ SolveResult team_ramg_pcg(BlockTeamRef &tm, const DevMes
             I.s[c] = 0.0;
             a3[0] = fma(rc, rc, a3[0]);
         }
-        tm.template sum<1>(a3);
-        const double rn = sqrt(a3[0]);
+        tm.template sum_then<1, 2>(a3, o, [=](int lane, double rr, double) {
+            return pick(lane, rr, flag64(residual_below(rr, limit, r0, tol)));
+        });
         res.iterations = it + 1;
-        res.finalRes = rn / r0;
-        if (res.finalRes < tol) { res.converged = 1; return res; }
+        res.finalSq = o[0];
+        if (is_set(o[1])) { res.converged = 1; return res; }
         ramg_precondition(tm, M, I, nLev);
         double a4[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) a4[0] = fma(I.r[c], I.s[c], a4[0]);
-        tm.template sum<1>(a4);
-        const double rzNew = a4[0];
-        const double beta = rzNew / (rz + 1e-30);
+        tm.template sum_then<1, 2>(a4, o, [rz](int lane, double t, double) { return pick(lane, t, t / (rz + 1e-30)); });
+        const double rzNew = o[0], beta = o[1];
         for (int c = tm.rank(); c < nC; c += tm.size()) I.pv[c] = I.s[c] + beta * I.pv[c];
         tm.sync();
         rz = rzNew;
@@ -404,10 +414,11 @@ __device__ __noinline__ SolveResult team_amg_pcg(T &tm, const DevMesh &M, DevIns
         I.s[c] = 0.0;
         a0[0] = fma(rc, rc, a0[0]);
     }
-    tm.template sum<1>(a0);
-    const double r0 = sqrt(a0[0]);
+    double o[3];
+    tm.template sum_then<1, 3>(a0, o, [tol](int lane, double rr, double) { return cg_start(lane, rr, tol); });
+    const double r0 = o[0], limit = o[2];
     res.initialRes = r0;
-    if (r0 < 1e-30) { res.converged = 1; return res; }
+    if (is_set(o[1])) { res.converged = 1; return res; }
     // The reference's breakdown guards (|p.Ap| < 1e-30, rz + 1e-30) are
     // absolute.  On grid meshes (above the one-CTA size) they are applied as
     // if the system had been scaled to a unit-norm right-hand side, as the
@@ -433,10 +444,11 @@ __device__ __noinline__ SolveResult team_amg_pcg(T &tm, const DevMesh &M, DevIns
             I.v[c] = ap;
             a2[0] = fma(LD(I.pv + c), ap, a2[0]);
         }
-        tm.template sum<1>(a2);
-        const double pAp = a2[0];
-        if (fabs(pAp) < guard) break;
-        const double alpha = rz / pAp;
+        tm.template sum_then<1, 2>(a2, o, [rz, guard](int lane, double pAp, double) {
+            return pick(lane, flag64(fabs(pAp) < guard), rz / pAp);
+        });
+        if (is_set(o[0])) break;
+        const double alpha = o[1];
         double a3[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             x[c] = fma(alpha, LD(I.pv + c), LD(x + c));
@@ -445,17 +457,19 @@ __device__ __noinline__ SolveResult team_amg_pcg(T &tm, const DevMesh &M, DevIns
             I.s[c] = 0.0;
             a3[0] = fma(rc, rc, a3[0]);
         }
-        tm.template sum<1>(a3);
-        const double rn = sqrt(a3[0]);
+        tm.template sum_then<1, 2>(a3, o, [=](int lane, double rr, double) {
+            return pick(lane, rr, flag64(residual_below(rr, limit, r0, tol)));
+        });
         res.iterations = it + 1;
-        res.finalRes = rn / r0;
-        if (res.finalRes < tol) { res.converged = 1; return res; }
+        res.finalSq = o[0];
+        if (is_set(o[1])) { res.converged = 1; return res; }
         AmgDriver<T>::vcycle(tm, M, I);
         double a4[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) a4[0] = fma(LD(I.r + c), LD(I.s + c), a4[0]);
-        tm.template sum<1>(a4);
-        const double rzNew = a4[0];
-        const double beta = rzNew / (rz + guard);
+        tm.template sum_then<1, 2>(a4, o, [rz, guard](int lane, double t, double) {
+            return pick(lane, t, t / (rz + guard));
+        });
+        const double rzNew = o[0], beta = o[1];
         for (int c = tm.rank(); c < nC; c += tm.size()) I.pv[c] = fma(beta, LD(I.pv + c), LD(I.s + c));
         tm.sync();
         rz = rzNew;
@@ -479,11 +493,15 @@ __device__ __noinline__ SolveResult team_pcg(T &tm, const DevMesh &M, DevInst &I
         a0[0] = fma(rc, rc, a0[0]);
         a0[1] = fma(rc, z, a0[1]);
     }
-    tm.template sum<2>(a0);
-    const double r0 = sqrt(a0[0]);
+    double o[4];
+    tm.template sum_then<2, 4>(a0, o, [tol](int lane, double rr, double t) {
+        const double start = cg_start(lane, rr, tol);
+        return lane == 3 ? t : start;
+    });
+    const double r0 = o[0], limit = o[2];
     res.initialRes = r0;
-    if (r0 < 1e-30) { res.converged = 1; return res; }
-    double rz = a0[1];
+    if (is_set(o[1])) { res.converged = 1; return res; }
+    double rz = o[3];
     for (int it = 0; it < maxIter; ++it) {
         if (!tm.ok()) break;
         double a2[1] = {0.0};
@@ -492,10 +510,11 @@ __device__ __noinline__ SolveResult team_pcg(T &tm, const DevMesh &M, DevInst &I
             I.v[c] = ap;
             a2[0] = fma(LD(I.pv + c), ap, a2[0]);
         }
-        tm.template sum<1>(a2);
-        const double pAp = a2[0];
-        if (fabs(pAp) < 1e-30) break;
-        const double alpha = rz / pAp;
+        tm.template sum_then<1, 2>(a2, o, [rz](int lane, double pAp, double) {
+            return pick(lane, flag64(fabs(pAp) < 1e-30), rz / pAp);
+        });
+        if (is_set(o[0])) break;
+        const double alpha = o[1];
         double a3[2] = {0.0, 0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             x[c] = fma(alpha, LD(I.pv + c), LD(x + c));
@@ -506,15 +525,17 @@ __device__ __noinline__ SolveResult team_pcg(T &tm, const DevMesh &M, DevInst &I
             a3[0] = fma(rc, rc, a3[0]);
             a3[1] = fma(rc, z, a3[1]);
         }
-        tm.template sum<2>(a3);
-        const double rn = sqrt(a3[0]);
+        tm.template sum_then<2, 4>(a3, o, [=](int lane, double rr, double t) {
+            const double beta = t / (rz + 1e-30);
+            return lane == 3 ? t : pick(lane, rr, flag64(residual_below(rr, limit, r0, tol)), beta);
+        });
         res.iterations = it + 1;
-        res.finalRes = rn / r0;
-        if (res.finalRes < tol) { res.converged = 1; return res; }
-        const double beta = a3[1] / (rz + 1e-30);
+        res.finalSq = o[0];
+        if (is_set(o[1])) { res.converged = 1; return res; }
+        const double beta = o[2];
         for (int c = tm.rank(); c < nC; c += tm.size()) I.pv[c] = fma(beta, LD(I.pv + c), LD(I.s + c));
         tm.sync();
-        rz = a3[1];
+        rz = o[3];
     }
     return res;
 }
@@ -565,8 +586,8 @@ __device__ __noinline__ SolveResult team_gauss_seidel(T &tm, const DevMesh &M, D
         }
         tm.template sum<1>(a1);
         res.iterations = it + 1;
-        res.finalRes = sqrt(a1[0]) / b0;
-        if (res.finalRes < tol) { res.converged = 1; return res; }
+        res.finalSq = a1[0];
+        if (sqrt(a1[0]) / b0 < tol) { res.converged = 1; return res; }
     }
     return res;
 }
@@ -707,6 +728,7 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
         clk.lap(6);
         // 5. k and omega
         SolveResult resK = {0, 0, 0, 0}, resW = {0, 0, 0, 0};
+        double change[4];   // largest k and omega, largest change of k and of omega
         if (turbUpdate) {
             for (int c = tm.rank(); c < nC; c += tm.size()) { I.kold[c] = LD(I.k + c); I.omold[c] = LD(I.om + c); }
             phase_turb_faces(tm, M, I, 0);
@@ -757,17 +779,14 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
                 mx[3] = smax(mx[3], fabs(omc - LD(I.omold + c)));
             }
             tm.template maxr<4>(mx);
-            lastKChange = mx[2] / mx[0];
-            lastOmChange = mx[3] / mx[1];
+            for (int q = 0; q < 4; ++q) change[q] = mx[q];
         }
         clk.lap(7);
-        // 6. residual bookkeeping and the convergence / divergence tests
+        // 6. residual bookkeeping and the convergence / divergence tests, by
+        // one warp (the quotients side by side in its lanes): lastKChange,
+        // lastOmChange, and how the iteration ends (0: on, 1: converged, 2: diverged)
         const double eUx = resU[0].initialRes, eUy = resU[1].initialRes, eUz = resU[2].initialRes;
         const double eP = resP.initialRes;
-        const double eK = turbActive ? lastKChange : 0.0, eW = turbActive ? lastOmChange : 0.0;
-        last[0] = eUx; last[1] = eUy; last[2] = eUz; last[3] = eP; last[4] = eK; last[5] = eW;
-        if (tm.leader() && I.hist && iter < I.histCap)
-            for (int q = 0; q < 6; ++q) I.hist[6 * (size_t)iter + q] = last[q];
         if (I.normFixed) {
             normUx0 = I.normIn[0];
             normUy0 = I.normIn[1];
@@ -779,22 +798,35 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
         } else if (iter < 50) {
             normP0 = smax(normP0, eP);
         }
-        const double normMom0 = smax(normUx0, normUy0);
-        const double nUx = normMom0 < 1e-20 ? 0.0 : eUx / normMom0;
-        const double nUy = normMom0 < 1e-20 ? 0.0 : eUy / normMom0;
-        const double nP = normP0 < 1e-20 ? 0.0 : eP / normP0;
-        double maxRes = smax(smax(nUx, nUy), nP);
-        if (turbActive) maxRes = smax(smax(maxRes, lastKChange), lastOmChange);
-        if (!isfinite(eUx) || !isfinite(eUy) || !isfinite(eUz) || !isfinite(eP) || !isfinite(eK) ||
-            !isfinite(eW) || !isfinite(lastKChange) || !isfinite(lastOmChange))
-            maxRes = INFINITY;
-        if (maxRes < S.convTol && iter > 0 && (!turbScheduled || (turbActive && turbEst))) {
-            converged = 1;
-            finalIter = iter;
-            break;
-        }
-        if (isnan(maxRes) || isinf(maxRes) || maxRes > S.divLimit) {
-            diverged = 1;
+        double end[3];
+        tm.template once<3>(end, [&](int lane) {
+            const double normMom0 = smax(normUx0, normUy0);
+            const double num = lane == 0 ? eUx : lane == 1 ? eUy : lane == 2 ? eP : change[lane == 3 ? 2 : 3];
+            const double den = lane < 2 ? normMom0 : lane == 2 ? normP0 : change[lane == 3 ? 0 : 1];
+            double q = num / den;
+            if (lane < 3 && den < 1e-20) q = 0.0;
+            const double nUx = __shfl_sync(0xffffffffu, q, 0), nUy = __shfl_sync(0xffffffffu, q, 1),
+                         nP = __shfl_sync(0xffffffffu, q, 2), qK = __shfl_sync(0xffffffffu, q, 3),
+                         qW = __shfl_sync(0xffffffffu, q, 4);
+            const double dK = turbUpdate ? qK : lastKChange, dW = turbUpdate ? qW : lastOmChange;
+            double maxRes = smax(smax(nUx, nUy), nP);
+            if (turbActive) maxRes = smax(smax(maxRes, dK), dW);
+            if (!isfinite(eUx) || !isfinite(eUy) || !isfinite(eUz) || !isfinite(eP) || !isfinite(dK) || !isfinite(dW))
+                maxRes = INFINITY;
+            double how = 0.0;
+            if (maxRes < S.convTol && iter > 0 && (!turbScheduled || (turbActive && turbEst))) how = 1.0;
+            else if (isnan(maxRes) || isinf(maxRes) || maxRes > S.divLimit) how = 2.0;
+            return pick(lane, dK, dW, how);
+        });
+        lastKChange = end[0];
+        lastOmChange = end[1];
+        const double eK = turbActive ? lastKChange : 0.0, eW = turbActive ? lastOmChange : 0.0;
+        last[0] = eUx; last[1] = eUy; last[2] = eUz; last[3] = eP; last[4] = eK; last[5] = eW;
+        if (tm.leader() && I.hist && iter < I.histCap)
+            for (int q = 0; q < 6; ++q) I.hist[6 * (size_t)iter + q] = last[q];
+        if (is_set(end[2])) {
+            converged = end[2] == 1.0;
+            diverged = !converged;
             finalIter = iter;
             break;
         }
@@ -843,7 +875,8 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
 // that two instances share an SM and hide each other's latency.
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block(DevInst *insts, int n) {
-    __shared__ double red[2 * 32 * kRedSlots];
+    __shared__ double red[NT > 2 * 32 * kRedSlots ? NT : 2 * 32 * kRedSlots];
+    __shared__ double tot[2 * (NT / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
     if (blockIdx.x >= n) return;
@@ -852,7 +885,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block(DevInst *insts, i
         sM = *sI.M;
     }
     __syncthreads();
-    BlockTeam tm{red, 0};
+    BlockTeam tm{red, 0, tot, 0};
     simple_solve(tm, sM, sI);
 }
 template __global__ void k_simple_block<256>(DevInst *, int);
@@ -862,7 +895,8 @@ template __global__ void k_simple_block<512>(DevInst *, int);
 // `xsCap` doubles of dynamic shared memory hold every level's x when they fit.
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block_ref(DevInst *insts, int n, int xsCap) {
-    __shared__ double red[2 * 32 * kRedSlots];
+    __shared__ double red[NT > 2 * 32 * kRedSlots ? NT : 2 * 32 * kRedSlots];
+    __shared__ double tot[2 * (NT / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
     extern __shared__ __align__(16) double xsm[];
@@ -876,6 +910,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block_ref(DevInst *inst
     BlockTeamRef tm;
     tm.red = red;
     tm.buf = 0;
+    tm.tot = tot;
+    tm.turn = 0;
     simple_solve(tm, sM, sI);
 }
 template __global__ void k_simple_block_ref<256>(DevInst *, int, int);
@@ -892,13 +928,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_simple_grid(DevInst *inst) {
         shAbort = 0;
     }
     __syncthreads();
-    GridTeam tm{red, 0, sI.gpart, sI.barrier, sI.err, &shAbort};
+    GridTeam tm{red, 0, sI.gpart, sI.barrier, sI.err, &shAbort, 0u};
     simple_solve(tm, sM, sI);
 }
 
 // Test hook: one phase on one CTA with the state already on the device.
 __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
-    __shared__ double red[2 * 32 * kRedSlots];
+    __shared__ double red[kThreads > 2 * 32 * kRedSlots ? kThreads : 2 * 32 * kRedSlots];
+    __shared__ double tot[2 * (kThreads / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
     if (threadIdx.x == 0) {
@@ -909,6 +946,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
     BlockTeamRef tm;
     tm.red = red;
     tm.buf = 0;
+    tm.tot = tot;
+    tm.turn = 0;
     const DevMesh &M = sM;
     DevInst &I = sI;
     const int ph = I.dbgPhase, arg = I.dbgArg;
@@ -967,7 +1006,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
     tm.sync();
     if (threadIdx.x == 0) {
         I.outLast[0] = res.iterations;
-        I.outLast[1] = res.finalRes;
+        I.outLast[1] = sqrt(res.finalSq) / (res.initialRes < 1e-30 ? 1.0 : res.initialRes);
         I.outLast[2] = res.initialRes;
         I.outLast[3] = res.converged;
     }

@@ -2100,7 +2100,8 @@ __device__ void stage_smem(DevMesh &M, DevInst &I, unsigned char *dsm, size_t ca
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_mixed_block(DevInst *insts, int n, int smemBytes) {
     extern __shared__ __align__(16) unsigned char dsm[];
-    __shared__ double red[2 * 32 * kRedSlots];
+    __shared__ double red[NT > 2 * 32 * kRedSlots ? NT : 2 * 32 * kRedSlots];
+    __shared__ double tot[2 * (NT / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
     __shared__ SmemCopy copies[4];
@@ -2120,7 +2121,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mixed_block(DevInst *insts, in
         for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     }
     __syncthreads();
-    BlockTeam tm{red, 0};
+    BlockTeam tm{red, 0, tot, 0};
     mixed_solve(tm, sM, sI);
 }
 template __global__ void k_mixed_block<256>(DevInst *, int, int);
@@ -2139,7 +2140,7 @@ __global__ void __launch_bounds__(kMixGridThreads, 1) k_mixed_grid(DevInst *inst
         shAbort = 0;
     }
     __syncthreads();
-    GridTeam tm{red, 0, sI.gpart, sI.barrier, sI.err, &shAbort};
+    GridTeam tm{red, 0, sI.gpart, sI.barrier, sI.err, &shAbort, 0u};
     mixed_solve(tm, sM, sI);
 }
 

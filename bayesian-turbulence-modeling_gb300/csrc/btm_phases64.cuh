@@ -597,34 +597,76 @@ __device__ __forceinline__ double gs_rd(double d) { return (fabs(d) > 1e-30) ? 1
 
 struct SolveResult {
     int iterations;
-    double finalRes, initialRes;
+    double finalSq, initialRes;   // squared residual norm at the end, norm at the start
     int converged;
 };
 
+// The stopping test of the Krylov solvers, sqrt(sq) / r0 < tol on the squared
+// residual norm sq, as sq < limit: both operations round monotonically, so
+// there is a smallest sq whose rounded quotient reaches tol.  It is found once
+// per solve by trying the 32 doubles around the real-valued limit in the lanes
+// of one warp, first for the division and then for the square root, which
+// takes an FP64 square root and a division (about 17 dependent FP64
+// instructions) out of every test with the same outcome.  Where the limit is
+// not bracketed (tolerances or norms at the ends of the range) `limit` is NaN
+// and the test divides.
+__device__ __forceinline__ double bits_step(double x, int ulps) {
+    return __longlong_as_double(__double_as_longlong(x) + ulps);
+}
+inline __device__ __noinline__ double residual_limit(double r0, double tol) {   // by a whole warp
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (tol <= 0.0) return 0.0;   // never below
+    const double t0 = r0 * tol;
+    if (!(t0 > 1e-140 && t0 < 1e140)) return NAN;
+    const unsigned reach = __ballot_sync(full, bits_step(t0, lane - 16) / r0 >= tol);
+    const int at = __ffs(reach) - 1;
+    if (at < 1) return NAN;
+    const double t = bits_step(t0, at - 16), s0 = t * t;
+    const unsigned reach2 = __ballot_sync(full, sqrt(bits_step(s0, lane - 16)) >= t);
+    const int at2 = __ffs(reach2) - 1;
+    return at2 < 1 ? (double)NAN : bits_step(s0, at2 - 16);
+}
+__device__ __forceinline__ bool residual_below(double sq, double limit, double r0, double tol) {
+    return isnan(limit) ? sqrt(sq) / r0 < tol : sq < limit;
+}
+__device__ __forceinline__ double pick(int lane, double a, double b) { return lane == 0 ? a : b; }
+__device__ __forceinline__ double pick(int lane, double a, double b, double c) { return lane == 2 ? c : pick(lane, a, b); }
+__device__ __forceinline__ double flag64(bool b) { return b ? 1.0 : 0.0; }
+// flags travel as 1.0 / 0.0; reading one is no FP64 operation
+__device__ __forceinline__ bool is_set(double f) { return __double2hiint(f) != 0; }
+
 // BiCGSTABSolver::solve (LinearSolver.hpp:191-247), right Jacobi preconditioned.
-// x is updated in place; A = (I.diag, I.upper, I.lower), b = I.src.
+// x is updated in place; A = (I.diag, I.upper, I.lower), b = I.src.  The
+// scalars of a step are formed by the warp that folds its dot products.
 template <class T>
 __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevInst &I, double *x, int maxIter, double tol) {
     SolveResult res = {0, 0.0, 0.0, 0};
     const int nC = M.nC;
-    double acc[2] = {0.0, 0.0};
+    double acc[1] = {0.0};
     for (int c = tm.rank(); c < nC; c += tm.size()) {
         double rc = LD(I.src + c) - ldu_row<T>(M, I, x, c);
         I.r[c] = rc; I.rh[c] = rc; I.pv[c] = 0.0; I.v[c] = 0.0;
         I.rd[c] = jac_rd(LD(I.diag + c));
         acc[0] = fma(rc, rc, acc[0]);
-        acc[1] = fma(rc, rc, acc[1]);
     }
-    tm.template sum<2>(acc);
-    const double r0 = sqrt(acc[0]);
+    double o[4];
+    // |r|^2 is also the first rho; with rho = alpha = omega = 1 before it, the
+    // first beta is rho itself
+    tm.template sum_then<1, 4>(acc, o, [tol](int lane, double rr, double) {
+        const double r0 = sqrt(rr);
+        const double limit = residual_limit(r0, tol);
+        return lane == 3 ? limit : pick(lane, rr, r0, flag64(r0 < 1e-30));
+    });
+    double rhoN = o[0];
+    const double r0 = o[1], limit = o[3];
     res.initialRes = r0;
-    if (r0 < 1e-30) { res.converged = 1; return res; }
-    double rhoN = acc[1];
-    double rho = 1, alpha = 1, omega = 1;
+    if (is_set(o[2])) { res.converged = 1; return res; }
+    double beta = rhoN, omega = 1.0;
+    bool small = fabs(rhoN) < 1e-30;
     for (int it = 0; it < maxIter; ++it) {
         if (!tm.ok()) break;
-        if (fabs(rhoN) < 1e-30) break;
-        const double beta = (rhoN / (rho + 1e-30)) * (alpha / (omega + 1e-30));
+        if (small) break;
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             double p = fma(beta, fma(-omega, LD(I.v + c), LD(I.pv + c)), LD(I.r + c));
             I.pv[c] = p;
@@ -637,10 +679,11 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
             I.v[c] = vc;
             a1[0] = fma(LD(I.rh + c), vc, a1[0]);
         }
-        tm.template sum<1>(a1);
-        const double rv = a1[0];
-        if (fabs(rv) < 1e-30) break;
-        alpha = rhoN / rv;
+        tm.template sum_then<1, 2>(a1, o, [rhoN](int lane, double rv, double) {
+            return pick(lane, flag64(fabs(rv) < 1e-30), rhoN / rv);
+        });
+        if (is_set(o[0])) break;
+        const double alpha = o[1];
         double a2[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             double sc = fma(-alpha, LD(I.v + c), LD(I.r + c));
@@ -648,11 +691,12 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
             I.sh[c] = sc * LD(I.rd + c);
             a2[0] = fma(sc, sc, a2[0]);
         }
-        tm.template sum<1>(a2);
-        const double sn = sqrt(a2[0]);
-        if (sn / r0 < tol) {
+        tm.template sum_then<1, 2>(a2, o, [=](int lane, double ss, double) {
+            return pick(lane, ss, flag64(residual_below(ss, limit, r0, tol)));
+        });
+        if (is_set(o[1])) {
             for (int c = tm.rank(); c < nC; c += tm.size()) x[c] = fma(alpha, LD(I.ph + c), LD(x + c));
-            res.iterations = it + 1; res.finalRes = sn / r0; res.converged = 1;
+            res.iterations = it + 1; res.finalSq = o[0]; res.converged = 1;
             tm.sync();
             return res;
         }
@@ -663,9 +707,8 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
             a3[0] = fma(tc, tc, a3[0]);
             a3[1] = fma(tc, LD(I.s + c), a3[1]);
         }
-        tm.template sum<2>(a3);
-        const double tt = a3[0];
-        omega = (tt > 1e-30) ? a3[1] / tt : 0.0;
+        tm.template sum_then<2, 1>(a3, o, [](int, double tt, double ts) { return (tt > 1e-30) ? ts / tt : 0.0; });
+        omega = o[0];
         double a4[2] = {0.0, 0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
             x[c] = LD(x + c) + fma(alpha, LD(I.ph + c), omega * LD(I.sh + c));
@@ -674,14 +717,22 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
             a4[0] = fma(rc, rc, a4[0]);
             a4[1] = fma(LD(I.rh + c), rc, a4[1]);
         }
-        tm.template sum<2>(a4);
-        const double rn = sqrt(a4[0]);
+        // how the iteration ends (0: on to the next, 1: converged, 2:
+        // breakdown), and the next beta = (rho' / rho) (alpha / omega): the two
+        // quotients side by side in two lanes
+        double e[4];
+        tm.template sum_then<2, 4>(a4, e, [=](int lane, double rr, double rho) {
+            const double end = residual_below(rr, limit, r0, tol) ? 1.0 : (fabs(omega) < 1e-30 ? 2.0 : 0.0);
+            const double q = pick(lane, rho, alpha) / (pick(lane, rhoN, omega) + 1e-30);
+            const double b = __shfl_sync(0xffffffffu, q, 0) * __shfl_sync(0xffffffffu, q, 1);
+            return lane == 3 ? end : pick(lane, rr, rho, b);
+        });
         res.iterations = it + 1;
-        res.finalRes = rn / r0;
-        if (res.finalRes < tol) { res.converged = 1; return res; }
-        if (fabs(omega) < 1e-30) break;
-        rho = rhoN;
-        rhoN = a4[1];
+        res.finalSq = e[0];
+        if (is_set(e[3])) { res.converged = e[3] == 1.0; return res; }
+        rhoN = e[1];
+        beta = e[2];
+        small = fabs(rhoN) < 1e-30;
     }
     return res;
 }

@@ -27,57 +27,136 @@ constexpr uint64_t kBarrierTimeoutNs = 2000000000ull;  // 2 s: a stuck barrier a
 // ---------------------------------------------------------------------------
 // teams
 // ---------------------------------------------------------------------------
+// FP64 reductions over one CTA.  A GB300 SM sub-partition (SMSP) holds its
+// FP64 unit for 64 clocks per warp instruction, whatever the number of active
+// lanes and however independent the instructions are (measured: 63.9 clocks
+// per dependent and per independent addition of one warp, 152 with two warps
+// on the SMSP).  What a reduction costs is therefore its FP64 warp
+// instructions, and a butterfly in every warp followed by a fold of all warp
+// partials in every thread spends most of them on copies of the same sums.
+// Here every warp does only the first step of its butterfly (two values at
+// once: each half of the lanes goes on with one of them) and leaves the 16
+// sums of each value in shared memory; half of the warps finish two source
+// warps each (16 lanes per source, later 8 per value: no addition is done
+// twice), and one warp adds the per-warp totals in warp order.  The additions,
+// their pairing and their order are those of the butterfly and the fold, so
+// the totals are the same bits.
+//
+// Shared memory: `red` [threads] doubles, shared with the FP32 reductions
+// (hence the barrier in front), and `tot` [2][warps] + 2: totals, result.
+struct RedAdd {
+    __device__ __forceinline__ static double op(double a, double b) { return a + b; }
+    __device__ __forceinline__ static double first(const double *) { return 0.0; }
+};
+struct RedMax {   // smax: the first operand survives ties and NaN
+    __device__ __forceinline__ static double op(double a, double b) { return smax(a, b); }
+    __device__ __forceinline__ static double first(const double *p) { return __ldcg(p); }
+};
+
+//
+// The folding warp goes on to `f(lane, t0, t1)`, the scalars that follow from
+// the totals (all its lanes call it; lane q < NOUT leaves result q): a
+// division costs 8 to 9 FP64 instructions, and formed in every warp of the
+// CTA they took as long as the matrix products of a BiCGSTAB iteration.
+constexpr int kRedResults = 6;
+template <int N, class Op, int NOUT, class F>
+__device__ __forceinline__ void block_reduce(double *red, double *tot, double *v, int turn, double *out, F f) {
+    static_assert((N == 1 || N == 2) && NOUT <= kRedResults, "one or two values at a time");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    double *res = tot + 2 * nw;
+    double h;
+    if (N == 2) {
+        const bool second = lane >= 16;
+        const double got = __shfl_xor_sync(0xffffffffu, second ? v[0] : v[1], 16);
+        h = second ? Op::op(got, v[1]) : Op::op(v[0], got);
+    } else {
+        h = Op::op(v[0], __shfl_xor_sync(0xffffffffu, v[0], 16));
+    }
+    __syncthreads();
+    if (N == 2 || lane < 16) red[warp * (16 * N) + lane] = h;   // [warp][value][16]
+    __syncthreads();
+    if (2 * warp < nw) {
+        const int src = 2 * warp + (lane >> 4), l = lane & 15;
+        double x;
+        if (N == 2) {
+            // lanes 0-7 of a source take the first value, 8-15 the second
+            const double *e = red + src * 32 + (l >> 3) * 16 + (l & 7);
+            x = Op::op(e[0], e[8]);
+        } else {
+            const double own = red[src * 16 + l];
+            x = Op::op(own, __shfl_xor_sync(0xffffffffu, own, 8));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) x = Op::op(x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (l == 0) tot[src] = x;
+        if (N == 2 && l == 8) tot[nw + src] = x;
+        // the folding warp (another one each time: a warp stays on its SMSP)
+        // waits for the totals, the other warps for the result only
+        asm volatile("bar.sync 1, %0;" ::"r"(nw << 4) : "memory");
+        if (warp == (turn & 3)) {
+            const double *t = tot + (lane < N ? lane * nw : 0);
+            double s = t[0];
+            for (int q = 1; q < nw; ++q) s = Op::op(s, t[q]);
+            const double t0 = __shfl_sync(0xffffffffu, s, 0), t1 = N == 2 ? __shfl_sync(0xffffffffu, s, 1) : 0.0;
+            const double r = f(lane, t0, t1);
+            if (lane < NOUT) res[lane] = r;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NOUT; ++j) out[j] = res[j];
+}
+template <int N, class Op>
+__device__ __noinline__ void block_totals(double *red, double *tot, double *v, int turn) {
+    block_reduce<N, Op, N>(red, tot, v, turn, v, [](int lane, double t0, double t1) { return lane == 0 ? t0 : t1; });
+}
+
+
 struct BlockTeam {
-    double *red;   // shared [2][32][kRedSlots]
+    double *red;   // shared [max(threads, 2 * 32 * kRedSlots)]
     int buf;
+    double *tot;   // shared [2 * warps + kRedResults]
+    int turn;
     __device__ __forceinline__ int rank() const { return threadIdx.x; }
     __device__ __forceinline__ int size() const { return blockDim.x; }
     __device__ __forceinline__ bool leader() const { return threadIdx.x == 0; }
     __device__ __forceinline__ bool sync() { __syncthreads(); return true; }
     __device__ __forceinline__ bool ok() const { return true; }
 
+    template <int N, class Op>
+    __device__ __forceinline__ void reduce(double *v) {
+        if constexpr (N > 2) {
+            reduce<2, Op>(v);
+            reduce<N - 2, Op>(v + 2);
+        } else {
+            block_totals<N, Op>(red, tot, v, turn++);
+        }
+    }
     // Sum N values over the team; every thread receives the identical totals.
     template <int N>
-    __device__ __forceinline__ void sum(double *v) {
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *rb = red + buf * 32 * kRedSlots;
-        if (lane == 0)
-#pragma unroll
-            for (int j = 0; j < N; ++j) rb[warp * kRedSlots + j] = v[j];
-        __syncthreads();
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            double s = 0.0;
-            for (int q = 0; q < nw; ++q) s += rb[q * kRedSlots + j];
-            v[j] = s;
-        }
-        buf ^= 1;
-    }
+    __device__ __forceinline__ void sum(double *v) { reduce<N, RedAdd>(v); }
     template <int N>
-    __device__ __forceinline__ void maxr(double *v) {
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[j] = smax(v[j], __shfl_xor_sync(0xffffffffu, v[j], o));
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *rb = red + buf * 32 * kRedSlots;
-        if (lane == 0)
-#pragma unroll
-            for (int j = 0; j < N; ++j) rb[warp * kRedSlots + j] = v[j];
+    __device__ __forceinline__ void maxr(double *v) { reduce<N, RedMax>(v); }
+    template <int N>
+    __device__ __forceinline__ void sumd(double *v) { reduce<N, RedAdd>(v); }
+    // Sums N values and leaves f(q, t0, t1) of the totals in out[q], q < NOUT,
+    // in every thread; one warp evaluates f.
+    template <int N, int NOUT, class F>
+    __device__ __forceinline__ void sum_then(double *v, double *out, F f) {
+        block_reduce<N, RedAdd, NOUT>(red, tot, v, turn++, out, f);
+    }
+    // The same for warp 0's values f(lane) that need no reduction
+    template <int NOUT, class F>
+    __device__ __forceinline__ void once(double *out, F f) {
+        double *res = tot + 2 * (blockDim.x >> 5);
         __syncthreads();
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            double s = rb[j];
-            for (int q = 1; q < nw; ++q) s = smax(s, rb[q * kRedSlots + j]);
-            v[j] = s;
+        if (threadIdx.x < 32) {
+            const double r = f((int)threadIdx.x);
+            if (threadIdx.x < NOUT) res[threadIdx.x] = r;
         }
-        buf ^= 1;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < NOUT; ++j) out[j] = res[j];
     }
 
     // FP32 sums (Krylov dot products of the mixed-precision engine): a warp
@@ -106,30 +185,6 @@ struct BlockTeam {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             v[j] = s;
-        }
-        buf ^= 1;
-    }
-    // FP64 sums folded across warps by lane 0 only (same totals as sum<N>
-    // would give in every thread, with FP64 work per warp instead of per thread)
-    template <int N>
-    __device__ __forceinline__ void sumd(double *v) {
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *rb = red + buf * 32 * kRedSlots;
-        if (lane == 0)
-#pragma unroll
-            for (int j = 0; j < N; ++j) rb[warp * kRedSlots + j] = v[j];
-        __syncthreads();
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            double s = 0.0;
-            if (lane == 0)
-                for (int q = 0; q < nw; ++q) s += rb[q * kRedSlots + j];
-            v[j] = __shfl_sync(0xffffffffu, s, 0);
         }
         buf ^= 1;
     }
@@ -167,81 +222,131 @@ struct GridTeam {
     double *red;            // shared [2][32][kRedSlots]
     int buf;
     double *gpart;          // global [2][gridDim][kRedSlots]
-    unsigned int *bar;      // [0] arrivals, [1] generation
+    unsigned int *bar;      // arrivals since the launch (zeroed before it)
     int32_t *err;
     int *shAbort;           // shared flag
+    unsigned int target;    // thread 0: arrivals that complete the next barrier
     __device__ __forceinline__ int rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
     __device__ __forceinline__ int size() const { return gridDim.x * blockDim.x; }
     __device__ __forceinline__ bool leader() const { return blockIdx.x == 0 && threadIdx.x == 0; }
     __device__ __forceinline__ bool ok() const { return *shAbort == 0; }
 
-    // Software grid barrier for a cooperative launch (all CTAs co-resident).
-    // Every wait is bounded: after kBarrierTimeoutNs the CTA flags the error
-    // and the whole team abandons the solve.
-    __device__ bool sync() {
+    // Software grid barrier for a cooperative launch (all CTAs co-resident):
+    // one release arrival per CTA on a counter that only grows, acquire polls
+    // of that counter (its wrap-around is harmless: the difference to the
+    // target is what counts).  A barrier is nothing but latency, one L2
+    // round trip for the arrival and one for the poll that sees the last; a
+    // clock read, a nanosleep or a second flag in every poll adds its own.
+    // Every wait is bounded: each kPollsPerCheck polls the CTA looks at the
+    // error flag and the clock, and after kBarrierTimeoutNs it flags the error
+    // and the whole team abandons the solve.  A CTA that has abandoned it no
+    // longer arrives.
+    __device__ __noinline__ bool sync() {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            volatile unsigned int *vgen = bar + 1;
-            unsigned int gen = *vgen;
-            __threadfence();
-            unsigned int arrived = atomicAdd(bar, 1u);
-            if (arrived == gridDim.x - 1) {
-                atomicExch(bar, 0u);
-                __threadfence();
-                atomicAdd(bar + 1, 1u);
-            } else {
-                uint64_t t0 = globaltimer_ns();
-                while (*vgen == gen) {
+        if (threadIdx.x == 0 && *shAbort == 0) {
+            target += gridDim.x;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+            uint64_t t0 = 0;
+            for (unsigned int polls = 1;; ++polls) {
+                unsigned int now;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
+                if ((int)(now - target) >= 0) break;
+                if ((polls & (kPollsPerCheck - 1)) == 0) {
                     if (*(volatile int32_t *)err) { *shAbort = 1; break; }
-                    if (globaltimer_ns() - t0 > kBarrierTimeoutNs) {
+                    const uint64_t t = globaltimer_ns();
+                    if (t0 == 0) {
+                        t0 = t;
+                    } else if (t - t0 > kBarrierTimeoutNs) {
                         atomicExch(err, 2);
                         *shAbort = 1;
                         break;
                     }
-                    __nanosleep(20);
                 }
             }
-            __threadfence();
-            if (*(volatile int32_t *)err) *shAbort = 1;
         }
         __syncthreads();
         return *shAbort == 0;
     }
+    static constexpr unsigned int kPollsPerCheck = 256;
 
+    // Totals of N values whose per-warp totals are in rb[warp][value] (shared,
+    // visible after the first barrier here): warp 0 adds them in warp order,
+    // lane j the j-th value; after the grid barrier warp j folds the CTAs'
+    // partials of value j (each lane a fixed strided subset, then a
+    // butterfly) for its CTA.  The order of the operations is that of a fold
+    // in every thread; one warp does them, because an FP64 warp instruction
+    // holds its SMSP for 64 clocks.
+    template <int N, class Op, int NOUT, class F>
+    __device__ __forceinline__ void fold_then(double *out, F f) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double *rb = red + buf * 32 * kRedSlots;
+        __syncthreads();
+        if (warp == 0 && lane < N) {
+            const int nw = blockDim.x >> 5;
+            double s = rb[lane];
+            for (int q = 1; q < nw; ++q) s = Op::op(s, rb[q * kRedSlots + lane]);
+            gpart[((size_t)buf * gridDim.x + blockIdx.x) * kRedSlots + lane] = s;
+        }
+        sync();
+        double *tot = rb + 31 * kRedSlots, *res = rb + 29 * kRedSlots;
+        if (warp < N) {
+            const double *gp = gpart + (size_t)buf * gridDim.x * kRedSlots + warp;
+            double s = Op::first(gp);
+            for (int q = lane; q < (int)gridDim.x; q += 32) s = Op::op(s, __ldcg(gp + (size_t)q * kRedSlots));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s = Op::op(s, __shfl_xor_sync(0xffffffffu, s, o));
+            if (lane == 0) tot[warp] = s;
+        }
+        if (N > 1) __syncthreads();
+        if (warp == 0) {
+            __syncwarp();
+            const double r = f(lane, tot[0], N > 1 ? tot[1] : 0.0);
+            if (lane < NOUT) res[lane] = r;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < NOUT; ++j) out[j] = res[j];
+        buf ^= 1;
+    }
+    template <int N, class Op>
+    __device__ __noinline__ void fold(double *v) {
+        fold_then<N, Op, N>(v, [this](int lane, double, double) {
+            return red[buf * 32 * kRedSlots + 31 * kRedSlots + (lane < N ? lane : 0)];
+        });
+    }
+    // warp totals of N values into rb[warp][value]
     template <int N>
-    __device__ void sum(double *v) {
+    __device__ __forceinline__ void leave(double *v) {
 #pragma unroll
         for (int j = 0; j < N; ++j)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *rb = red + buf * 32 * kRedSlots;
-        if (lane == 0)
+        if ((threadIdx.x & 31) == 0)
 #pragma unroll
-            for (int j = 0; j < N; ++j) rb[warp * kRedSlots + j] = v[j];
+            for (int j = 0; j < N; ++j) red[buf * 32 * kRedSlots + (threadIdx.x >> 5) * kRedSlots + j] = v[j];
+    }
+    template <int N, int NOUT, class F>
+    __device__ __forceinline__ void sum_then(double *v, double *out, F f) {
+        leave<N>(v);
+        fold_then<N, RedAdd, NOUT>(out, f);
+    }
+    template <int NOUT, class F>
+    __device__ __forceinline__ void once(double *out, F f) {
+        double *res = red + buf * 32 * kRedSlots + 29 * kRedSlots;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const int nw = blockDim.x >> 5;
-            double *gp = gpart + ((size_t)buf * gridDim.x + blockIdx.x) * kRedSlots;
-            for (int j = 0; j < N; ++j) {
-                double s = 0.0;
-                for (int q = 0; q < nw; ++q) s += rb[q * kRedSlots + j];
-                gp[j] = s;
-            }
+        if (threadIdx.x < 32) {
+            const double r = f((int)threadIdx.x);
+            if (threadIdx.x < NOUT) res[threadIdx.x] = r;
         }
-        sync();
-        // each lane folds a fixed strided subset of the CTA partials, then a
-        // butterfly: identical totals in every thread of every CTA
-        const double *gp = gpart + (size_t)buf * gridDim.x * kRedSlots;
+        __syncthreads();
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-            double s = 0.0;
-            for (int q = lane; q < (int)gridDim.x; q += 32) s += __ldcg(gp + q * kRedSlots + j);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            v[j] = s;
-        }
+        for (int j = 0; j < NOUT; ++j) out[j] = res[j];
         buf ^= 1;
+    }
+    template <int N>
+    __device__ void sum(double *v) {
+        leave<N>(v);
+        fold<N, RedAdd>(v);
     }
     template <int N>
     __device__ void maxr(double *v) {
@@ -249,49 +354,23 @@ struct GridTeam {
         for (int j = 0; j < N; ++j)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[j] = smax(v[j], __shfl_xor_sync(0xffffffffu, v[j], o));
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *rb = red + buf * 32 * kRedSlots;
-        if (lane == 0)
+        if ((threadIdx.x & 31) == 0)
 #pragma unroll
-            for (int j = 0; j < N; ++j) rb[warp * kRedSlots + j] = v[j];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const int nw = blockDim.x >> 5;
-            double *gp = gpart + ((size_t)buf * gridDim.x + blockIdx.x) * kRedSlots;
-            for (int j = 0; j < N; ++j) {
-                double s = rb[j];
-                for (int q = 1; q < nw; ++q) s = smax(s, rb[q * kRedSlots + j]);
-                gp[j] = s;
-            }
-        }
-        sync();
-        const double *gp = gpart + (size_t)buf * gridDim.x * kRedSlots;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            double s = __ldcg(gp + j);
-            for (int q = lane; q < (int)gridDim.x; q += 32) s = smax(s, __ldcg(gp + q * kRedSlots + j));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s = smax(s, __shfl_xor_sync(0xffffffffu, s, o));
-            v[j] = s;
-        }
-        buf ^= 1;
+            for (int j = 0; j < N; ++j) red[buf * 32 * kRedSlots + (threadIdx.x >> 5) * kRedSlots + j] = v[j];
+        fold<N, RedMax>(v);
     }
-    // FP32 values, FP64 accumulation from the warp level up (see BlockTeam::sumf)
+    // FP32 values, FP64 accumulation from the warp totals up
     template <int N>
     __device__ void sumf(float *v) {
-        double d[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
+        for (int j = 0; j < N; ++j)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-            d[j] = (double)v[j];
-        }
-        // the warp-level totals enter the FP64 grid reduction as lane-0 values
-        const int lane = threadIdx.x & 31;
-        if (lane != 0)
+        if ((threadIdx.x & 31) == 0)
 #pragma unroll
-            for (int j = 0; j < N; ++j) d[j] = 0.0;
-        sum<N>(d);
+            for (int j = 0; j < N; ++j) red[buf * 32 * kRedSlots + (threadIdx.x >> 5) * kRedSlots + j] = (double)v[j];
+        double d[N];
+        fold<N, RedAdd>(d);
 #pragma unroll
         for (int j = 0; j < N; ++j) v[j] = (float)d[j];
     }
@@ -299,10 +378,15 @@ struct GridTeam {
     __device__ void sumd(double *v) { sum<N>(v); }
     template <int N>
     __device__ void maxf(float *v) {
-        double d[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) d[j] = (double)v[j];
-        maxr<N>(d);
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[j] = smaxf(v[j], __shfl_xor_sync(0xffffffffu, v[j], o));
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+            for (int j = 0; j < N; ++j) red[buf * 32 * kRedSlots + (threadIdx.x >> 5) * kRedSlots + j] = (double)v[j];
+        double d[N];
+        fold<N, RedMax>(d);
 #pragma unroll
         for (int j = 0; j < N; ++j) v[j] = (float)d[j];
     }
