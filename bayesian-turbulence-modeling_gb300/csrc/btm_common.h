@@ -15,6 +15,7 @@ constexpr int kCoarseDirect = 32;    // coarsest level at or below this size: de
 // cap at ~530 rows), and each level costs the V-cycle ~27 dependent phases on
 // one CTA, while a dense inverse of this size is one grid-wide mat-vec.
 constexpr int kCoarseDirectGrid = 1024;
+constexpr int kPanel = 16;           // pivots per pass of the grid's dense inverse (btm_dense.cuh)
 constexpr int kCoarseSweeps = 50;    // GS sweeps when the coarsest level is larger
 constexpr int kRedSlots = 4;         // values per fused team reduction
 constexpr int kAndersonMax = 8;      // stored differences of the Anderson acceleration (BTM_ANDERSON_MAX)
@@ -138,6 +139,11 @@ struct DevMesh {
     const int32_t *cfOff;      // [nC+1] internal-face gather list, ascending face index
     const int32_t *cfFace;     // face index
     const int32_t *cfOther;    // other cell, negated-1 when this cell is the neighbour: other = -(x+1)
+    // the same lists by position in the list, [rowW][nC] (rowW =
+    // max(maxCellFaces, 1)): entry id of the matrix coefficient in
+    // diag | upper | lower and the other cell; -1 in rowCol past a list's end
+    int32_t rowW;
+    const int32_t *rowEnt, *rowCol;
     const int32_t *cbOff;      // [nC+1] boundary faces, ascending face index (b indices)
     const int32_t *cbFace;
     const int32_t *cbpOff;     // [nC+1] boundary faces in patch iteration order
@@ -275,7 +281,7 @@ int engine_launch_debug(DevInst *dInst, void *stream);
 int engine_wall_distance(const double *dCentres, int nC, const double *dWall, int nW, double *dOut, void *stream);
 
 // mixed-precision engine entry points (btm_mixed.cu)
-size_t mixed_smem_bytes(int nC, int nIF, int64_t vecTotal, int64_t valTotal, int coarseN, int band);
+size_t mixed_smem_bytes(int nC, int nIF, int64_t vecTotal, int64_t valTotal, int coarseN, int band, int rowW);
 int mixed_launch_block(DevInst *dInsts, int n, int threads, size_t smemBytes, void *stream);
 int mixed_grid_blocks(int *blocks_out);
 int mixed_launch_grid(DevInst *dInst, int blocks, void *stream);

@@ -23,6 +23,7 @@
 #include "btm_phases64.cuh"
 #include "btm_observe.cuh"
 #include "btm_ramg.cuh"
+#include "btm_dense.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -76,11 +77,12 @@ __device__ void amg_level_rd(T &tm, const DevMesh &M, DevInst &I, int l) {
     }
 }
 
-// dense inverse of the coarsest level by Gauss-Jordan with ping-pong buffers;
-// one reciprocal per pivot, no pivoting (the level matrix is SPD: Galerkin
-// product of the pinned / Dirichlet-bounded pressure Laplacian)
+// Dense inverse of the coarsest level (Galerkin product of the pinned /
+// Dirichlet-bounded pressure Laplacian: SPD).  A matrix with a vanishing pivot
+// is no such product; its rows are passed over one by one, which needs the
+// sweep over all 2n columns with ping-pong buffers.
 template <class T>
-__device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst &I) {
+__device__ __noinline__ void amg_coarse_inverse_sweep(T &tm, const DevMesh &M, DevInst &I) {
     const int l = M.nLevels - 1;
     const AmgLevelDev &L = M.lev[l];
     const int n = L.n, w2 = 2 * n;
@@ -126,6 +128,34 @@ __device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst
     tm.sync();
 }
 
+template <class T>
+__device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst &I) {
+    const int l = M.nLevels - 1, n = M.lev[l].n;
+    const AmgLevelDev &L = M.lev[l];
+    double *A = I.ainv;
+    const double *val = lev_vals(I, M, l);
+    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
+    tm.sync();
+    for (int i = tm.rank(); i < n; i += tm.size()) {
+        double *row = A + (size_t)i * n;
+        if (l == 0) {
+            row[i] = LD(I.diag + i);  // level 0 as coarsest: LDU rows
+            for (int e = M.cfOff[i]; e < M.cfOff[i + 1]; ++e) {
+                const int f = M.cfFace[e], oth = M.cfOther[e];
+                if (oth >= 0) row[oth] = LD(I.upper + f);
+                else row[-(oth + 1)] = LD(I.lower + f);
+            }
+        } else {
+            for (int q = L.rowPtr[i]; q < L.rowPtr[i + 1]; ++q) row[L.colIdx[q]] = LD(val + q);
+        }
+    }
+    tm.sync();
+    if (!dense_inverse(tm, A, I.gj, n)) {
+        tm.sync();
+        amg_coarse_inverse_sweep(tm, M, I);
+    }
+}
+
 // one colour-ordered Gauss-Seidel sweep (forward or reverse colour order)
 template <class T>
 __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
@@ -141,18 +171,8 @@ __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, i
             const double ri = LD(rd + i);
             if (ri == 0.0) continue;
             double s = LD(b + i);
-            if (l == 0) {
-                for (int e = M.cfOff[i]; e < M.cfOff[i + 1]; ++e) {
-                    const int f = M.cfFace[e], oth = M.cfOther[e];
-                    if (oth >= 0) s = fma(-LD(I.upper + f), LD(x + oth), s);
-                    else s = fma(-LD(I.lower + f), LD(x + (-(oth + 1))), s);
-                }
-            } else {
-                for (int q2 = L.rowPtr[i]; q2 < L.rowPtr[i + 1]; ++q2) {
-                    const int j = L.colIdx[q2];
-                    if (j != i) s = fma(-LD(val + q2), LD(x + j), s);
-                }
-            }
+            if (l == 0) s = ldu_off<T, true>(M, I.diag, x, i, s);
+            else s = csr_off<T, true>(L, val, x, i, i, s);
             x[i] = s * ri;
         }
         tm.sync();
@@ -170,8 +190,7 @@ __device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, i
         if (l == 0) {
             s = ldu_row<T>(M, I, x, i);
         } else {
-            s = 0.0;
-            for (int q = L.rowPtr[i]; q < L.rowPtr[i + 1]; ++q) s = fma(LD(val + q), LD(x + L.colIdx[q]), s);
+            s = csr_off<T, false>(L, val, x, i, -1, 0.0);
         }
         r[i] = LD(b + i) - s;
     }
@@ -242,8 +261,7 @@ __device__ __noinline__ void amg_jacobi(T &tm, const DevMesh &M, DevInst &I, int
     const AmgLevelDev &L = M.lev[l];
     const double *b = lev_b(I, M, l), *val = lev_vals(I, M, l), *rd = lev_rd(I, M, l);
     for (int i = tm.rank(); i < L.n; i += tm.size()) {
-        double s = LD(b + i);
-        for (int q = L.rowPtr[i]; q < L.rowPtr[i + 1]; ++q) s = fma(-LD(val + q), LD(x + L.colIdx[q]), s);
+        const double s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
         out[i] = fma(kJacobiWeight64 * LD(rd + i), s, LD(x + i));
     }
     tm.sync();

@@ -497,6 +497,15 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
             }
     }
     D.maxCellFaces = maxCF;
+    D.rowW = std::max(maxCF, 1);
+    std::vector<int> rowEnt((size_t)D.rowW * nC, 0), rowCol((size_t)D.rowW * nC, -1);
+    for (int c = 0; c < nC; ++c)
+        for (int e = cfOff[c]; e < cfOff[c + 1]; ++e) {
+            const size_t at = (size_t)(e - cfOff[c]) * nC + c;
+            const int f = cfFace[e], oth = cfOther[e];
+            rowEnt[at] = oth >= 0 ? nC + f : nC + nIF + f;
+            rowCol[at] = oth >= 0 ? oth : -(oth + 1);
+        }
 
     // ---- pressure AMG hierarchy on the geometric Laplacian ----------------
     std::vector<HLevel> lv(1);
@@ -609,6 +618,8 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
     inRange(cfFace, 0, std::max(nIF, 1), "cfFace");
     for (int x : cfOther)
         if (!((x >= 0 && x < nC) || (x < 0 && -(x + 1) < nC))) throw BtmError(BTM_ERR_INTERNAL, "cfOther");
+    inRange(rowEnt, 0, nC + 2 * nIF, "rowEnt");
+    inRange(rowCol, -1, nC, "rowCol");
     if (cbOff[nC] > 0) inRange(std::vector<int>(cbFace.begin(), cbFace.begin() + cbOff[nC]), 0, nB, "cbFace");
     if (cbpOff[nC] > 0) inRange(std::vector<int>(cbpFace.begin(), cbpFace.begin() + cbpOff[nC]), 0, nB, "cbpFace");
     inRange(pin, -1, std::max(nB, 1), "pinFace");
@@ -648,7 +659,8 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
            o_bvUy = P(bvUy), o_bvUz = P(bvUz), o_bvP = P(bvP), o_bvK = P(bvK), o_bvW = P(bvW);
     std::vector<double> vol(m->cell_volume, m->cell_volume + nC), wd(m->wall_distance, m->wall_distance + nC);
     size_t o_vol = P(vol), o_wd = P(wd), o_cfOff = P(cfOff), o_cfFace = P(cfFace), o_cfOther = P(cfOther),
-           o_cbOff = P(cbOff), o_cbFace = P(cbFace), o_cbpOff = P(cbpOff), o_cbpFace = P(cbpFace), o_pin = P(pin);
+           o_cbOff = P(cbOff), o_cbFace = P(cbFace), o_cbpOff = P(cbpOff), o_cbpFace = P(cbpFace), o_pin = P(pin),
+           o_rowEnt = P(rowEnt), o_rowCol = P(rowCol);
     // FP32 geometry for the mixed-precision engine; reciprocals are formed in
     // FP64 and rounded once
     auto f32 = [](const std::vector<double> &v) { return std::vector<float>(v.begin(), v.end()); };
@@ -706,6 +718,7 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
     D.vol = F64(o_vol); D.wd = F64(o_wd); D.cfOff = I32(o_cfOff); D.cfFace = I32(o_cfFace); D.cfOther = I32(o_cfOther);
     D.cbOff = I32(o_cbOff); D.cbFace = I32(o_cbFace); D.cbpOff = I32(o_cbpOff); D.cbpFace = I32(o_cbpFace);
     D.pinFace = I32(o_pin);
+    D.rowEnt = I32(o_rowEnt); D.rowCol = I32(o_rowCol);
     D.aOverD = F64(o_aod);
     D.r0Ent = I32(o_r0Ent);
     D.wf0Off = I32(o_wf0Off);
@@ -728,6 +741,10 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
     ck(cudaMemcpy(C->dMeshPtr, &D, sizeof D, cudaMemcpyHostToDevice), "cudaMemcpy(DevMesh)");
 }
 
+// Work of the coarsest level's inverse: the ping-pong buffers of the sweep
+// over 2n columns, or a panel's multipliers and pivot rows.
+size_t gj_doubles(int nc) { return std::max((size_t)4 * nc * nc, (size_t)2 * btm::kPanel * nc); }
+
 // Carve one instance slab (fields + work + AMG + control words).
 void make_slab(btm_case *C, Slab &S) {
     const int nC = C->nC, nIF = C->nIF, nB = C->nB;
@@ -741,7 +758,7 @@ void make_slab(btm_case *C, Slab &S) {
     doubles += face;                          // fflux
     doubles += 7 * bnd;                       // boundary arrays
     doubles += up(C->amgValTotal) + 3 * up(C->amgVecTotal) + up(nC + C->amgVecTotal);
-    doubles += up((size_t)nc * nc) + up((size_t)4 * nc * nc);
+    doubles += up((size_t)nc * nc) + up(gj_doubles(nc));
     int gridBlocks = C->maxGridBlocks > 0 ? C->maxGridBlocks : 1024;
     doubles += up((size_t)2 * gridBlocks * btm::kRedSlots);
     doubles += 32;                            // outLast
@@ -772,7 +789,7 @@ void make_slab(btm_case *C, Slab &S) {
     I.amgR = take(std::max<int64_t>(C->amgVecTotal, 1));
     I.amgRd = take((size_t)nC + C->amgVecTotal);
     I.ainv = take((size_t)nc * nc);
-    I.gj = take((size_t)4 * nc * nc);
+    I.gj = take(gj_doubles(nc));
     I.gpart = take((size_t)2 * gridBlocks * btm::kRedSlots);
     I.outLast = take(32);
     char *ctl = (char *)d;
@@ -798,7 +815,7 @@ void ensure_mixed(btm_case *C, Slab &S) {
     floats += 32 * cell;                      // cell arrays
     floats += up((size_t)nC + 2 * (size_t)nIF) + 2 * face + bnd;
     floats += up(std::max<int64_t>(C->amgValTotal, 1)) + 3 * up(std::max<int64_t>(C->amgVecTotal, 1)) +
-              up((size_t)nC + C->amgVecTotal) + up((size_t)2 * nc * nc) + up((size_t)8 * nc * nc);
+              up((size_t)nC + C->amgVecTotal) + up((size_t)2 * nc * nc) + up(2 * gj_doubles(nc));
     floats += 2 * face + 2 * cell;            // FP64 mass flux [nIF] and right-hand side [nC]
     floats += up((size_t)nC * (2 * btm::kBandMax + 1)) + cell;   // banded Cholesky factor (two layouts), 1 / diagonal
     const size_t aaLen = (size_t)btm::kAaFields * nC;             // Anderson vectors
@@ -829,7 +846,7 @@ void ensure_mixed(btm_case *C, Slab &S) {
     F.amgR = take(std::max<int64_t>(C->amgVecTotal, 1));
     F.amgRd = take((size_t)nC + C->amgVecTotal);
     F.ainv = (double *)take((size_t)2 * nc * nc);
-    F.gj = (double *)take((size_t)8 * nc * nc);
+    F.gj = (double *)take(2 * gj_doubles(nc));
     F.mflux = (double *)take(2 * (size_t)std::max(nIF, 1));
     F.src64 = (double *)take(2 * (size_t)nC);
     F.band = take((size_t)nC * (2 * btm::kBandMax + 1));
@@ -1121,7 +1138,7 @@ void autotune_case(btm_case *C, const double *coeffs, int variant) {
         ck(cudaEventCreate(&ev[0]), "event");
         ck(cudaEventCreate(&ev[1]), "event");
         const size_t smem = engine == 1 ? btm::mixed_smem_bytes(C->nC, C->nIF, C->amgVecTotal, C->amgValTotal,
-                                                                C->dmesh.coarseDirect ? C->amgCoarseN : 1, C->dmesh.band)
+                                                                C->dmesh.coarseDirect ? C->amgCoarseN : 1, C->dmesh.band, C->dmesh.rowW)
                                         : 0;
         const int shapes[2] = {256, 512};
         auto launch = [&](int k, int n) {
@@ -1654,7 +1671,7 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
                     if (g.engine == 1)
                         smem = std::max(smem, btm::mixed_smem_bytes(Cm->nC, Cm->nIF, Cm->amgVecTotal, Cm->amgValTotal,
                                                                     Cm->dmesh.coarseDirect ? Cm->amgCoarseN : 1,
-                                                                    Cm->dmesh.band));
+                                                                    Cm->dmesh.band, Cm->dmesh.rowW));
                 }
                 const int e = g.engine == 0
                                   ? btm::engine_launch_block(dInsts + at, (int)g.idx.size(), g.threads, gs, refAmg, maxCells)

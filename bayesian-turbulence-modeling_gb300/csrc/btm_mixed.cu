@@ -30,6 +30,7 @@
 #include "btm_bc.cuh"
 #include "btm_phases64.cuh"
 #include "btm_observe.cuh"
+#include "btm_dense.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -509,13 +510,7 @@ __device__ __noinline__ double mx_turb_cells(T &tm, const DevMesh &M, DevInst &I
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ float ldu_rowf(const DevMesh &M, const DevWork32 &F, const float *x, int c) {
-    float y = LD(F.diag + c) * LD(x + c);
-    for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-        const int f = M.cfFace[e], oth = M.cfOther[e];
-        if (oth >= 0) y = fmaf(LD(F.upper + f), LD(x + oth), y);
-        else y = fmaf(LD(F.lower + f), LD(x + (-(oth + 1))), y);
-    }
-    return y;
+    return ldu_off<T, false>(M, (const float *)F.diag, x, c, LD(F.diag + c) * LD(x + c));
 }
 __device__ __forceinline__ float jac_rdf(float d) { return (fabsf(d) > 1e-30f) ? 1.0f / d : 1.0f; }
 __device__ __forceinline__ float gs_rdf(float d) { return (fabsf(d) > 1e-30f) ? 1.0f / d : 0.0f; }
@@ -651,14 +646,14 @@ __device__ void mx_amg_level_rd(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     }
 }
 
-// Dense inverse of the coarsest level (Gauss-Jordan, ping-pong buffers), in
-// FP64: the coarsest Galerkin matrix of a pinned pure-Neumann pressure system
+// Dense inverse of the coarsest level in FP64: the coarsest Galerkin matrix of a pinned pure-Neumann pressure system
 // is nearly singular (its condition grows with the mesh), and an FP32 inverse
 // of it wrecked the preconditioner on a 2M-cell duct (39 PCG iterations per
 // solve instead of about one).  At most 32 rows, refreshed every
-// kAmgRefresh outer iterations.
+// kAmgRefresh outer iterations.  The sweep with ping-pong buffers is for a
+// matrix with a vanishing pivot, whose rows are passed over.
 template <class T>
-__device__ __noinline__ void mx_amg_coarse_inverse(T &tm, const DevMesh &M, DevWork32 &F) {
+__device__ __noinline__ void mx_amg_coarse_inverse_sweep(T &tm, const DevMesh &M, DevWork32 &F) {
     const int l = M.nLevels - 1;
     const AmgLevelDev &L = M.lev[l];
     const int n = L.n, w2 = 2 * n;
@@ -705,6 +700,34 @@ __device__ __noinline__ void mx_amg_coarse_inverse(T &tm, const DevMesh &M, DevW
 }
 
 template <class T>
+__device__ __noinline__ void mx_amg_coarse_inverse(T &tm, const DevMesh &M, DevWork32 &F) {
+    const int l = M.nLevels - 1, n = M.lev[l].n;
+    const AmgLevelDev &L = M.lev[l];
+    double *A = F.ainv;
+    const float *val = lev_valsf(F, M, l);
+    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
+    tm.sync();
+    for (int i = tm.rank(); i < n; i += tm.size()) {
+        double *row = A + (size_t)i * n;
+        if (l == 0) {
+            row[i] = LD(F.diag + i);
+            for (int e = M.cfOff[i]; e < M.cfOff[i + 1]; ++e) {
+                const int f = M.cfFace[e], oth = M.cfOther[e];
+                if (oth >= 0) row[oth] = LD(F.upper + f);
+                else row[-(oth + 1)] = LD(F.lower + f);
+            }
+        } else {
+            for (int q = L.rowPtr[i]; q < L.rowPtr[i + 1]; ++q) row[L.colIdx[q]] = LD(val + q);
+        }
+    }
+    tm.sync();
+    if (!dense_inverse(tm, A, F.gj, n)) {
+        tm.sync();
+        mx_amg_coarse_inverse_sweep(tm, M, F);
+    }
+}
+
+template <class T>
 __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 &F, int l, bool reverse) {
     const AmgLevelDev &L = M.lev[l];
     float *x = lev_xf(F, M, l);
@@ -718,18 +741,8 @@ __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 
             const float ri = LD(rd + i);
             if (ri == 0.0f) continue;
             float s = LD(b + i);
-            if (l == 0) {
-                for (int e = M.cfOff[i]; e < M.cfOff[i + 1]; ++e) {
-                    const int f = M.cfFace[e], oth = M.cfOther[e];
-                    if (oth >= 0) s = fmaf(-LD(F.upper + f), LD(x + oth), s);
-                    else s = fmaf(-LD(F.lower + f), LD(x + (-(oth + 1))), s);
-                }
-            } else {
-                for (int q2 = L.rowPtr[i]; q2 < L.rowPtr[i + 1]; ++q2) {
-                    const int j = L.colIdx[q2];
-                    if (j != i) s = fmaf(-LD(val + q2), LD(x + j), s);
-                }
-            }
+            if (l == 0) s = ldu_off<T, true>(M, (const float *)F.diag, (const float *)x, i, s);
+            else s = csr_off<T, true>(L, val, (const float *)x, i, i, s);
             x[i] = s * ri;
         }
         tm.sync();
@@ -749,8 +762,7 @@ __device__ __noinline__ void mx_amg_jacobi(T &tm, const DevMesh &M, DevWork32 &F
     const float *val = lev_valsf(F, M, l);
     const float *rd = lev_rdf(F, M, l);
     for (int i = tm.rank(); i < L.n; i += tm.size()) {
-        float s = LD(b + i);
-        for (int k = L.rowPtr[i]; k < L.rowPtr[i + 1]; ++k) s = fmaf(-LD(val + k), LD(x + L.colIdx[k]), s);
+        const float s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
         out[i] = fmaf(kJacobiWeight * LD(rd + i), s, LD(x + i));
     }
     tm.sync();
@@ -770,8 +782,7 @@ __device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 
             if (l == 0) {
                 s = ldu_rowf<T>(M, F, x, i);
             } else {
-                s = 0.0f;
-                for (int k = L.rowPtr[i]; k < L.rowPtr[i + 1]; ++k) s = fmaf(LD(val + k), LD(x + L.colIdx[k]), s);
+                s = csr_off<T, false>(L, val, x, i, -1, 0.0f);
             }
             acc += LD(b + i) - s;
         }
@@ -2027,14 +2038,14 @@ __device__ __host__ inline size_t smem_round(size_t b) { return (b + kSmemAlign 
 // not fit, or that the instance does not use, stays in global memory.
 enum SmemItem : int {
     SI_SYS = 0, SI_BAND, SI_BANDRD, SI_R, SI_S, SI_T, SI_PV, SI_V, SI_PP, SI_X, SI_AMGRD, SI_AMGX, SI_AMGB, SI_AMGR,
-    SI_AMGVAL, SI_RH, SI_PH, SI_SH, SI_RD, SI_SRC, SI_AINV, SI_CFOFF, SI_CFFACE, SI_CFOTHER, SI_COUNT
+    SI_AMGVAL, SI_RH, SI_PH, SI_SH, SI_RD, SI_SRC, SI_AINV, SI_ROWCOL, SI_ROWENT, SI_CFOFF, SI_CFFACE, SI_CFOTHER, SI_COUNT
 };
 
 // sizes in placement order (bytes, 0: not staged); returns the count.  With
 // a band factor (band > 0) the pressure correction does not use the AMG
 // arrays, which stay in global memory for the fallback solve.
 __device__ __host__ inline int smem_items(int nC, int nIF, int64_t vec, int64_t val, int nc, int nGather, int band,
-                                          size_t *sz) {
+                                          int rowW, size_t *sz) {
     const bool amg = band == 0;
     sz[SI_SYS] = 4 * ((size_t)nC + 2 * (size_t)nIF);                  // diag | upper | lower
     sz[SI_BAND] = band ? 4 * (size_t)nC * (2 * band + 1) : 0;          // banded Cholesky factor, two layouts
@@ -2045,6 +2056,7 @@ __device__ __host__ inline int smem_items(int nC, int nIF, int64_t vec, int64_t 
     sz[SI_AMGVAL] = amg ? 4 * (size_t)(val > 0 ? val : 1) : 0;
     for (int q = SI_RH; q <= SI_SRC; ++q) sz[q] = 4 * (size_t)nC;      // rh ph sh rd src
     sz[SI_AINV] = amg ? 8 * (size_t)nc * nc : 0;                       // coarse inverse (FP64)
+    sz[SI_ROWCOL] = sz[SI_ROWENT] = 4 * (size_t)nC * rowW;
     sz[SI_CFOFF] = 4 * ((size_t)nC + 1);
     sz[SI_CFFACE] = 4 * (size_t)nGather;
     sz[SI_CFOTHER] = 4 * (size_t)nGather;
@@ -2057,7 +2069,7 @@ __device__ void stage_smem(DevMesh &M, DevInst &I, unsigned char *dsm, size_t ca
     const int nc = M.coarseDirect ? M.lev[M.nLevels - 1].n : 1;
     const int nGather = 2 * nIF;
     size_t sz[SI_COUNT];
-    const int nItems = smem_items(nC, nIF, M.amgVecTotal, M.amgValTotal, nc, nGather, M.band, sz);
+    const int nItems = smem_items(nC, nIF, M.amgVecTotal, M.amgValTotal, nc, nGather, M.band, M.rowW, sz);
     size_t off = 0;
     int nc_ = 0;
     for (int q = 0; q < nItems; ++q) {
@@ -2088,6 +2100,8 @@ __device__ void stage_smem(DevMesh &M, DevInst &I, unsigned char *dsm, size_t ca
             case SI_RD: F.rd = f; break;
             case SI_SRC: F.src = f; break;
             case SI_AINV: F.ainv = (double *)p; break;
+            case SI_ROWCOL: copies[nc_++] = {p, M.rowCol, (int)sz[q]}; M.rowCol = (const int32_t *)p; break;
+            case SI_ROWENT: copies[nc_++] = {p, M.rowEnt, (int)sz[q]}; M.rowEnt = (const int32_t *)p; break;
             case SI_CFOFF: copies[nc_++] = {p, M.cfOff, (int)sz[q]}; M.cfOff = (const int32_t *)p; break;
             case SI_CFFACE: copies[nc_++] = {p, M.cfFace, (int)sz[q]}; M.cfFace = (const int32_t *)p; break;
             case SI_CFOTHER: copies[nc_++] = {p, M.cfOther, (int)sz[q]}; M.cfOther = (const int32_t *)p; break;
@@ -2104,7 +2118,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mixed_block(DevInst *insts, in
     __shared__ double tot[2 * (NT / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
-    __shared__ SmemCopy copies[4];
+    __shared__ SmemCopy copies[5];
     __shared__ int nCopies;
     if (blockIdx.x >= n) return;
     if (threadIdx.x == 0) {
@@ -2161,9 +2175,9 @@ int mixed_launch_grid(DevInst *dInst, int blocks, void *stream) {
 }
 
 // dynamic shared memory that would hold an instance's whole solver working set
-size_t mixed_smem_bytes(int nC, int nIF, int64_t vecTotal, int64_t valTotal, int coarseN, int band) {
+size_t mixed_smem_bytes(int nC, int nIF, int64_t vecTotal, int64_t valTotal, int coarseN, int band, int rowW) {
     size_t sz[SI_COUNT];
-    const int n = smem_items(nC, nIF, vecTotal, valTotal, coarseN, 2 * nIF, band, sz);
+    const int n = smem_items(nC, nIF, vecTotal, valTotal, coarseN, 2 * nIF, band, rowW, sz);
     size_t t = 0;
     for (int q = 0; q < n; ++q) t += smem_round(sz[q]);
     return t;

@@ -579,14 +579,7 @@ __device__ __noinline__ void phase_turb_cells(T &tm, const DevMesh &M, DevInst &
 // y = A x for one cell: diag*x, then face terms in ascending face order
 template <class T>
 __device__ __forceinline__ double ldu_row(const DevMesh &M, const DevInst &I, const double *x, int c) {
-    double y = LD(I.diag + c) * LD(x + c);
-    for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-        const int f = M.cfFace[e];
-        const int oth = M.cfOther[e];
-        if (oth >= 0) y = fma(LD(I.upper + f), LD(x + oth), y);
-        else y = fma(LD(I.lower + f), LD(x + (-(oth + 1))), y);
-    }
-    return y;
+    return ldu_off<T, false>(M, I.diag, x, c, LD(I.diag + c) * LD(x + c));
 }
 
 // reciprocal for the Jacobi preconditioner (LinearSolver.hpp:137-140): rows
