@@ -1037,30 +1037,98 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
 // (dx*dx + dy*dy) + dz*dz without contraction and the square root is taken
 // once of the minimum: sqrt is correctly rounded and monotone, so the result
 // is bit-identical to the reference's minimum of square roots.
+//
+// Nine FP64 instructions per pair at 1/64 of the FP32 rate bound the plain
+// search (1.9 ms for 122,880 cells and 992 faces).  A first pass finds each
+// cell's least distance in FP32, a second one the faces whose FP32 distance is
+// within twice its error of that, and only those are measured in FP64 (a
+// handful per cell, kept in a list so that the lanes measure theirs together).
+//
+// Error of an FP32 distance: coordinates relative to the first wall centre are
+// formed in FP64 and rounded once (|error| <= 2^-24 R, R the largest of them in
+// the cell and the walls), their differences once more; with the rounding of
+// the squares, sum and root the distance is off by less than 2^-20 R.  The
+// pass allows 2^-18 R.  Non-finite or overflowing coordinates make the
+// threshold infinite: every face is measured.
 // ---------------------------------------------------------------------------
 constexpr int kWallTile = 1024;
+constexpr int kWallList = 8;
+__device__ __forceinline__ double wall_d2(double x, double y, double z, const double *w) {
+    const double dx = __dsub_rn(x, w[0]), dy = __dsub_rn(y, w[1]), dz = __dsub_rn(z, w[2]);
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+}
 __global__ void __launch_bounds__(256) k_wall_distance(const double *cc, int nC, const double *wp, int nW,
                                                         double *out) {
-    __shared__ double sx[kWallTile], sy[kWallTile], sz[kWallTile];
+    __shared__ float sx[kWallTile], sy[kWallTile], sz[kWallTile];
+    __shared__ unsigned int reach;   // largest |wall coordinate|, as float bits (NaN and infinity largest)
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double x = 0.0, y = 0.0, z = 0.0;
+    const double ox = wp[0], oy = wp[1], oz = wp[2];
+    double x = ox, y = oy, z = oz;
     if (c < nC) { x = cc[3 * (size_t)c]; y = cc[3 * (size_t)c + 1]; z = cc[3 * (size_t)c + 2]; }
-    double best = INFINITY;
+    const float fx = (float)(x - ox), fy = (float)(y - oy), fz = (float)(z - oz);
+    if (threadIdx.x == 0) reach = 0;
+    auto stage = [&](int t0, int n, bool measure) {
+        __syncthreads();
+        float m = 0.0f;
+        for (int j = threadIdx.x; j < n; j += blockDim.x) {
+            const double *w = wp + 3 * (size_t)(t0 + j);
+            const float ax = (float)(w[0] - ox), ay = (float)(w[1] - oy), az = (float)(w[2] - oz);
+            sx[j] = ax; sy[j] = ay; sz[j] = az;
+            if (measure) {
+                const unsigned int big = max(__float_as_uint(fabsf(ax)),
+                                             max(__float_as_uint(fabsf(ay)), __float_as_uint(fabsf(az))));
+                m = __uint_as_float(max(__float_as_uint(m), big));
+            }
+        }
+        if (measure) atomicMax(&reach, __float_as_uint(m));
+        __syncthreads();
+    };
+    float least = INFINITY;
     for (int t0 = 0; t0 < nW; t0 += kWallTile) {
         const int n = min(kWallTile, nW - t0);
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            sx[j] = wp[3 * (size_t)(t0 + j)];
-            sy[j] = wp[3 * (size_t)(t0 + j) + 1];
-            sz[j] = wp[3 * (size_t)(t0 + j) + 2];
-        }
-        __syncthreads();
+        stage(t0, n, true);
+#pragma unroll 4
         for (int j = 0; j < n; ++j) {
-            const double dx = __dsub_rn(x, sx[j]), dy = __dsub_rn(y, sy[j]), dz = __dsub_rn(z, sz[j]);
-            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            best = d2 < best ? d2 : best;
+            const float dx = fx - sx[j], dy = fy - sy[j], dz = fz - sz[j];
+            least = fminf(least, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
         }
-        __syncthreads();
     }
+    float size = fmaxf(fmaxf(fabsf(fx), fabsf(fy)), fmaxf(fabsf(fz), __uint_as_float(reach)));
+    if (isnan(fx) || isnan(fy) || isnan(fz) || isnan(__uint_as_float(reach))) size = INFINITY;
+    const float edge = sqrtf(least) + 2.0f * 0x1p-18f * size;
+    float limit = fmaf(edge, edge, 1e-37f) * 1.00001f;
+    if (isnan(limit)) limit = INFINITY;
+    double best = INFINITY;
+    int list[kWallList], held = 0;
+    auto measure = [&]() {
+        int most = held;
+        for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+        for (int q = 0; q < most; ++q) {
+            if (q < held) {
+                int j = list[0];
+#pragma unroll
+                for (int e = 1; e < kWallList; ++e) j = q == e ? list[e] : j;
+                const double d2 = wall_d2(x, y, z, wp + 3 * (size_t)j);
+                best = d2 < best ? d2 : best;
+            }
+        }
+        held = 0;
+    };
+    for (int t0 = 0; t0 < nW; t0 += kWallTile) {
+        const int n = min(kWallTile, nW - t0);
+        if (nW > kWallTile) stage(t0, n, false);
+        for (int j = 0; j < n; ++j) {
+            const float dx = fx - sx[j], dy = fy - sy[j], dz = fz - sz[j];
+            // (a NaN here is a NaN in FP64 too, which is never the least)
+            if (!(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > limit)) {
+#pragma unroll
+                for (int e = 0; e < kWallList; ++e) list[e] = held == e ? t0 + j : list[e];
+                ++held;
+            }
+            if (__any_sync(0xffffffffu, held == kWallList)) measure();
+        }
+    }
+    measure();
     if (c < nC) out[c] = sqrt(best);
 }
 

@@ -292,7 +292,16 @@ struct GridTeam {
         if (warp < N) {
             const double *gp = gpart + (size_t)buf * gridDim.x * kRedSlots + warp;
             double s = Op::first(gp);
-            for (int q = lane; q < (int)gridDim.x; q += 32) s = Op::op(s, __ldcg(gp + (size_t)q * kRedSlots));
+            // all loads before the additions: a wait for L2 each would cost
+            // more than the barrier (3.8 us a sum instead of 2.6)
+            for (int q0 = lane; q0 < (int)gridDim.x; q0 += 32 * 8) {
+                double p[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) p[i] = __ldcg(gp + (size_t)min(q0 + 32 * i, (int)gridDim.x - 1) * kRedSlots);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (q0 + 32 * i < (int)gridDim.x) s = Op::op(s, p[i]);
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s = Op::op(s, __shfl_xor_sync(0xffffffffu, s, o));
             if (lane == 0) tot[warp] = s;

@@ -1,0 +1,70 @@
+"""Kernels whose paths depend on sizes, at the sizes where they can go wrong.
+
+  * wall distance: FP32 search with FP64 measurement against the numpy brute
+    force, bit for bit, at the edges of the shared-memory tile (1024 faces), of
+    the candidate list (8 faces at the same distance) and of the warp, with
+    coordinates far from the origin and beyond the FP32 range;
+  * dense coarsest inverse on the grid: a pressure correction to 1e-10 takes
+    about as many CG iterations as with an exact coarse solve.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import cases
+from rans_sst_py import Case, solve
+from rans_sst_py._lib import check, dptr, lib
+
+pytestmark = pytest.mark.gpu
+
+COEFF = np.array(cases.COEFF_DEFAULTS)
+
+
+def _device_distance(cc, wp):
+    L = lib()
+    L.btm_wall_distance.argtypes = [C.c_int32, C.POINTER(C.c_double), C.c_int32, C.POINTER(C.c_double),
+                                    C.POINTER(C.c_double)]
+    out = np.empty(len(cc))
+    check(L.btm_wall_distance(len(cc), dptr(cc), len(wp), dptr(wp), dptr(out)))
+    return out
+
+
+@pytest.mark.parametrize("n_wall", [1, 7, 8, 9, 1023, 1024, 1025, 2500])
+@pytest.mark.parametrize("n_cells", [1, 33, 257])
+@pytest.mark.parametrize("kind", ["random", "offset", "equidistant", "near", "huge", "tiny"])
+def test_wall_distance_bits(n_wall, n_cells, kind):
+    rng = np.random.default_rng(n_wall * 1000 + n_cells)
+    wp, cc = rng.uniform(-1, 1, (n_wall, 3)), rng.uniform(-1, 1, (n_cells, 3))
+    if kind == "offset":
+        wp, cc = wp + 1e6, cc + 1e6
+    elif kind == "equidistant":   # every face at one distance of every cell on the axis
+        a = np.linspace(0, 2 * np.pi, n_wall, endpoint=False)
+        wp, cc = np.stack([np.cos(a), np.sin(a), 0 * a], 1), cc * np.array([0, 0, 1.0])
+    elif kind == "near":
+        cc = wp[rng.integers(0, n_wall, n_cells)] + 1e-9 * cc
+    elif kind == "huge":
+        wp, cc = wp * 1e30, cc * 1e30
+    elif kind == "tiny":
+        wp, cc = wp * 1e-30, cc * 1e-30
+    wp, cc = np.ascontiguousarray(wp), np.ascontiguousarray(cc)
+    d = cc[:, None, :] - wp[None, :, :]
+    host = np.sqrt((d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2]).min(1)
+    assert np.array_equal(_device_distance(cc, wp), host)
+
+
+@pytest.mark.parametrize("a", [12, 13, 14])
+def test_grid_pressure_solve(a, oracle):
+    """One cold iteration on meshes just above the one-CTA size (17,280 to
+    23,520 cells; coarsest levels of different sizes modulo the panel width),
+    inner solves to 1e-10, against the oracle: they agree to the inner
+    tolerance times the conditioning of the systems (1e-7)."""
+    m, b, nu, ini = cases.bfs_case(2 * a, 12 * a, 6 * a, 3 * a)
+    s = cases.bfs_settings(1, 0.0)
+    s.inner_tolerance = 1e-10
+    s.inner_iterations = 1000
+    out = solve(Case(m, b, nu, s), COEFF, 0, ini)
+    ref, _ = oracle.solve(m, b, nu, s, COEFF, 0, **ini)
+    for f in ("U", "p"):
+        assert cases.rel_l2(out.state[f], ref[f]) < 1e-7, f
+    assert out.inner_split[1] < 200
