@@ -268,7 +268,28 @@ struct DevInst {
     RamgWork rg;
 };
 
+// One instance's share of a staging buffer between the host and the slabs of a
+// batch.  Downloads: kStageHead words (residuals and scales [0..8], error flag
+// [9], out [10..13] as 32-bit pairs, outInner [14..18], outTime [19..30]), the
+// observation outputs [nObs], then (state != 0) the state.  A state is U
+// [3 nC, xyz-interleaved], kStageCells cell arrays [nC] (p, k, omega, nuT, F1,
+// F2, Pk, CDkw), Ub [3 nB, interleaved], pb, kb, omegab [nB].
+constexpr int kStageHead = 32, kStageCells = 8;
+struct StageItem {
+    double *u[3], *cell[kStageCells];   // null cell arrays are skipped (uploads)
+    double *ub[3], *bnd[3];
+    const double *last, *obs;
+    const int32_t *err, *out;
+    const int64_t *inner;
+    const uint64_t *time;
+    int64_t at;                         // first word of the item's share
+    int32_t nC, nB, nObs, state;
+};
+inline int64_t stage_state_words(int nC, int nB) { return (int64_t)(3 + kStageCells) * nC + (int64_t)6 * nB; }
+
 // engine entry points (btm_engine.cu)
+int engine_pack(const StageItem *dItems, int n, int maxCells, double *dStage, void *stream);
+int engine_unpack(const StageItem *dItems, int n, int maxCells, const double *dStage, void *stream);
 int engine_block_threads();
 // refAmg: some instance of the launch uses the reference-order AMG (the
 // kernel instantiated with that solver is launched); maxCells: the largest

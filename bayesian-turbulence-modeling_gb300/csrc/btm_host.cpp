@@ -1054,6 +1054,108 @@ void download_state(btm_case *C, const btm::DevInst &I, btm_state *o, cudaStream
         for (int b = 0; b < nB; ++b) { o->Ub[3 * b] = hb[b]; o->Ub[3 * b + 1] = hb[nB + b]; o->Ub[3 * b + 2] = hb[2 * nB + b]; }
 }
 
+// ---- staging of batches -------------------------------------------------------
+constexpr size_t kStageBytes = size_t(64) << 20;
+constexpr size_t kStageItems = 32768;   // instances per part (a grid dimension)
+
+void free_stage(StageMem &M) {
+    if (M.pin) cudaFreeHost(M.pin);
+    if (M.dev) cudaFree(M.dev);
+    M = StageMem{};
+}
+
+// `bytes` of pinned and device staging memory (nothing in flight on the old)
+void ensure_stage(StageMem &M, size_t bytes) {
+    if (M.bytes >= bytes) return;
+    const size_t want = std::min(kStageBytes, std::max(bytes, 2 * M.bytes));
+    free_stage(M);
+    ck(cudaMallocHost((void **)&M.pin, want), "cudaMallocHost(staging)");
+    ck(cudaMalloc((void **)&M.dev, want), "cudaMalloc(staging)");
+    M.bytes = want;
+}
+
+btm::StageItem stage_item(const btm_case *C, const btm::DevInst &I) {
+    btm::StageItem S{};
+    double *u[3] = {I.ux, I.uy, I.uz}, *ub[3] = {I.ubx, I.uby, I.ubz}, *bnd[3] = {I.pb, I.kb, I.omb};
+    double *cell[btm::kStageCells] = {I.p, I.k, I.om, I.nut, I.f1, I.f2, I.pk, I.cdkw};
+    for (int q = 0; q < 3; ++q) { S.u[q] = u[q]; S.ub[q] = ub[q]; S.bnd[q] = bnd[q]; }
+    for (int q = 0; q < btm::kStageCells; ++q) S.cell[q] = cell[q];
+    S.last = I.outLast; S.obs = I.obsOut; S.err = I.err; S.out = I.out; S.inner = I.outInner; S.time = I.outTime;
+    S.nC = C->nC; S.nB = C->nB;
+    return S;
+}
+
+// Start states of a batch to the slabs: packed on the host (a state that
+// several instances start from once), one copy and one kernel per part.
+struct StageUpload {
+    StageMem &M;
+    cudaStream_t st;
+    std::vector<btm::StageItem> items;
+    std::vector<const btm_state *> from;
+    std::vector<int64_t> where;      // first word of from[q]
+    int64_t words = 0;
+    int maxCells = 0;
+    bool inFlight = false;
+    // false: too large for the staging memory
+    bool add(const btm_case *C, const btm::DevInst &I, const btm_state *ws, size_t batchWords) {
+        const int64_t need = btm::stage_state_words(C->nC, C->nB);
+        const int64_t itemWords = (int64_t)(sizeof(btm::StageItem) + 7) / 8;
+        if ((size_t)(need + 2 * itemWords) * 8 > kStageBytes) return false;
+        ensure_first(batchWords);
+        int64_t at = -1;
+        for (size_t q = from.size(); q-- > 0 && at < 0;)
+            if (from[q] == ws) at = where[q];
+        const int64_t extra = at < 0 ? need : 0;
+        if (items.size() == kStageItems || (size_t)(words + extra + (int64_t)(items.size() + 1) * itemWords) * 8 > M.bytes) {
+            flush();
+            at = -1;
+        }
+        if (at < 0) {
+            at = words;
+            from.push_back(ws);
+            where.push_back(at);
+            words += need;
+            double *o = (double *)M.pin + at;
+            const size_t nC = C->nC, nB = C->nB;
+            auto put = [&](const double *src, size_t n) {
+                if (src && n) std::memcpy(o, src, 8 * n);
+                o += n;
+            };
+            put(ws->U, 3 * nC);
+            for (const double *f : {ws->p, ws->k, ws->omega, ws->nuT, ws->F1, ws->F2, ws->Pk, ws->CDkw}) put(f, nC);
+            put(ws->Ub, 3 * nB);
+            for (const double *f : {ws->pb, ws->kb, ws->omegab}) put(f, nB);
+        }
+        btm::StageItem S = stage_item(C, I);
+        S.at = at;
+        const double *given[btm::kStageCells] = {ws->p, ws->k, ws->omega, ws->nuT, ws->F1, ws->F2, ws->Pk, ws->CDkw};
+        for (int q = 0; q < btm::kStageCells; ++q)
+            if (!given[q]) S.cell[q] = nullptr;
+        items.push_back(S);
+        maxCells = std::max(maxCells, std::max(C->nC, C->nB));
+        return true;
+    }
+    void ensure_first(size_t batchWords) {
+        if (items.empty() && !inFlight) ensure_stage(M, std::min(kStageBytes, 8 * batchWords));
+    }
+    void flush() {
+        if (items.empty()) return;
+        std::memcpy(M.pin + 8 * words, items.data(), sizeof(btm::StageItem) * items.size());
+        ck(cudaMemcpyAsync(M.dev, M.pin, 8 * words + sizeof(btm::StageItem) * items.size(), cudaMemcpyHostToDevice, st),
+           "upload");
+        const int e = btm::engine_unpack((const btm::StageItem *)(M.dev + 8 * words), (int)items.size(), maxCells,
+                                         (const double *)M.dev, st);
+        if (e) throw BtmError(BTM_ERR_CUDA, std::string("unpack: ") + cudaGetErrorString((cudaError_t)e));
+        // the pinned memory is written again by the next part, or by the results
+        ck(cudaStreamSynchronize(st), "upload sync");
+        items.clear();
+        from.clear();
+        where.clear();
+        words = 0;
+        inFlight = true;
+    }
+};
+
 // Launch-shape policy (overridable for tuning): instances up to
 // BTM_BLOCK_MAX_CELLS cells run one CTA each; CTAs have 256 threads (two
 // instances per SM) when every instance in the launch has at most
@@ -1278,6 +1380,7 @@ int btm_case_create(const btm_mesh *mesh, const btm_patch_bc *bcs, double nu, co
 void btm_case_destroy(btm_case *C) {
     if (!C) return;
     for (Slab &s : C->slabs) free_slab(s);
+    free_stage(C->stage);
     if (C->meshArena) cudaFree(C->meshArena);
     if (C->obsArena) cudaFree(C->obsArena);
     if (C->injTarget) cudaFree(C->injTarget);
@@ -1579,6 +1682,11 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
         std::vector<std::vector<double>> histBufs(n);
         std::vector<double *> histDev(n, nullptr);
         CallResources res;
+        size_t batchWords = 0;   // staging of the whole batch, items included
+        for (int i = 0; i < n; ++i)
+            batchWords += btm::kStageHead + cases[i]->dmesh.obs.n + 1 + btm::stage_state_words(cases[i]->nC, cases[i]->nB) +
+                          (sizeof(btm::StageItem) + 7) / 8;
+        StageUpload up{cases[0]->stage, st};
         for (int i = 0; i < n; ++i) {
             Job &J = jobs[i];
             btm::DevInst &I = J.S->inst;
@@ -1598,7 +1706,7 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
                 fill_inst(J.C, I, coeffs + 11 * (size_t)i, variants ? variants[i] : 0, ini);
                 if (ini && ini->mode == BTM_INIT_WARM) {
                     if (!ini->warm) throw BtmError(BTM_ERR_ARG, "warm init without a state");
-                    upload_state(J.C, I, ini->warm, st, stage);
+                    if (!up.add(J.C, I, ini->warm, batchWords)) upload_state(J.C, I, ini->warm, st, stage);
                 }
             }
             I.hist = nullptr;
@@ -1623,6 +1731,7 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
                 gridIdx.push_back(i);
             }
         }
+        up.flush();
         // one persistent launch per engine and launch shape for all
         // block-mode instances: an instance runs with its case's shape
         // (autotuned or by rule), whatever else is in the batch, so its
@@ -1710,56 +1819,107 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
         float ms = 0.0f;
         if (se == cudaSuccess && cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) g_launch_ms = ms;
         if (se != cudaSuccess) throw BtmError(BTM_ERR_CUDA, std::string("solve: ") + cudaGetErrorString(se));
-        // per-instance device timestamps: [8] start, [9] end of each solve
-        std::vector<std::array<uint64_t, btm::kPhaseSlots + 2>> times(n);
-        uint64_t t0 = 0;
-        for (int i = 0; i < n; ++i) {
-            ck(cudaMemcpy(times[i].data(), jobs[i].S->inst.outTime, sizeof(uint64_t) * (btm::kPhaseSlots + 2),
-                          cudaMemcpyDeviceToHost),
-               "status");
-            const uint64_t ts = times[i][btm::kPhaseSlots];
-            if (ts && (!t0 || ts < t0)) t0 = ts;
-        }
-        for (int i = 0; i < n; ++i) {
-            Job &J = jobs[i];
-            const btm::DevInst &I = J.S->inst;
-            int32_t outv[8];
-            int64_t innerv[5] = {0, 0, 0, 0, 0};
-            int32_t errv = 0;
-            double lastv[6];
-            ck(cudaMemcpy(outv, I.out, sizeof outv, cudaMemcpyDeviceToHost), "status");
-            ck(cudaMemcpy(innerv, I.outInner, sizeof innerv, cudaMemcpyDeviceToHost), "status");
-            ck(cudaMemcpy(lastv, I.outLast, sizeof lastv, cudaMemcpyDeviceToHost), "status");
-            ck(cudaMemcpy(&errv, I.err, sizeof errv, cudaMemcpyDeviceToHost), "status");
-            J.S->hasState = errv == 0;
-            J.S->lastTurbEst = outv[5];
-            const uint64_t *tns = times[i].data();
-            if (hists) {
-                btm_history &h = hists[i];
-                h.status = outv[0];
-                h.converged = outv[1];
-                h.diverged = outv[2];
-                h.final_iter = outv[3];
-                h.iterations_run = outv[4];
-                h.inner_iterations = innerv[0];
-                for (int q = 0; q < 4; ++q) h.inner_split[q] = innerv[q + 1];
-                h.polish_start = outv[7];
-                for (int q = 0; q < 6; ++q) h.last_residual[q] = lastv[q];
-                for (int q = 0; q < btm::kPhaseSlots; ++q) h.phase_ms[q] = 1e-6 * (double)tns[q];
-                const uint64_t t1 = tns[btm::kPhaseSlots], t2 = tns[btm::kPhaseSlots + 1];
-                h.solve_ms = t2 > t1 ? 1e-6 * (double)(t2 - t1) : 0.0;
-                h.finish_ms = (t0 && t2 > t0) ? 1e-6 * (double)(t2 - t0) : 0.0;
-                if (histDev[i]) {
-                    int rows = std::min(h.residual_capacity, outv[4]);
-                    ck(cudaMemcpy(h.residuals, histDev[i], sizeof(double) * 6 * rows, cudaMemcpyDeviceToHost), "hist");
+        // results through the staging memory, as many instances at a time as fit
+        std::vector<std::array<uint64_t, 2>> times(n);   // start and end of each solve
+        StageMem &M = cases[0]->stage;
+        const size_t itemWords = (sizeof(btm::StageItem) + 7) / 8;
+        for (int i0 = 0; i0 < n;) {
+            std::vector<btm::StageItem> items;
+            size_t words = 0;
+            int maxCells = 1, i1 = i0;
+            for (; i1 < n; ++i1) {
+                Job &J = jobs[i1];
+                btm::StageItem S = stage_item(J.C, J.S->inst);
+                const bool wantObs = J.S->inst.obsOut && hists && hists[i1].predictions;
+                S.nObs = wantObs ? J.C->dmesh.obs.n + 1 : 0;
+                const size_t head = btm::kStageHead + S.nObs, state = btm::stage_state_words(S.nC, S.nB);
+                S.state = outs && 8 * (head + state + itemWords) <= kStageBytes;
+                const size_t need = head + (S.state ? state : 0);
+                if (i1 > i0 && (items.size() == kStageItems || 8 * (words + need + (items.size() + 1) * itemWords) > kStageBytes)) break;
+                S.at = (int64_t)words;
+                words += need;
+                if (S.state) maxCells = std::max(maxCells, std::max(S.nC, S.nB));
+                items.push_back(S);
+            }
+            ensure_stage(M, 8 * (words + items.size() * itemWords));
+            ck(cudaMemcpyAsync(M.dev + 8 * words, items.data(), sizeof(btm::StageItem) * items.size(),
+                               cudaMemcpyHostToDevice, st),
+               "stage items");
+            const int e = btm::engine_pack((const btm::StageItem *)(M.dev + 8 * words), (int)items.size(), maxCells,
+                                           (double *)M.dev, st);
+            if (e) throw BtmError(BTM_ERR_CUDA, std::string("pack: ") + cudaGetErrorString((cudaError_t)e));
+            ck(cudaMemcpyAsync(M.pin, M.dev, 8 * words, cudaMemcpyDeviceToHost, st), "results");
+            ck(cudaStreamSynchronize(st), "results");
+            for (int i = i0; i < i1; ++i) {
+                Job &J = jobs[i];
+                const btm::DevInst &I = J.S->inst;
+                const btm::StageItem &S = items[i - i0];
+                const double *w = (const double *)M.pin + S.at;
+                int64_t errv;
+                int32_t outv[8];
+                int64_t innerv[5];
+                uint64_t tns[btm::kPhaseSlots + 2];
+                std::memcpy(&errv, w + 9, sizeof errv);
+                std::memcpy(outv, w + 10, sizeof outv);
+                std::memcpy(innerv, w + 14, sizeof innerv);
+                std::memcpy(tns, w + 19, sizeof tns);
+                times[i] = {tns[btm::kPhaseSlots], tns[btm::kPhaseSlots + 1]};
+                J.S->hasState = errv == 0;
+                J.S->lastTurbEst = outv[5];
+                if (hists) {
+                    btm_history &h = hists[i];
+                    h.status = outv[0];
+                    h.converged = outv[1];
+                    h.diverged = outv[2];
+                    h.final_iter = outv[3];
+                    h.iterations_run = outv[4];
+                    h.inner_iterations = innerv[0];
+                    for (int q = 0; q < 4; ++q) h.inner_split[q] = innerv[q + 1];
+                    h.polish_start = outv[7];
+                    for (int q = 0; q < 6; ++q) h.last_residual[q] = w[q];
+                    for (int q = 0; q < btm::kPhaseSlots; ++q) h.phase_ms[q] = 1e-6 * (double)tns[q];
+                    if (histDev[i]) {
+                        int rows = std::min(h.residual_capacity, outv[4]);
+                        ck(cudaMemcpy(h.residuals, histDev[i], sizeof(double) * 6 * rows, cudaMemcpyDeviceToHost), "hist");
+                    }
+                    if (S.nObs > 0) {
+                        const double *o = w + btm::kStageHead;
+                        for (int k = 0; k + 1 < S.nObs; ++k) h.predictions[k] = o[k];
+                        h.log_lik = o[S.nObs - 1];
+                    }
                 }
-                download_obs(J.C, I, &h, st);
+                if (outs) {
+                    if (S.state) {
+                        const double *o = w + btm::kStageHead + S.nObs;
+                        const size_t nC = S.nC, nB = S.nB;
+                        auto get = [&](double *dst, size_t m) {
+                            if (dst && m) std::memcpy(dst, o, 8 * m);
+                            o += m;
+                        };
+                        get(outs[i].U, 3 * nC);
+                        for (double *f : {outs[i].p, outs[i].k, outs[i].omega, outs[i].nuT, outs[i].F1, outs[i].F2,
+                                          outs[i].Pk, outs[i].CDkw})
+                            get(f, nC);
+                        get(outs[i].Ub, 3 * nB);
+                        for (double *f : {outs[i].pb, outs[i].kb, outs[i].omegab}) get(f, nB);
+                    } else {
+                        download_state(J.C, I, &outs[i], st, stage);
+                    }
+                    outs[i].turb_established = outv[5];
+                }
+                if (errv) throw BtmError(BTM_ERR_TIMEOUT, "a bounded device wait timed out; the solve was abandoned");
             }
-            if (outs) {
-                download_state(J.C, I, &outs[i], st, stage);
-                outs[i].turb_established = outv[5];
+            i0 = i1;
+        }
+        if (hists) {
+            uint64_t t0 = 0;
+            for (const auto &t : times)
+                if (t[0] && (!t0 || t[0] < t0)) t0 = t[0];
+            for (int i = 0; i < n; ++i) {
+                const uint64_t t1 = times[i][0], t2 = times[i][1];
+                hists[i].solve_ms = t2 > t1 ? 1e-6 * (double)(t2 - t1) : 0.0;
+                hists[i].finish_ms = (t0 && t2 > t0) ? 1e-6 * (double)(t2 - t0) : 0.0;
             }
-            if (errv) throw BtmError(BTM_ERR_TIMEOUT, "a bounded device wait timed out; the solve was abandoned");
         }
     } catch (const BtmError &e) {
         return fail(e.code, e.what());

@@ -28,6 +28,14 @@ struct Slab {
     btm::DevInst inst{};      // host copy with device pointers
 };
 
+// Staging memory of a case's batches: pinned host memory and its device
+// counterpart, grown to what the largest batch needed (kStageBytes at most:
+// larger results go through it in parts) and freed with the case.
+struct StageMem {
+    char *pin = nullptr, *dev = nullptr;
+    size_t bytes = 0;
+};
+
 struct btm_case {
     int nC = 0, nIF = 0, nB = 0, nF = 0, nP = 0;
     double nu = 0.0;
@@ -41,6 +49,7 @@ struct btm_case {
     int amgCoarseN = 0;
     int64_t amgValTotal = 0, amgVecTotal = 0;
     std::vector<Slab> slabs;
+    StageMem stage;
     void *obsArena = nullptr;        // observation plan (dmesh.obs points into it)
     double *injTarget = nullptr;     // injection target anisotropy (dmesh.bTarget)
     bool injAllRealizable = true;

@@ -23,7 +23,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 
 from . import _lib
-from ._lib import BtmHistory, BtmInit, Case, check, dptr, lib, new_state, state_struct
+from ._lib import BtmHistory, BtmInit, Case, check, dptr, lib, new_states, state_struct
 from ._types import (EvaluationResult, EvaluationStatus, InferenceParameterSet, SolverSettings,
                      Vec3, _vec)
 
@@ -95,15 +95,17 @@ def solve_batch(cases: Sequence[Case], coeffs, variants=None, inits=None, want_s
     n = len(cases)
     coeffs = np.ascontiguousarray(np.asarray(coeffs, np.float64).reshape(n, 11))
     var = np.ascontiguousarray(np.zeros(n, np.int32) if variants is None else np.asarray(variants, np.int32))
-    keep = []
+    keep, seen = [], {}
     ini_arr = (BtmInit * n)()
     for i in range(n):
-        ini_arr[i] = _init_struct(None if inits is None else inits[i], keep)
-    states = [new_state(c.n_cells, c.n_bnd) if want_state else None for c in cases]
-    st_arr = (_lib.BtmState * n)()
+        ini = None if inits is None else inits[i]
+        if id(ini) not in seen:   # instances that start alike share one struct
+            seen[id(ini)] = _init_struct(ini, keep)
+        ini_arr[i] = seen[id(ini)]
     if want_state:
-        for i in range(n):
-            st_arr[i] = state_struct(states[i])
+        states, st_arr = new_states(cases)
+    else:
+        states, st_arr = [None] * n, None
     hist = (BtmHistory * n)()
     res_bufs = [None] * n
     if history_capacity:

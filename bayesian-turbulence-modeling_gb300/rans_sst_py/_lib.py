@@ -235,6 +235,7 @@ def settings_struct(s) -> BtmSettings:
 
 CELL_FIELDS = ("p", "k", "omega", "nuT", "F1", "F2", "Pk", "CDkw")
 BND_FIELDS = ("pb", "kb", "omegab")
+STATE_ORDER = ("U",) + CELL_FIELDS + ("Ub",) + BND_FIELDS   # the pointers of BtmState
 
 
 def new_state(n_cells: int, n_bnd: int) -> dict:
@@ -245,6 +246,37 @@ def new_state(n_cells: int, n_bnd: int) -> dict:
         st[f] = np.zeros(max(n_bnd, 1))
     st["turb_established"] = 0
     return st
+
+
+def new_states(cases):
+    """States of a batch, one block of memory per instance, and the BtmState
+    array that points into them (addresses filled in one array operation per
+    case: thousands of pointer objects cost milliseconds)."""
+    n = len(cases)
+    arr = (BtmState * n)()
+    words = np.frombuffer(arr, np.uint64).reshape(n, C.sizeof(BtmState) // 8)
+    states, base, offs, layouts = [], np.empty(n, np.uint64), [], {}
+    for i, c in enumerate(cases):
+        key = (c.n_cells, c.n_bnd)
+        if key not in layouts:
+            nC, nB = c.n_cells, max(c.n_bnd, 1)
+            at, cuts = 0, {}
+            for f, size in [("U", 3 * nC)] + [(f, nC) for f in CELL_FIELDS] + [("Ub", 3 * nB)] + \
+                    [(f, nB) for f in BND_FIELDS]:
+                cuts[f] = (at, at + size)
+                at += size
+            layouts[key] = (at, cuts, np.array([8 * cuts[f][0] for f in STATE_ORDER], np.uint64))
+        size, cuts, off = layouts[key]
+        block = np.zeros(size)
+        st = {f: block[a:b] for f, (a, b) in cuts.items()}
+        st["U"], st["Ub"] = st["U"].reshape(-1, 3), st["Ub"].reshape(-1, 3)
+        st["turb_established"] = 0
+        states.append(st)
+        base[i] = block.ctypes.data
+        offs.append(off)
+    if n:
+        words[:, :len(STATE_ORDER)] = base[:, None] + np.array(offs)
+    return states, arr
 
 
 def state_struct(st: dict) -> BtmState:

@@ -4,6 +4,8 @@
     force, bit for bit, at the edges of the shared-memory tile (1024 faces), of
     the candidate list (8 faces at the same distance) and of the warp, with
     coordinates far from the origin and beyond the FP32 range;
+  * staging of a batch: states that several instances start from and results
+    of meshes of uneven size equal the same solves one by one, bit for bit;
   * dense coarsest inverse on the grid: a pressure correction to 1e-10 takes
     about as many CG iterations as with an exact coarse solve.
 """
@@ -13,12 +15,13 @@ import numpy as np
 import pytest
 
 import cases
-from rans_sst_py import Case, solve
+from rans_sst_py import Case, solve, solve_batch
 from rans_sst_py._lib import check, dptr, lib
 
 pytestmark = pytest.mark.gpu
 
 COEFF = np.array(cases.COEFF_DEFAULTS)
+FIELDS = ("U", "p", "k", "omega", "nuT", "F1", "F2", "Pk", "CDkw", "Ub", "pb", "kb", "omegab")
 
 
 def _device_distance(cc, wp):
@@ -51,6 +54,31 @@ def test_wall_distance_bits(n_wall, n_cells, kind):
     d = cc[:, None, :] - wp[None, :, :]
     host = np.sqrt((d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2]).min(1)
     assert np.array_equal(_device_distance(cc, wp), host)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batch_staging_equals_single_solves(precision):
+    """Cold, host-warm (shared and own states) and device-warm instances of
+    two meshes in one call."""
+    made = []
+    for m, b, nu, ini in (cases.periodic_channel(16, 120.0), cases.bfs_case()):
+        s = cases.channel_settings(6, 0.0) if nu > 1e-3 else cases.bfs_settings(6, 0.0)
+        s.precision = precision
+        made.append((Case(m, b, nu, s), ini))
+    first = [solve(c, COEFF, 0, ini) for c, ini in made]
+    warm = [o.state for o in first]
+    own = {k: (v * (1.0 + 1e-6) if isinstance(v, np.ndarray) else v) for k, v in warm[0].items()}
+    plan = [(0, made[0][1]), (1, warm[1]), (0, warm[0]), (1, made[1][1]), (0, warm[0]), (0, own), (1, warm[1])]
+    th = [COEFF * (1.0 + 0.01 * q) for q in range(len(plan))]
+    batch = solve_batch([made[k][0] for k, _ in plan], th, inits=[i for _, i in plan])
+    for q, (k, ini) in enumerate(plan):
+        alone = solve(made[k][0], th[q], 0, ini)
+        for f in FIELDS:
+            assert np.array_equal(batch[q].state[f], alone.state[f]), (q, f)
+        assert batch[q].iterations_run == alone.iterations_run
+        assert batch[q].inner_iterations == alone.inner_iterations
+        assert list(batch[q].last_residual) == list(alone.last_residual)
+        assert batch[q].state["turb_established"] == alone.state["turb_established"]
 
 
 @pytest.mark.parametrize("a", [12, 13, 14])
