@@ -82,8 +82,9 @@ struct ObsDev {
 // kRamgLevInts + field]): rows, offsets of the level's CSR row pointers,
 // entries, vectors, its map to the next level (-1: coarsest), the next
 // level's member offsets and members, its wavefront offsets, wavefront count
-// and entry count.
-enum : int { RL_N = 0, RL_PTR, RL_ENT, RL_VEC, RL_MAP, RL_MOFF, RL_MEM, RL_WFO, RL_NWF, RL_NNZ, kRamgLevInts };
+// and entry count, and where the records of its packed rows start (-1: not
+// packed).
+enum : int { RL_N = 0, RL_PTR, RL_ENT, RL_VEC, RL_MAP, RL_MOFF, RL_MEM, RL_WFO, RL_NWF, RL_NNZ, RL_REC, kRamgLevInts };
 
 // Per-instance pools of the reference-order AMG (btm_ramg.cuh): coarse levels
 // rebuilt from the actual matrix at every solve.  rowPool = 2 nC + 64 coarse

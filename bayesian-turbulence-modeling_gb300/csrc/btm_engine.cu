@@ -338,7 +338,7 @@ __device__ __noinline__ SolveResult team_ramg_pcg(BlockTeamRef &tm, const DevMes
     SolveResult res = {0, 0.0, 0.0, 0};
     const int nC = M.nC;
     const uint64_t t0 = tm.leader() ? globaltimer_ns() : 0;
-    const int nLev = ramg_setup(tm, M, I);
+    const int nLev = ramg_setup(tm, M, I, x != I.pp);
     if (tm.leader()) I.rg.setupNs += globaltimer_ns() - t0;
     double a0[1] = {0.0};
     for (int c = tm.rank(); c < nC; c += tm.size()) {
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
             res = team_gauss_seidel(tm, M, I, I.pp, I.S.innerIter, I.S.innerTol);
             break;
         case 12:  // reference-order AMG hierarchy of (diag, upper, lower)
-            if (I.S.refAmg) res.iterations = ramg_setup(tm, M, I);
+            if (I.S.refAmg) res.iterations = ramg_setup(tm, M, I, true);
             break;
     }
     tm.sync();

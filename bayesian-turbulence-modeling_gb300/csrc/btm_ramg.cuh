@@ -42,7 +42,7 @@ namespace btm {
 constexpr int kRamgMinCoarse = 50;     // minCoarseSize_ (LinearSolver.hpp:509)
 constexpr int kRamgCoarseSweeps = 50;  // coarseSweeps_
 constexpr int kRamgMaxCoarsen = 20;    // maxLevels_
-constexpr int kRamgWarpRows = 192;     // levels up to this size run on warp 0
+constexpr int kRamgWarpRows = 64;     // levels up to this size run on warp 0
 
 // One level as the device functions see it.  Level 0 reads its values from
 // the LDU system through entry ids (the lduToCSR layout built per case).
@@ -55,6 +55,8 @@ struct RLevel {
     double *x, *b, *r;
     const int32_t *map;             // this level -> next level (null at the coarsest)
     const int32_t *memOff, *mem;    // next level's members in this level, ascending
+    const double *rec, *rds;        // packed rows (null: not packed) and their 1/diag (not level 0)
+    bool shared;                    // x is in shared memory
     __device__ __forceinline__ double v(int j) const { return ent ? ldu[ent[j]] : val[j]; }
     __device__ __forceinline__ double d(int i) const { return ent ? ldu[i] : dg[i]; }
 };
@@ -81,6 +83,9 @@ __device__ __forceinline__ RLevel ramg_level(const DevMesh &M, const DevInst &I,
     L.map = t[RL_MAP] >= 0 ? W.map + t[RL_MAP] : nullptr;
     L.memOff = t[RL_MAP] >= 0 ? W.memOff + t[RL_MOFF] : nullptr;
     L.mem = t[RL_MAP] >= 0 ? W.mem + t[RL_MEM] : nullptr;
+    L.rec = t[RL_REC] < 0 ? nullptr : l == 0 ? I.g[0] : I.amgVal + t[RL_REC];
+    L.rds = W.cv + (l == 0 ? 0 : t[RL_VEC]);
+    L.shared = W.xs != nullptr;
     return L;
 }
 
@@ -135,41 +140,297 @@ struct RGroup {
 };
 
 // CSRMatrix::gaussSeidelSweep (LinearSolver.hpp:328-337), wavefront by
-// wavefront.  The reference divides by the diagonal; the sweep multiplies by
-// the reciprocal formed once per setup (at most one unit in the last place
-// per update), which keeps the FP64 division sequence off the chain of
+// wavefront.  The reference divides by the diagonal and subtracts products;
+// the sweeps multiply by the reciprocal formed once per setup and use fused
+// multiply-adds (at most a unit in the last place per operation), which keeps
+// the FP64 division and half of the FP64 instructions off the chain of
 // dependent operations every wavefront waits for.
-__device__ __noinline__ void ramg_gs(const RGroup &g, const RLevel &L) {
-    for (int w = 0; w < L.nWf; ++w) {
-        for (int q = L.wfOff[w] + g.rank; q < L.wfOff[w + 1]; q += g.size) {
-            const int i = L.wfRows[q];
-            double s = L.b[i];
+//
+// A wavefront is a short dependent step (a few rows per warp, 4 to 5 entries
+// each, 64 clocks per multiply-add), 4 sweeps of about 12 of them per level and
+// 50 sweeps of about 7 on the coarsest: read row by row from the CSR arrays,
+// the index, value and vector loads in front of each multiply-add took 1.5 us
+// (39 rows) to 4.7 us (1920 rows) a wavefront.  With one warp to an SMSP every
+// instruction and every wait on a load between two barriers counts, so the rows
+// are packed (ramg_pack) as records in wavefront order, read with three to five
+// 16-byte loads, and the two halves of the CTA take turns: while one half
+// computes a wavefront the other one fetches its rows of the next and works out
+// where their x are.  Between two barriers are left the x loads, the
+// multiply-adds and a store.  Rows are padded with zeros in their own column
+// (no branch per entry).  A coarsest level of up to 64 rows stays in the
+// registers of warp 0 for all its sweeps.  The entries of a row past the
+// eighth, and rows past the CTA's size, are read in place.
+constexpr int kRowRegs = 8;
+constexpr int kRec = 10, kRec0 = 6;   // doubles per record: values, columns (level 0: and 1/diag), by 16-byte parts
+__device__ __forceinline__ bool nonzero64(double v) { return (__double_as_longlong(v) << 1) != 0; }
+// x of a level, in shared memory (addresses of 32 bits) or global memory
+template <bool SM> struct RX;
+template <> struct RX<true> {
+    using At = uint32_t;
+    uint32_t base;
+    __device__ __forceinline__ RX(const RLevel &L) : base((uint32_t)__cvta_generic_to_shared(L.x)) {}
+    __device__ __forceinline__ At at(int i) const { return base + 8u * (unsigned int)i; }
+    __device__ __forceinline__ static double get(At a) {
+        double v;
+        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ static void put(At a, double v) {
+        asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+    }
+};
+template <> struct RX<false> {
+    using At = double *;
+    double *base;
+    __device__ __forceinline__ RX(const RLevel &L) : base(L.x) {}
+    __device__ __forceinline__ At at(int i) const { return base + i; }
+    __device__ __forceinline__ static double get(At a) { return *a; }
+    __device__ __forceinline__ static void put(At a, double v) { *a = v; }
+};
+template <int W, bool SM>
+struct RRow {
+    double b, rd, val[W];
+    typename RX<SM>::At to, from[W];
+    int row;       // -1: nothing to store
+    bool wide;     // more entries than W
+};
+template <int W, bool SM>
+__device__ __forceinline__ void ramg_record(const RX<SM> &x, const double *rec, const double *rds, int n, int slot,
+                                            RRow<W, SM> &R) {
+    const double2 *p = reinterpret_cast<const double2 *>(rec) + slot;
+#pragma unroll
+    for (int k = 0; k < W / 2; ++k) {
+        const double2 v = p[k * n];
+        R.val[2 * k] = v.x;
+        R.val[2 * k + 1] = v.y;
+    }
+    const double2 c = p[W / 2 * n];
+    const unsigned int col[4] = {(unsigned int)__double2loint(c.x), (unsigned int)__double2hiint(c.x),
+                                 (unsigned int)__double2loint(c.y), (unsigned int)__double2hiint(c.y)};
+    R.rd = W == 4 ? c.y : rds[slot];
+    R.wide = col[0] >> 15 & 1;
+#pragma unroll
+    for (int k = 0; k < W; ++k) R.from[k] = x.at(k & 1 ? col[k >> 1] >> 16 : col[k >> 1] & 0x7fffu);
+}
+// entries of a wide row i past the first kRowRegs off-diagonal ones (columns
+// ascend, so the diagonal is before entry j when its column is past i)
+__device__ __forceinline__ double ramg_rest(const RLevel &L, int i, double s) {
+    const int j0 = L.ptr[i], j1 = L.ptr[i + 1];
+    for (int j = j0 + kRowRegs; j < j1; ++j) {
+        const int c = L.col[j];
+        if (c != i && j - j0 - (c > i ? 1 : 0) >= kRowRegs) s = fma(-L.val[j], L.x[c], s);
+    }
+    return s;
+}
+// b minus the products of the row's first W entries
+template <int W, bool SM>
+__device__ __forceinline__ double ramg_sum(const RRow<W, SM> &R) {
+    double x[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) x[k] = RX<SM>::get(R.from[k]);
+    double s = R.b;
+#pragma unroll
+    for (int k = 0; k < W; ++k) s = fma(-R.val[k], x[k], s);
+    return s;
+}
+template <int W, bool SM>
+__device__ __forceinline__ void ramg_relax(const RLevel &L, const RRow<W, SM> &R) {
+    double s = ramg_sum(R);
+    if (W == kRowRegs && R.wide) s = ramg_rest(L, R.row, s);
+    RX<SM>::put(R.to, s * R.rd);
+}
+// The wavefronts of a level in the lanes of a warp (at most 32 of them):
+// first slot and number of rows
+struct RWaves {
+    int off, num;
+    __device__ __forceinline__ RWaves(const RLevel &L) {
+        const int w = threadIdx.x & 31;
+        off = w < L.nWf ? L.wfOff[w] : 0;
+        num = w < L.nWf ? L.wfOff[w + 1] - off : 0;
+    }
+    __device__ __forceinline__ static int of(int v, int w) { return __shfl_sync(0xffffffffu, v, w); }
+};
+// All sweeps of a level of at most 64 rows on one warp: slot s of the
+// wavefront order belongs to lane s % 32.  Wide rows keep up to kRowMore further
+// entries, which only their wavefronts spend instructions on.  False (and
+// nothing done): a row has more.
+constexpr int kRowMore = 6;
+template <bool SM>
+__device__ __noinline__ bool ramg_gs_resident(const RLevel &L, int sweeps) {
+    const RWaves T(L);
+    const int lane = threadIdx.x & 31, nWf = L.nWf, n = L.n;
+    const RX<SM> x(L);
+    RRow<8, SM> R[2];
+    double more[2][kRowMore];
+    typename RX<SM>::At moreAt[2][kRowMore];
+    int wave[2] = {-1, -1};
+    unsigned int used[2] = {0, 0};   // wavefronts with rows in slots 0-31 / 32-63
+    unsigned int wide[2] = {0, 0};   // ... and wide rows among them
+    bool fits = true;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int slot = min(lane + 32 * h, n - 1);
+        ramg_record(x, L.rec, L.rds, n, slot, R[h]);
+        const int i = R[h].row = L.wfRows[slot];
+        R[h].to = x.at(i);
+        R[h].b = L.b[i];
+#pragma unroll
+        for (int k = 0; k < kRowMore; ++k) { more[h][k] = 0.0; moreAt[h][k] = R[h].to; }
+        if (R[h].wide) {
+            int k = 0;
             for (int j = L.ptr[i]; j < L.ptr[i + 1]; ++j) {
-                const int c = L.col[j];
-                if (c != i) s -= L.v(j) * L.x[c];
+                if (L.col[j] == i || k++ < kRowRegs) continue;
+                if (k > kRowRegs + kRowMore) fits = false;
+#pragma unroll
+                for (int q = 0; q < kRowMore; ++q)
+                    if (q == k - 1 - kRowRegs) { more[h][q] = L.val[j]; moreAt[h][q] = x.at(L.col[j]); }
             }
-            const double ri = L.rd[i];
-            if (ri != 0.0) L.x[i] = s * ri;
         }
-        g.sync();
+    }
+    if (!__all_sync(0xffffffffu, fits)) return false;
+    for (int w = 0; w < nWf; ++w) {
+        const int o = RWaves::of(T.off, w), num = RWaves::of(T.num, w);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (o < 32 * h + 32 && o + num > 32 * h) used[h] |= 1u << w;
+            const int slot = lane + 32 * h;
+            const bool mine = slot >= o && slot < o + num;
+            if (mine && nonzero64(R[h].rd)) wave[h] = w;
+            if (__any_sync(0xffffffffu, mine && R[h].wide)) wide[h] |= 1u << w;
+        }
+    }
+    for (int t = 0; t < sweeps; ++t) {
+        for (int w = 0; w < nWf; ++w) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (used[h] >> w & 1) {
+                    double s = ramg_sum(R[h]);
+                    if (wide[h] >> w & 1) {
+#pragma unroll
+                        for (int k = 0; k < kRowMore; ++k) s = fma(-more[h][k], RX<SM>::get(moreAt[h][k]), s);
+                    }
+                    s = s * R[h].rd;
+                    if (wave[h] == w) RX<SM>::put(R[h].to, s);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    return true;
+}
+// sweeps of a level over the CTA; W = 4: level 0.  Thread r of a half takes row
+// r of the wavefronts of its half's turn and row r + half of the others.
+template <int W, bool SM>
+__device__ __noinline__ void ramg_gs_packed(const RLevel &L, int sweeps) {
+    const RWaves T(L);
+    const int nWf = L.nWf, n = L.n, nt = blockDim.x, half = nt >> 1, t0 = threadIdx.x;
+    const int rank[2] = {t0, t0 < half ? t0 + half : t0 - half};
+    const RX<SM> x(L);
+    const double *__restrict__ b = L.b, *__restrict__ rds = L.rds, *__restrict__ rec = L.rec;
+    const int32_t *__restrict__ rows = L.wfRows;
+    auto read = [&](int slot, RRow<W, SM> &R) {
+        const int row = rows[slot];
+        ramg_record(x, rec, rds, n, slot, R);
+        R.b = b[row];
+        R.to = x.at(row);
+        R.row = nonzero64(R.rd) ? row : -1;
+    };
+    auto fetch = [&](int w, int r, RRow<W, SM> &R) {
+        const int num = RWaves::of(T.num, w), o = RWaves::of(T.off, w);
+        R.row = -1;
+        if (r < num) read(o + r, R);
+    };
+    auto plus = [nWf](int w, int d) { w += d; return w >= nWf ? w - nWf : w; };
+    const int steps = sweeps * nWf;
+    RRow<W, SM> R[2];
+    int w = 0;
+    const int two = nWf > 1 ? 2 % nWf : 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) fetch(plus(0, h % nWf), rank[h], R[h]);
+    for (int t = 0; t < steps; t += 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (t + h < steps) {
+                const int num = RWaves::of(T.num, w);
+                if (R[h].row >= 0) ramg_relax(L, R[h]);
+                if (num > nt) {
+                    const int o = RWaves::of(T.off, w);
+                    for (int r = rank[h] + nt; r < num; r += nt) {
+                        RRow<W, SM> more;
+                        read(o + r, more);
+                        if (more.row >= 0) ramg_relax(L, more);
+                    }
+                }
+                __syncthreads();
+                fetch(plus(w, two), rank[h], R[h]);
+                w = plus(w, 1);
+            }
+        }
+    }
+}
+template <bool SM>
+__device__ __forceinline__ bool ramg_gs_records(const RGroup &g, const RLevel &L, int sweeps) {
+    // (level 0 has records of its own kind; a mesh of at most kRamgWarpRows
+    // cells sweeps it on warp 0 from its CSR rows)
+    if (g.wm) return !L.ent && L.n <= 64 && ramg_gs_resident<SM>(L, sweeps);
+    if (L.ent) ramg_gs_packed<4, SM>(L, sweeps);
+    else ramg_gs_packed<8, SM>(L, sweeps);
+    return true;
+}
+__device__ __noinline__ void ramg_gs(const RGroup &g, const RLevel &L, int sweeps) {
+    if (L.rec && (L.shared ? ramg_gs_records<true>(g, L, sweeps) : ramg_gs_records<false>(g, L, sweeps))) return;
+    for (int t = 0; t < sweeps; ++t) {
+        for (int w = 0; w < L.nWf; ++w) {
+            for (int q = L.wfOff[w] + g.rank; q < L.wfOff[w + 1]; q += g.size) {
+                const int i = L.wfRows[q];
+                double s = L.b[i];
+                for (int j = L.ptr[i]; j < L.ptr[i + 1]; ++j) {
+                    const int c = L.col[j];
+                    if (c != i) s = fma(-L.v(j), L.x[c], s);
+                }
+                const double ri = L.rd[i];
+                if (ri != 0.0) L.x[i] = s * ri;
+            }
+            g.sync();
+        }
     }
 }
 
 // CSRMatrix::residual (:318-326), then the restriction of the V-cycle
 // (:571-575): coarse b = sum of the members' residuals in ascending row
-// order, coarse x = 0
+// order, coarse x = 0.  A row's entries are fetched together.
 __device__ __noinline__ void ramg_restrict(const RGroup &g, const RLevel &L, const RLevel &Cl) {
-    for (int i = g.rank; i < L.n; i += g.size) {
+    // (locals: a store through one of the pointers would have the others read again)
+    const int32_t *__restrict__ ptr = L.ptr, *__restrict__ col = L.col, *__restrict__ ent = L.ent;
+    const double *__restrict__ vals = ent ? L.ldu : L.val, *__restrict__ x = L.x, *__restrict__ b = L.b;
+    double *res = L.r;
+    const int n = L.n, size = g.size, nc = Cl.n;
+    for (int i = g.rank; i < n; i += size) {
         double s = 0.0;
-        for (int j = L.ptr[i]; j < L.ptr[i + 1]; ++j) s += L.v(j) * L.x[L.col[j]];
-        L.r[i] = L.b[i] - s;
+        const int j1 = ptr[i + 1];
+        for (int j = ptr[i]; j < j1; j += kRowRegs) {
+            int at[kRowRegs];
+            double v[kRowRegs], xv[kRowRegs];
+#pragma unroll
+            for (int k = 0; k < kRowRegs; ++k) at[k] = min(j + k, j1 - 1);
+#pragma unroll
+            for (int k = 0; k < kRowRegs; ++k) xv[k] = x[col[at[k]]];
+#pragma unroll
+            for (int k = 0; k < kRowRegs; ++k) v[k] = vals[ent ? ent[at[k]] : at[k]];
+#pragma unroll
+            for (int k = 0; k < kRowRegs; ++k)
+                if (j + k < j1) s = fma(v[k], xv[k], s);
+        }
+        res[i] = b[i] - s;
     }
     g.sync();
-    for (int J = g.rank; J < Cl.n; J += g.size) {
+    const int32_t *__restrict__ memOff = L.memOff, *__restrict__ mem = L.mem;
+    double *cb = Cl.b, *cx = Cl.x;
+    for (int J = g.rank; J < nc; J += size) {
         double s = 0.0;
-        for (int q = L.memOff[J]; q < L.memOff[J + 1]; ++q) s += L.r[L.mem[q]];
-        Cl.b[J] = s;
-        Cl.x[J] = 0.0;
+        for (int q = memOff[J]; q < memOff[J + 1]; ++q) s += res[mem[q]];
+        cb[J] = s;
+        cx[J] = 0.0;
     }
     g.sync();
 }
@@ -185,21 +446,19 @@ __device__ void ramg_vcycle_range(const RGroup &g, const DevMesh &M, const DevIn
     if (down) {
         for (int l = l0; l < l1; ++l) {
             const RLevel L = ramg_level(M, I, l), Cl = ramg_level(M, I, l + 1);
-            ramg_gs(g, L);
-            ramg_gs(g, L);
+            ramg_gs(g, L, 2);
             ramg_restrict(g, L, Cl);
         }
     }
     if (down && up) {
         const RLevel Lc = ramg_level(M, I, l1);
-        for (int s = 0; s < kRamgCoarseSweeps; ++s) ramg_gs(g, Lc);
+        ramg_gs(g, Lc, kRamgCoarseSweeps);
     }
     if (up) {
         for (int l = l1 - 1; l >= l0; --l) {
             const RLevel L = ramg_level(M, I, l), Cl = ramg_level(M, I, l + 1);
             ramg_prolong(g, L, Cl);
-            ramg_gs(g, L);
-            ramg_gs(g, L);
+            ramg_gs(g, L, 2);
         }
     }
 }
@@ -245,15 +504,68 @@ __device__ int ramg_wavefronts(T &tm, const RamgWork &W, const int32_t *ptr, con
     return nWf;
 }
 
+// Packs the rows of every level as records in wavefront order (the coarsest
+// level first: its 50 sweeps are the longest chain).  Nothing is allocated for
+// them: the coarse levels take the place of the other AMG form's arrays, which
+// an instance with this one does not use (amgVal up to gpart is one stretch of
+// the slab), with their 1/diag in that of the Galerkin contributions, level 0 of a mesh of quadrilaterals that of the velocity
+// gradients, which the pressure correction leaves free (formed anew at the
+// start of every outer iteration; `vel`: they are still needed).  A level that
+// does not fit, or has more than 32 wavefronts, is swept from its CSR rows.
+template <class T>
+__device__ void ramg_pack(T &tm, const DevMesh &M, DevInst &I, int nLev, bool vel) {
+    const RamgWork &W = I.rg;
+    const int64_t cap = I.gpart - I.amgVal;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    int64_t used = 0;
+    for (int l = nLev - 1; l >= 0; --l) {
+        const RLevel L = ramg_level(M, I, l);
+        if (L.nWf > 32 || L.n > 32767) continue;
+        const int vec = l == 0 ? 0 : W.lev[l * kRamgLevInts + RL_VEC];
+        if (l == 0 ? vel || M.maxCellFaces > 4 : used + (int64_t)kRec * L.n > cap || vec + L.n > M.nnz0) continue;
+        double *rec = l == 0 ? I.g[0] : I.amgVal + used;
+        for (int w = warp; w < L.nWf; w += nw) {
+            const int o = L.wfOff[w], rows = L.wfOff[w + 1] - o;
+            for (int r = lane; r < rows; r += 32) {
+                const int i = L.wfRows[o + r];
+                // entry k and column k of the record
+                const int W8 = l == 0 ? 4 : kRowRegs, slot = o + r;
+                auto val = [&](int k) -> double & { return rec[2 * ((size_t)(k >> 1) * L.n + slot) + (k & 1)]; };
+                uint16_t *col = reinterpret_cast<uint16_t *>(rec + 2 * ((size_t)(W8 >> 1) * L.n + slot));
+                int k = 0;
+                for (int j = L.ptr[i]; j < L.ptr[i + 1]; ++j) {
+                    const int c = L.col[j];
+                    if (c == i) continue;
+                    if (k < W8) {
+                        val(k) = L.v(j);
+                        col[k] = (uint16_t)c;
+                    }
+                    ++k;
+                }
+                if (k > W8) col[0] |= 0x8000;
+                for (; k < W8; ++k) {
+                    val(k) = 0.0;
+                    col[k] = (uint16_t)i;
+                }
+                if (l == 0) rec[2 * ((size_t)2 * L.n + slot) + 1] = L.rd[i];
+                else W.cv[vec + slot] = L.rd[i];
+            }
+        }
+        if (threadIdx.x == 0) W.lev[l * kRamgLevInts + RL_REC] = (int)used;
+        if (l > 0) used += (int64_t)kRec * L.n;
+    }
+    tm.sync();
+}
+
 // Builds levels 1.. from level 0 (whose values are the current system) and
 // every level's reciprocal diagonals.  Returns the level count.
 template <class T>
-__device__ __noinline__ int ramg_setup(T &tm, const DevMesh &M, DevInst &I) {
+__device__ __noinline__ int ramg_setup(T &tm, const DevMesh &M, DevInst &I, bool vel) {
     const RamgWork &W = I.rg;
     const int n0 = M.nC;
     if (tm.leader()) {
         int32_t *t = W.lev;
-        t[RL_N] = n0; t[RL_PTR] = 0; t[RL_ENT] = 0; t[RL_VEC] = 0; t[RL_MAP] = -1; t[RL_NWF] = M.nWf0;
+        t[RL_N] = n0; t[RL_PTR] = 0; t[RL_ENT] = 0; t[RL_VEC] = 0; t[RL_MAP] = -1; t[RL_NWF] = M.nWf0; t[RL_REC] = -1;
     }
     for (int i = tm.rank(); i < n0; i += tm.size()) {
         const double d = I.diag[i];
@@ -410,7 +722,7 @@ __device__ __noinline__ int ramg_setup(T &tm, const DevMesh &M, DevInst &I) {
             t[RL_MAP] = mapUsed; t[RL_MOFF] = moffUsed; t[RL_MEM] = memUsed;
             int32_t *u = W.lev + (l + 1) * kRamgLevInts;
             u[RL_N] = nc; u[RL_PTR] = ptrUsed; u[RL_ENT] = entsUsed; u[RL_VEC] = rowsUsed; u[RL_MAP] = -1;
-            u[RL_WFO] = wfoUsed; u[RL_NWF] = nWf; u[RL_NNZ] = nnzc;
+            u[RL_WFO] = wfoUsed; u[RL_NWF] = nWf; u[RL_NNZ] = nnzc; u[RL_REC] = -1;
         }
         mapUsed += n; moffUsed += nc + 1; memUsed += n;
         ptrUsed += nc + 1; entsUsed += nnzc; rowsUsed += nc; wfoUsed += nWf + 1;
@@ -418,6 +730,7 @@ __device__ __noinline__ int ramg_setup(T &tm, const DevMesh &M, DevInst &I) {
         tm.sync();
     }
     tm.sync();
+    ramg_pack(tm, M, I, nLev, vel);
     return nLev;
 }
 

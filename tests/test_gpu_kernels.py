@@ -6,6 +6,8 @@
     coordinates far from the origin and beyond the FP32 range;
   * staging of a batch: states that several instances start from and results
     of meshes of uneven size equal the same solves one by one, bit for bit;
+  * reference-order AMG sweeps (packed rows, one warp, one CTA) on meshes at the
+    edges of their paths, against the oracle;
   * dense coarsest inverse on the grid: a pressure correction to 1e-10 takes
     about as many CG iterations as with an exact coarse solve.
 """
@@ -15,8 +17,9 @@ import numpy as np
 import pytest
 
 import cases
-from rans_sst_py import Case, solve, solve_batch
-from rans_sst_py._lib import check, dptr, lib
+from rans_sst_py import Case, FlowBoundaryConditions, Mesh, solve, solve_batch
+from rans_sst_py._forward import _init_struct
+from rans_sst_py._lib import BtmHistory, check, dptr, lib, new_state, state_struct
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +99,41 @@ def test_grid_pressure_solve(a, oracle):
     for f in ("U", "p"):
         assert cases.rel_l2(out.state[f], ref[f]) < 1e-7, f
     assert out.inner_split[1] < 200
+
+
+def _permuted_duct():
+    m = Mesh.make_square_duct_periodic_3d(3, 8, 8, 10.0, 2.0, 1.2)
+    m = m.permuted(np.random.default_rng(3).permutation(m.n_cells()))
+    m.compute_wall_distance()
+    b = FlowBoundaryConditions.channel_defaults(m, 0.0, 0.0, 0.0)
+    return m, b, 1.0 / 150.0, dict(u=(15.0, 0.0, 0.0), p=0.0, k=1e-2, omega=10.0)
+
+
+REFERENCE_AMG_MESHES = {
+    "64 cells, all levels on one warp": lambda: cases.periodic_channel(16, 120.0),
+    "72 cells, one level above the warp's": lambda: cases.periodic_channel(18, 120.0),
+    "more than 32 wavefronts": lambda: cases.periodic_channel(64, 180.0),
+    "hexahedra, level 0 from its CSR rows": _permuted_duct,
+    "3,597 cells, wide coarse rows, long wavefronts": lambda: cases.bfs_case(11, 66, 33, 16),
+}
+
+
+@pytest.mark.parametrize("momentum", ["BiCGSTAB", "AMG"])
+@pytest.mark.parametrize("name", sorted(REFERENCE_AMG_MESHES))
+def test_reference_amg_sweeps(name, momentum, oracle):
+    """Two cold iterations with the reference-order AMG (also as the momentum
+    solver, where the velocity gradients are still needed), inner solves to
+    1e-11, against the oracle: they agree to the inner tolerance times the
+    conditioning of the systems (1e-8)."""
+    m, b, nu, ini = REFERENCE_AMG_MESHES[name]()
+    s = cases.channel_settings(2, 0.0) if nu > 1e-3 else cases.bfs_settings(2, 0.0)
+    s.amg_order = "reference"
+    s.momentum_solver = momentum
+    s.inner_tolerance, s.inner_iterations = 1e-11, 400
+    # (the allocation-free call: the launch shape by rule, no tuning probe)
+    case, state, hist = Case(m, b, nu, s), new_state(m.n_cells(), m.n_boundary_faces()), BtmHistory()
+    st, start = state_struct(state), _init_struct(ini, [])
+    check(lib().btm_solve_noalloc(case.h, dptr(COEFF), 0, C.byref(start), C.byref(st), C.byref(hist)))
+    ref, _ = oracle.solve(m, b, nu, s, COEFF, 0, **ini)
+    for f in ("U", "k", "omega"):
+        assert cases.rel_l2(state[f], ref[f]) < 1e-8, f
