@@ -125,18 +125,20 @@ struct DevMesh {
     const double *nx, *ny, *nz, *sfx, *sfy, *sfz; // unit normal, n * area
     const double *ex, *ey, *ez;                   // d / max(delta, 1e-30)
     const double *aOverD;                         // area / deltaC (FP64-accurate fast assembly)
+    const double *wn, *rdelta;                    // 1 - w; 1 / deltaC
     // boundary faces [nB] (index b = face - nIF)
     const int32_t *bown;
     const double *barea, *bdeltaC, *bdeltaW;      // bdeltaW = max(delta, 1e-20) for omega wall BC
     const double *bnx, *bny, *bnz, *bsfx, *bsfy, *bsfz;
     const double *baOverD;                        // barea / bdeltaC
+    const double *brdelta;                        // 1 / bdeltaC
     const int32_t *bwall;                         // face belongs to a 'wall' patch
     const int32_t *bout;                          // face belongs to an 'outlet' patch
     const int32_t *bcU, *bcP, *bcK, *bcW;         // BC codes (BC_*) per face
     const int32_t *bcPp;                          // p' boundary rule: 0 copy owner, 1 keep zero
     const double *bvUx, *bvUy, *bvUz, *bvP, *bvK, *bvW;
     // cells [nC]
-    const double *vol, *wd;
+    const double *vol, *rvol, *wd;                // rvol = 1 / vol
     const int32_t *cfOff;      // [nC+1] internal-face gather list, ascending face index
     const int32_t *cfFace;     // face index
     const int32_t *cfOther;    // other cell, negated-1 when this cell is the neighbour: other = -(x+1)
@@ -175,6 +177,8 @@ struct DevSettings {
     int32_t maxIter, innerIter, turbStart, turbInterval, nutFloorIters, useWallFn;
     int32_t momSolver, turbSolver, pSolver;
     double convTol, divLimit, alphaU, alphaP, alphaK, alphaW, innerTol;
+    double relaxU, relaxK, relaxW;       // (1 - alpha) / alpha
+    double rAlphaU, rAlphaK, rAlphaW;    // 1 / alpha
     double bodyForce[3];
     double kMin, kMax, omegaMin, vonKarman;
     double alphaInj;       // blend factor of the Reynolds-stress injection source

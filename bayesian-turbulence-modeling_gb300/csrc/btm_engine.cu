@@ -670,6 +670,14 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
     clk.start(tm.leader());
     const uint64_t tStart = tm.leader() ? globaltimer_ns() : 0;
     if (tm.leader()) I.rg.setupNs = 0;
+    const bool d2 = M.is2d && !I.solveZ;   // no z normals, no z velocity
+    // the momentum diffusion coefficients fit kold | omold (adjacent, idle until
+    // the turbulence equations) on meshes of quadrilaterals
+    double *keepD = (I.omold + nC) - I.kold >= M.nIF ? I.kold : nullptr;
+    if (d2) {
+        phase_grad_init(tm, M, I);
+        tm.sync();
+    }
 
     for (int iter = 0; iter < S.maxIter; ++iter) {
         if (!tm.ok()) break;
@@ -677,13 +685,17 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
         const bool turbActive = iter >= S.turbStart;
         const bool turbUpdate = turbActive && ((iter - S.turbStart) % S.turbInterval == 0);
         // 1. turbulence closure fields at the start-of-iteration U
-        phase_velgrad(tm, M, I, 7);
-        phase_grad1(tm, M, I.p, I.pb, I.gpx, I.gpy, I.gpz);
+        // (the injection source also reads the z gradients, which the packed rows
+        // of the reference-order AMG may have replaced)
+        if (d2 && I.inj) phase_grad_init(tm, M, I);
+        if (d2) phase_grads<T, true>(tm, M, I, 15);
+        else phase_grads<T, false>(tm, M, I, 15);
         tm.sync();
         if (turbUpdate) {
             if (!turbEst && iter >= S.turbStart + S.nutFloorIters) turbEst = 1;
             const double nutMin = turbEst ? 0.0 : 0.1 * nu;
-            phase_sst(tm, M, I, nutMin);
+            if (d2) phase_closure<T, true>(tm, M, I, nutMin);
+            else phase_closure<T, false>(tm, M, I, nutMin);
             tm.sync();
         }
         clk.lap(0);
@@ -693,13 +705,15 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
         for (int comp = 0; comp < 3; ++comp) {
             if (comp == 2 && !I.solveZ) break;
             if (comp > 0) {
-                phase_velgrad(tm, M, I, 1 << (comp - 1));
+                if (d2) phase_grads<T, true>(tm, M, I, 1 << (comp - 1));
+                else phase_grads<T, false>(tm, M, I, 1 << (comp - 1));
                 tm.sync();
             }
             if (comp == 0 && I.inj) phase_inj(tm, M, I, I.g, I.nut, iter == 0);
-            phase_mom_faces(tm, M, I, comp);
+            if (d2) phase_momq_faces<T, true>(tm, M, I, comp, comp == 0, keepD);
+            else phase_momq_faces<T, false>(tm, M, I, comp, comp == 0, keepD);
             tm.sync();
-            phase_mom_cells(tm, M, I, comp);
+            phase_momq_cells(tm, M, I, comp);
             tm.sync();
             clk.lap(1);
             double *x = comp == 0 ? I.ux : (comp == 1 ? I.uy : I.uz);
@@ -709,11 +723,13 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
             clk.lap(2);
         }
         phase_bc_u(tm, M, I);
+        phase_dp(tm, M, I);
         tm.sync();
         // 3. pressure correction
-        phase_p_faces(tm, M, I);
+        if (d2) phase_pq_faces<T, true>(tm, M, I);
+        else phase_pq_faces<T, false>(tm, M, I);
         tm.sync();
-        phase_p_cells(tm, M, I);
+        phase_pq_cells(tm, M, I);
         tm.sync();
         clk.lap(3);
         SolveResult resP = team_solve(tm, M, I, S.pSolver, I.pp, S.innerIter, S.innerTol);
@@ -729,13 +745,14 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
             const double alphaP = S.alphaP;
             for (int c = tm.rank(); c < nC; c += tm.size()) {
                 double gx[1], gy[1], gz[1];
-                gg_cell<T, 1>(M, c, P, PB, gx, gy, gz);
+                if (d2) gq_cell<T, 1, true>(M, c, P, PB, gx, gy, gz);
+                else gq_cell<T, 1, false>(M, c, P, PB, gx, gy, gz);
                 const double aP = LD(I.aPx + c);
                 double rAP = (fabs(aP) > 1e-30) ? 1.0 / aP : 0.0;
                 double vol = M.vol[c];
                 I.ux[c] = LD(I.ux + c) - rAP * gx[0] * vol;
                 I.uy[c] = LD(I.uy + c) - rAP * gy[0] * vol;
-                I.uz[c] = LD(I.uz + c) - rAP * gz[0] * vol;
+                if (!d2) I.uz[c] = LD(I.uz + c) - rAP * gz[0] * vol;
                 I.p[c] = LD(I.p + c) + alphaP * LD(I.pp + c);
             }
             tm.sync();
@@ -749,9 +766,10 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
         double change[4];   // largest k and omega, largest change of k and of omega
         if (turbUpdate) {
             for (int c = tm.rank(); c < nC; c += tm.size()) { I.kold[c] = LD(I.k + c); I.omold[c] = LD(I.om + c); }
-            phase_turb_faces(tm, M, I, 0);
+            if (d2) phase_turbq_faces<T, true>(tm, M, I, 0, true);
+            else phase_turbq_faces<T, false>(tm, M, I, 0, true);
             tm.sync();
-            phase_turb_cells(tm, M, I, 0);
+            phase_turbq_cells(tm, M, I, 0);
             tm.sync();
             resK = team_solve(tm, M, I, S.turbSolver, I.k, S.innerIter, S.innerTol);
             innerTurb += resK.iterations;
@@ -760,9 +778,10 @@ __device__ void simple_solve(T &tm, const DevMesh &M, DevInst &I) {
             tm.sync();
             phase_bc_k(tm, M, I, true);
             tm.sync();
-            phase_turb_faces(tm, M, I, 1);
+            if (d2) phase_turbq_faces<T, true>(tm, M, I, 1, false);
+            else phase_turbq_faces<T, false>(tm, M, I, 1, false);
             tm.sync();
-            phase_turb_cells(tm, M, I, 1);
+            phase_turbq_cells(tm, M, I, 1);
             tm.sync();
             resW = team_solve(tm, M, I, S.turbSolver, I.om, S.innerIter, S.innerTol);
             innerTurb += resW.iterations;
@@ -969,36 +988,49 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
     const DevMesh &M = sM;
     DevInst &I = sI;
     const int ph = I.dbgPhase, arg = I.dbgArg;
+    const bool d2 = M.is2d && !I.solveZ;
+    auto grads = [&]() {
+        if (d2) {
+            phase_grad_init(tm, M, I);
+            tm.sync();
+            phase_grads<BlockTeamRef, true>(tm, M, I, 15);
+        } else {
+            phase_grads<BlockTeamRef, false>(tm, M, I, 15);
+        }
+        tm.sync();
+    };
     SolveResult res = {0, 0.0, 0.0, 0};
     switch (ph) {
         case 1:  // greenGaussGrad of p -> gp
-            phase_grad1(tm, M, I.p, I.pb, I.gpx, I.gpy, I.gpz);
+            grads();
             break;
         case 2:  // computeFields (no floor) + |S|
-            phase_velgrad(tm, M, I, 7);
-            tm.sync();
-            phase_sst(tm, M, I, -1.0);
+            grads();
+            if (d2) phase_closure<BlockTeamRef, true>(tm, M, I, -1.0);
+            else phase_closure<BlockTeamRef, false>(tm, M, I, -1.0);
             break;
         case 3:  // assembleMomentum(comp = arg)
-            phase_velgrad(tm, M, I, 7);
-            phase_grad1(tm, M, I.p, I.pb, I.gpx, I.gpy, I.gpz);
+            grads();
+            if (d2) phase_momq_faces<BlockTeamRef, true>(tm, M, I, arg, true, nullptr);
+            else phase_momq_faces<BlockTeamRef, false>(tm, M, I, arg, true, nullptr);
             tm.sync();
-            phase_mom_faces(tm, M, I, arg);
-            tm.sync();
-            phase_mom_cells(tm, M, I, arg);
+            phase_momq_cells(tm, M, I, arg);
             break;
         case 4:  // assemblePressureCorrection with I.aPx
-            phase_grad1(tm, M, I.p, I.pb, I.gpx, I.gpy, I.gpz);
+            grads();
+            phase_dp(tm, M, I);
             tm.sync();
-            phase_p_faces(tm, M, I);
+            if (d2) phase_pq_faces<BlockTeamRef, true>(tm, M, I);
+            else phase_pq_faces<BlockTeamRef, false>(tm, M, I);
             tm.sync();
-            phase_p_cells(tm, M, I);
+            phase_pq_cells(tm, M, I);
             break;
         case 5:
         case 6:  // assembleKEquation / assembleOmegaEquation
-            phase_turb_faces(tm, M, I, ph - 5);
+            if (d2) phase_turbq_faces<BlockTeamRef, true>(tm, M, I, ph - 5, true);
+            else phase_turbq_faces<BlockTeamRef, false>(tm, M, I, ph - 5, true);
             tm.sync();
-            phase_turb_cells(tm, M, I, ph - 5);
+            phase_turbq_cells(tm, M, I, ph - 5);
             break;
         case 7:  // v = A r
             for (int c = tm.rank(); c < M.nC; c += tm.size()) I.v[c] = ldu_row<BlockTeamRef>(M, I, I.r, c);

@@ -322,6 +322,12 @@ btm::DevSettings dev_settings(const btm_settings &s) {
     d.alphaP = s.alpha_p;
     d.alphaK = s.alpha_k;
     d.alphaW = s.alpha_omega;
+    d.relaxU = (1.0 - s.alpha_u) / s.alpha_u;
+    d.relaxK = (1.0 - s.alpha_k) / s.alpha_k;
+    d.relaxW = (1.0 - s.alpha_omega) / s.alpha_omega;
+    d.rAlphaU = 1.0 / s.alpha_u;
+    d.rAlphaK = 1.0 / s.alpha_k;
+    d.rAlphaW = 1.0 / s.alpha_omega;
     d.innerTol = s.inner_tolerance;
     for (int i = 0; i < 3; ++i) d.bodyForce[i] = s.body_force[i];
     d.kMin = s.k_min;
@@ -678,6 +684,13 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
     for (int f = 0; f < nIF; ++f) aOverD[f] = area[f] / dC[f];
     for (int b = 0; b < nB; ++b) baOverD[b] = barea[b] / bdC[b];
     const size_t o_aod = P(aOverD), o_baod = P(baOverD);
+    // complements and reciprocals, each rounded once (the divisions by them on
+    // the device are the same bits, see div_by)
+    std::vector<double> wn(nIF), rdC(nIF), rbdC(nB), rvol(nC);
+    for (int f = 0; f < nIF; ++f) { wn[f] = 1.0 - w[f]; rdC[f] = 1.0 / dC[f]; }
+    for (int b = 0; b < nB; ++b) rbdC[b] = 1.0 / bdC[b];
+    for (int c = 0; c < nC; ++c) rvol[c] = 1.0 / vol[c];
+    const size_t o_wn = P(wn), o_rdC = P(rdC), o_rbdC = P(rbdC), o_rvol = P(rvol);
     struct LevOff { size_t rowPtr, colIdx, diagPos, gOff, gIdx, map, aggOff, aggMem, colorOff, colorRows; };
     const size_t o_r0Ent = P(lv[0].entry), o_wf0Off = P(wf0Off), o_wf0Rows = P(wf0Rows);
     std::vector<LevOff> lo(nL);
@@ -720,6 +733,7 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
     D.pinFace = I32(o_pin);
     D.rowEnt = I32(o_rowEnt); D.rowCol = I32(o_rowCol);
     D.aOverD = F64(o_aod);
+    D.wn = F64(o_wn); D.rdelta = F64(o_rdC); D.brdelta = F64(o_rbdC); D.rvol = F64(o_rvol);
     D.r0Ent = I32(o_r0Ent);
     D.wf0Off = I32(o_wf0Off);
     D.wf0Rows = I32(o_wf0Rows);
@@ -2001,6 +2015,9 @@ int btm_debug_phase(btm_case *C, int32_t phase, const double *coeffs, int32_t va
         std::vector<double> bx(nB), by(nB), bz(nB);
         for (int b = 0; b < nB; ++b) { bx[b] = q[3 * b]; by[b] = q[3 * b + 1]; bz[b] = q[3 * b + 2]; }
         q += 3 * (size_t)nB;
+        // a state with z velocity has its z terms, also on a 2-D mesh
+        for (double v : uz) if (v != 0.0) I.solveZ = 1;
+        for (double v : bz) if (v != 0.0) I.solveZ = 1;
         if (nB > 0) {
             ck(cudaMemcpyAsync(I.ubx, bx.data(), 8 * nB, cudaMemcpyHostToDevice, st), "dbg");
             ck(cudaMemcpyAsync(I.uby, by.data(), 8 * nB, cudaMemcpyHostToDevice, st), "dbg");

@@ -1,7 +1,9 @@
 // btm_phases64.cuh - the FP64 closure, gradient and assembly phases and the
-// FP64 LDU row product and BiCGSTAB.  The FP64 engine compiles them with
-// -fmad=false so the assembly rounds exactly like the reference; the
-// mixed-precision engine uses them for its FP64 polishing stage.
+// FP64 LDU row product and BiCGSTAB, in two forms: the mixed-precision engine's
+// FP64 polishing stage (phase_velgrad, phase_grad1, phase_sst, phase_mom_*,
+// phase_p_*, phase_turb_*: FP64-accurate) and the FP64 engine's (phase_grads,
+// phase_closure, phase_momq_*, phase_pq_*, phase_turbq_*), compiled with
+// -fmad=false, whose assembly rounds exactly like the reference.
 #pragma once
 #include "btm_common.h"
 #include "btm_team.cuh"
@@ -25,50 +27,15 @@ __device__ __forceinline__ Coef load_coef(const DevInst &I) {
 }
 __device__ __forceinline__ double blend(double p1, double p2, double F1) { return F1 * p1 + (1.0 - F1) * p2; }
 
-__device__ __forceinline__ double sst_F1(const Coef &c, double k, double omega, double y, double nu, double CDkw_pos) {
-    double sqrtK = sqrt(smax(k, 0.0));
-    double omSafe = smax(omega, 1e-20);
-    double ySafe = smax(y, 1e-20);
-    double y2s = ySafe * ySafe;
-    double term1 = sqrtK / (c.bstar * omSafe * ySafe);
-    double term2 = 500.0 * nu / (y2s * omSafe);
-    double CDpos = smax(CDkw_pos, 1e-20);
-    double term3 = 4.0 * c.sw2 * smax(k, 0.0) / (CDpos * y2s);
-    double arg1 = smin(smax(term1, term2), term3);
-    double a4 = arg1 * arg1 * arg1 * arg1;
-    return tanh(a4);
-}
-__device__ __forceinline__ double sst_F2(const Coef &c, double k, double omega, double y, double nu) {
-    double sqrtK = sqrt(smax(k, 0.0));
-    double omSafe = smax(omega, 1e-20);
-    double ySafe = smax(y, 1e-20);
-    double y2 = ySafe * ySafe;
-    double term1 = 2.0 * sqrtK / (c.bstar * omSafe * ySafe);
-    double term2 = 500.0 * nu / (y2 * omSafe);
-    double arg2 = smax(term1, term2);
-    return tanh(arg2 * arg2);
-}
-__device__ __forceinline__ double sst_nut(const Coef &c, double k, double omega, double S, double F2) {
-    double kSafe = smax(k, 0.0);
-    if (c.variant == 1) return kSafe / smax(omega, 1e-20);
-    double denom = smax(c.a1 * omega, S * F2);
-    denom = smax(denom, 1e-20);
-    return c.a1 * kSafe / denom;
-}
-__device__ __forceinline__ double sst_Pk(const Coef &c, double nuT, double S, double k, double omega) {
-    double Pk_raw = nuT * S * S;
-    double Pk_lim = 10.0 * c.bstar * smax(k, 0.0) * smax(omega, 1e-20);
-    return smin(Pk_raw, Pk_lim);
-}
 __device__ __forceinline__ double sst_Pw(const Coef &c, double nuT, double S, double k, double omega) {
     double S2 = S * S;
     double lim = 10.0 * c.bstar * smax(k, 0.0) * smax(omega, 1e-20) / smax(nuT, 1e-30);
     return smin(S2, lim);
 }
 
-// The same closure with FP64 reciprocals formed once per cell (the mixed
-// engine's FP64 polishing stage: FP64-accurate, not reference-rounded; GB300
-// spends tens of FP64 instructions on every division).
+// The closure (core/src/SSTModel.cpp:9-96) with FP64 reciprocals formed once per
+// cell (the mixed engine's FP64 polishing stage: FP64-accurate, not
+// reference-rounded; phase_closure is the FP64 engine's).
 struct SstCell { double F1, F2, nuT, Pk, CDkw; };
 __device__ __forceinline__ SstCell sst_cell_fast(const Coef &c, double kc, double wc, double y, double nu, double S,
                                                  double gradDot) {
@@ -103,7 +70,7 @@ __device__ __forceinline__ SstCell sst_cell_fast(const Coef &c, double kc, doubl
 // Green-Gauss gradients (core/include/Field.hpp:122-152): per cell, internal
 // faces in ascending face order, then boundary faces, then / V.
 // ---------------------------------------------------------------------------
-template <class T, int NF, bool Fast = false>
+template <class T, int NF>
 __device__ __forceinline__ void gg_cell(const DevMesh &M, int c, const double *const *phi,
                                         const double *const *phib, double *gx, double *gy, double *gz) {
     double ax[NF], ay[NF], az[NF], pc[NF];
@@ -147,42 +114,438 @@ __device__ __forceinline__ void gg_cell(const DevMesh &M, int c, const double *c
     }
     const double V = M.vol[c];
     if (V > 1e-30) {
-        if (Fast) {
-            const double rv = 1.0 / V;
+        const double rv = 1.0 / V;
 #pragma unroll
-            for (int q = 0; q < NF; ++q) { ax[q] *= rv; ay[q] *= rv; az[q] *= rv; }
-        } else {
-#pragma unroll
-            for (int q = 0; q < NF; ++q) { ax[q] = ax[q] / V; ay[q] = ay[q] / V; az[q] = az[q] / V; }
-        }
+        for (int q = 0; q < NF; ++q) { ax[q] *= rv; ay[q] *= rv; az[q] *= rv; }
     }
 #pragma unroll
     for (int q = 0; q < NF; ++q) { gx[q] = ax[q]; gy[q] = ay[q]; gz[q] = az[q]; }
 }
 
+// ---------------------------------------------------------------------------
+// The FP64 engine's forms of the phases.  An FP64 instruction costs 16 to
+// 19 clocks of an SM per warp and 64 of its SMSP, so these do without the ones
+// whose result is known: divisions by a known divisor (div_by), 1 - w, the
+// reciprocals and relaxation factors of the settings, quotients shared between
+// faces or closure functions, sign tests; and with D2 (all normals in the x-y
+// plane and no z velocity: DevMesh::is2d and no z-momentum system) the z terms,
+// which are zero.  Every remaining operation rounds as in the reference, in the
+// same order.  4x128 channel, one instance: closure 124 -> 52 us an outer
+// iteration, momentum assembly 70 -> 43, p' assembly 27 -> 16.
+// ---------------------------------------------------------------------------
+// x / d, correctly rounded, from r = 1 / d correctly rounded: one
+// multiplication and two fused multiply-adds (P. Markstein, IBM J. Res. Dev. 34
+// (1990) 111; N. Brisebarre, J.-M. Muller, S. K. Raina, IEEE Trans. Comput. 53
+// (2004) 1069: exact when nothing over- or underflows on the way).  Exponents
+// outside 2^-620 .. 2^620 of x, d or r take the division itself.
+__device__ __forceinline__ bool mid_range(double v) {
+    return ((unsigned int)__double2hiint(v) & 0x7fffffffu) - 0x19300000u < 0x4d800000u;
+}
+__device__ __forceinline__ double div_by(double x, double d, double r) {
+    if (mid_range(x) && mid_range(d)) {
+        const double q = x * r;
+        return fma(fma(-q, d, x), r, q);
+    }
+    if (x == 0.0 && mid_range(d)) return x * r;
+    return x / d;
+}
+// smax(v, 0) and smax(-v, 0) without an FP64 comparison (the sign of zero aside)
+__device__ __forceinline__ bool is_negative(double v) {   // v < 0: a NaN and -0 are not
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return u - 0x8000000000000001ull < 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ double pos_part(double v) { return is_negative(v) ? 0.0 : v; }
+__device__ __forceinline__ double flip(double v, bool neg) {
+    return __hiloint2double(__double2hiint(v) ^ (neg ? 0x80000000 : 0), __double2loint(v));
+}
+
+// The internal faces of cell c in ascending face order: body(face, other cell,
+// c is the owner), four list entries fetched at a time.
+template <class F>
+__device__ __forceinline__ void cell_faces(const DevMesh &M, int c, F body) {
+    const int nC = M.nC, nIF = M.nIF, width = M.rowW;
+    for (int w0 = 0; w0 < width; w0 += 4) {
+        int ent[4], col[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const size_t at = (size_t)(w0 + k < width ? w0 + k : 0) * nC + c;
+            col[k] = w0 + k < width ? M.rowCol[at] : -1;
+            ent[k] = M.rowEnt[at] - nC;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (col[k] >= 0) body(ent[k] < nIF ? ent[k] : ent[k] - nIF, col[k], ent[k] < nIF);
+    }
+}
+
+template <class T, int NF, bool D2>
+__device__ __forceinline__ void gq_cell(const DevMesh &M, int c, const double *const *phi, const double *const *phib,
+                                        double *gx, double *gy, double *gz) {
+    double pc[NF];
+#pragma unroll
+    for (int q = 0; q < NF; ++q) { gx[q] = 0.0; gy[q] = 0.0; gz[q] = 0.0; pc[q] = LD(phi[q] + c); }
+    cell_faces(M, c, [&](int f, int oth, bool own) {
+        const double w = M.w[f], wn = M.wn[f];
+        const double wa = own ? w : wn, wb = own ? wn : w;   // this cell's weight, the other's
+        const double sx = flip(M.sfx[f], !own), sy = flip(M.sfy[f], !own), sz = D2 ? 0.0 : flip(M.sfz[f], !own);
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+            const double phiF = pc[q] * wa + LD(phi[q] + oth) * wb;
+            gx[q] = gx[q] + sx * phiF;
+            gy[q] = gy[q] + sy * phiF;
+            if (!D2) gz[q] = gz[q] + sz * phiF;
+        }
+    });
+    for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
+        const int b = M.cbFace[e];
+        const double sx = M.bsfx[b], sy = M.bsfy[b], sz = D2 ? 0.0 : M.bsfz[b];
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+            const double pb = LD(phib[q] + b);
+            gx[q] = gx[q] + sx * pb;
+            gy[q] = gy[q] + sy * pb;
+            if (!D2) gz[q] = gz[q] + sz * pb;
+        }
+    }
+    const double V = M.vol[c], r = M.rvol[c];
+    if (V > 1e-30) {
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+            gx[q] = div_by(gx[q], V, r);
+            gy[q] = div_by(gy[q], V, r);
+            if (!D2) gz[q] = div_by(gz[q], V, r);
+        }
+    }
+}
+
+// pressure gradient and the velocity gradients of the components in `which`
+// (bits 0-2; 8: the pressure) in one pass.  D2: component z and z derivatives
+// are left as they are (zeroed once, see phase_grad_init).
+template <class T, bool D2>
+__device__ __noinline__ void phase_grads(T &tm, const DevMesh &M, DevInst &I, int which) {
+    const double *U[3] = {I.ux, I.uy, I.uz};
+    const double *UB[3] = {I.ubx, I.uby, I.ubz};
+    auto keep = [&](int i, int c, double x, double y, double z) {
+        I.g[3 * i][c] = x;
+        I.g[3 * i + 1][c] = y;
+        if (!D2) I.g[3 * i + 2][c] = z;
+    };
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        if ((which & 7) == 7) {
+            constexpr int NU = D2 ? 2 : 3;
+            const double *P[4] = {U[0], U[1], D2 ? I.p : U[2], I.p};
+            const double *PB[4] = {UB[0], UB[1], D2 ? I.pb : UB[2], I.pb};
+            double gx[NU + 1], gy[NU + 1], gz[NU + 1];
+            gq_cell<T, NU + 1, D2>(M, c, P, PB, gx, gy, gz);
+#pragma unroll
+            for (int i = 0; i < NU; ++i) keep(i, c, gx[i], gy[i], gz[i]);
+            I.gpx[c] = gx[NU];
+            I.gpy[c] = gy[NU];
+            if (!D2) I.gpz[c] = gz[NU];
+        } else {
+            const int i = which == 1 ? 0 : which == 2 ? 1 : 2;
+            const double *P[1] = {U[i]};
+            const double *PB[1] = {UB[i]};
+            double gx[1], gy[1], gz[1];
+            gq_cell<T, 1, D2>(M, c, P, PB, gx, gy, gz);
+            keep(i, c, gx[0], gy[0], gz[0]);
+        }
+    }
+}
+// the gradients that D2 passes never write
+template <class T>
+__device__ void phase_grad_init(T &tm, const DevMesh &M, DevInst &I) {
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        I.g[2][c] = I.g[5][c] = 0.0;
+        I.g[6][c] = I.g[7][c] = I.g[8][c] = 0.0;
+        I.gpz[c] = 0.0;
+    }
+}
+
+// SSTModel::computeFields + frozen |S| + startup floor (SIMPLESolver.cpp:736-768;
+// core/src/SSTModel.cpp:9-96), from the gradients in I.g; nutMin < 0 skips the floor
+template <class T, bool D2>
+__device__ __noinline__ void phase_closure(T &tm, const DevMesh &M, DevInst &I, double nutMin) {
+    const Coef cf = load_coef(I);
+    const double nu = I.nu;
+    const double *P[2] = {I.k, I.om};
+    const double *PB[2] = {I.kb, I.omb};
+    const double nu500 = 500.0 * nu, sw2x2 = 2.0 * cf.sw2, sw2x4 = 4.0 * cf.sw2, ten = 10.0 * cf.bstar;
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        const double S11 = LD(I.g[0] + c), S22 = LD(I.g[4] + c);
+        const double S12 = 0.5 * (LD(I.g[1] + c) + LD(I.g[3] + c));
+        double Sc;
+        if (D2) {
+            Sc = sqrt(2.0 * (S11 * S11 + S22 * S22 + 2.0 * (S12 * S12)));
+        } else {
+            const double S33 = LD(I.g[8] + c);
+            const double S13 = 0.5 * (LD(I.g[2] + c) + LD(I.g[6] + c));
+            const double S23 = 0.5 * (LD(I.g[5] + c) + LD(I.g[7] + c));
+            Sc = sqrt(2.0 * (S11 * S11 + S22 * S22 + S33 * S33 + 2.0 * (S12 * S12 + S13 * S13 + S23 * S23)));
+        }
+        double gx[2], gy[2], gz[2];
+        gq_cell<T, 2, D2>(M, c, P, PB, gx, gy, gz);
+        const double kc = pos_part(LD(I.k + c));
+        const double wc = smax(LD(I.om + c), 1e-20);
+        const double y = smax(M.wd[c], 1e-20), y2 = y * y;
+        double dot = gx[0] * gx[1] + gy[0] * gy[1];
+        if (!D2) dot = dot + gz[0] * gz[1];
+        const double CDkw = sw2x2 / wc * dot;
+        // (2 a) / b is twice a / b: F2's first argument is twice F1's, and its
+        // second one F1's
+        const double term1 = sqrt(kc) / (cf.bstar * wc * y);
+        const double term2 = nu500 / (y2 * wc);
+        double F1 = 1.0;
+        if (cf.variant != 2) {
+            const double term3 = sw2x4 * kc / (smax(CDkw, 1e-20) * y2);
+            const double arg1 = smin(smax(term1, term2), term3);
+            F1 = tanh(arg1 * arg1 * arg1 * arg1);
+        }
+        const double arg2 = smax(2.0 * term1, term2);
+        const double F2 = tanh(arg2 * arg2);
+        const double nuT = cf.variant == 1 ? kc / wc : cf.a1 * kc / smax(smax(cf.a1 * wc, Sc * F2), 1e-20);
+        I.smag[c] = Sc;
+        I.cdkw[c] = CDkw;
+        I.f1[c] = F1;
+        I.f2[c] = F2;
+        I.pk[c] = smin(nuT * Sc * Sc, ten * kc * wc);
+        I.nut[c] = (nutMin < 0.0) ? nuT : smax(nuT, nutMin);
+    }
+}
+
+// momentum assembly (SIMPLESolver.cpp:56-203).  `first`: the diffusion
+// coefficient is formed and, where `keepD` is given, kept for the next component
+// (viscosity and geometry do not change between components).
+template <class T, bool D2>
+__device__ __noinline__ void phase_momq_faces(T &tm, const DevMesh &M, DevInst &I, int comp, bool first,
+                                              double *keepD) {
+    const double nu = I.nu;
+    const double *gc0 = I.g[comp], *gc1 = I.g[3 + comp], *gc2 = I.g[6 + comp];
+    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+        const int o = M.own[f], n = M.nbr[f];
+        const double Sf = M.area[f], w = M.w[f], wn = M.wn[f];
+        const double nuo = LD(I.nut + o), nun = LD(I.nut + n);
+        double Df;
+        if (first || !keepD) {
+            const double nuEff_f = w * (nu + nuo) + wn * (nu + nun);
+            Df = div_by(nuEff_f * Sf, M.deltaC[f], M.rdelta[f]);
+            if (keepD) keepD[f] = Df;
+        } else {
+            Df = keepD[f];   // written by this thread
+        }
+        const double nx = M.nx[f], ny = M.ny[f], nz = D2 ? 0.0 : M.nz[f];
+        double m = (LD(I.ux + o) * w + LD(I.ux + n) * wn) * nx + (LD(I.uy + o) * w + LD(I.uy + n) * wn) * ny;
+        if (!D2) m = m + (LD(I.uz + o) * w + LD(I.uz + n) * wn) * nz;
+        const double mFlux = m * Sf;
+        I.upper[f] = -(Df + pos_part(-mFlux));
+        I.lower[f] = -(Df + pos_part(mFlux));
+        double t = (LD(gc0 + o) * w + LD(gc0 + n) * wn) * nx + (LD(gc1 + o) * w + LD(gc1 + n) * wn) * ny;
+        if (!D2) t = t + (LD(gc2 + o) * w + LD(gc2 + n) * wn) * nz;
+        I.fflux[f] = (w * nuo + wn * nun) * t * Sf;
+    }
+}
+template <class T>
+__device__ __noinline__ void phase_momq_cells(T &tm, const DevMesh &M, DevInst &I, int comp) {
+    const double nu = I.nu, fb = I.S.bodyForce[comp];
+    const double *Uc = comp == 0 ? I.ux : (comp == 1 ? I.uy : I.uz);
+    const double *Ubc = comp == 0 ? I.ubx : (comp == 1 ? I.uby : I.ubz);
+    const double *gp = comp == 0 ? I.gpx : (comp == 1 ? I.gpy : I.gpz);
+    const double *gc0 = I.g[comp], *gc1 = I.g[3 + comp], *gc2 = I.g[6 + comp];
+    const bool wallFn = I.S.useWallFn != 0;
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        double diag = 0.0, ts = 0.0, src = 0.0;
+        cell_faces(M, c, [&](int f, int, bool own) {
+            diag = diag + flip(LD((own ? I.lower : I.upper) + f), true);
+            ts = ts + flip(LD(I.fflux + f), !own);
+        });
+        const double nutc = LD(I.nut + c);
+        for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
+            const int b = M.cbFace[e];
+            const double Sf = M.barea[b];
+            const double nuEff = (M.bwall[b] && !wallFn) ? nu : nu + nutc;
+            const double Db = div_by(nuEff * Sf, M.bdeltaC[b], M.brdelta[b]);
+            const double Ub = LD(Ubc + b);
+            const double mFlux = (LD(I.ubx + b) * M.bnx[b] + LD(I.uby + b) * M.bny[b] + LD(I.ubz + b) * M.bnz[b]) * Sf;
+            if (mFlux >= 0) {
+                diag = diag + (mFlux + Db);
+                src = src + Db * Ub;
+            } else {
+                diag = diag + Db;
+                src = src + (Db - mFlux) * Ub;
+            }
+        }
+        // transpose stress, wall-aware boundary treatment in patch order
+        if (M.cbpOff[c] < M.cbpOff[c + 1]) {
+            const double gcx = LD(gc0 + c), gcy = LD(gc1 + c), gcz = LD(gc2 + c);
+            for (int e = M.cbpOff[c]; e < M.cbpOff[c + 1]; ++e) {
+                const int b = M.cbpFace[e];
+                const double cfac = M.bwall[b] ? 0.0 : nutc;
+                ts = ts + cfac * (gcx * M.bnx[b] + gcy * M.bny[b] + gcz * M.bnz[b]) * M.barea[b];
+            }
+        }
+        const double vol = M.vol[c];
+        src = src - LD(gp + c) * vol;
+        if (fb != 0.0) src = src + fb * vol;
+        src = src + ts;
+        if (I.inj) src = src + LD(I.inj + (size_t)comp * M.nC + c);
+        src = src + I.S.relaxU * diag * LD(Uc + c);
+        diag = div_by(diag, I.S.alphaU, I.S.rAlphaU);
+        I.diag[c] = diag;
+        I.src[c] = src;
+        if (comp == 0) I.aPx[c] = diag;
+    }
+}
+
+// V / aP of every cell (both sides of its faces and the boundary use it) into
+// I.ph, which the momentum solves are done with
+template <class T>
+__device__ __forceinline__ void phase_dp(T &tm, const DevMesh &M, DevInst &I) {
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        const double aP = LD(I.aPx + c);
+        I.ph[c] = (fabs(aP) > 1e-30) ? M.vol[c] / aP : 0.0;
+    }
+}
+// pressure-correction assembly (SIMPLESolver.cpp:322-450) with that quotient
+template <class T, bool D2>
+__device__ __noinline__ void phase_pq_faces(T &tm, const DevMesh &M, DevInst &I) {
+    const bool rc = M.rhieChow != 0;
+    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+        const int o = M.own[f], n = M.nbr[f];
+        const double Sf = M.area[f], delta = M.deltaC[f], rdelta = M.rdelta[f], w = M.w[f], wn = M.wn[f];
+        const double dP_f = w * LD(I.ph + o) + wn * LD(I.ph + n);
+        const double dPS = dP_f * Sf;
+        const double coeff = div_by(dPS, delta, rdelta);
+        I.upper[f] = -coeff;
+        I.lower[f] = -coeff;
+        double m = (LD(I.ux + o) * w + LD(I.ux + n) * wn) * M.nx[f] + (LD(I.uy + o) * w + LD(I.uy + n) * wn) * M.ny[f];
+        if (!D2) m = m + (LD(I.uz + o) * w + LD(I.uz + n) * wn) * M.nz[f];
+        double massFlux = m * Sf;
+        if (rc) {
+            double gb = (LD(I.gpx + o) * w + LD(I.gpx + n) * wn) * M.ex[f] + (LD(I.gpy + o) * w + LD(I.gpy + n) * wn) * M.ey[f];
+            if (!D2) gb = gb + (LD(I.gpz + o) * w + LD(I.gpz + n) * wn) * M.ez[f];
+            massFlux += -dPS * (div_by(LD(I.p + n) - LD(I.p + o), delta, rdelta) - gb);
+        }
+        I.fflux[f] = massFlux;
+    }
+}
+template <class T>
+__device__ __noinline__ void phase_pq_cells(T &tm, const DevMesh &M, DevInst &I) {
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        double diag = 0.0, src = 0.0;
+        cell_faces(M, c, [&](int f, int, bool own) {
+            diag = diag + flip(LD(I.upper + f), true);
+            src = src + flip(LD(I.fflux + f), own);
+        });
+        for (int e = M.cbpOff[c]; e < M.cbpOff[c + 1]; ++e) {
+            const int b = M.cbpFace[e];
+            const double Sf = M.barea[b];
+            const double massFlux = (LD(I.ubx + b) * M.bnx[b] + LD(I.uby + b) * M.bny[b] + LD(I.ubz + b) * M.bnz[b]) * Sf;
+            src = src - massFlux;
+            if (M.bout[b]) diag = diag + div_by(LD(I.ph + c) * Sf, M.bdeltaC[b], M.brdelta[b]);
+        }
+        if (!M.hasOutlet && c == 0) diag += fabs(diag) > 1e-30 ? diag : 1.0;
+        I.diag[c] = diag;
+        I.src[c] = src;
+        I.pp[c] = 0.0;
+    }
+}
+
+// k (which = 0) or omega (which = 1) face pass; without `flux` it takes the face
+// mass flux that the last pass left in I.fflux (U does not change from k to omega)
+template <class T, bool D2>
+__device__ __noinline__ void phase_turbq_faces(T &tm, const DevMesh &M, DevInst &I, int which, bool flux) {
+    const Coef cf = load_coef(I);
+    const double nu = I.nu;
+    const double s1 = which == 0 ? cf.sk1 : cf.sw1, s2 = which == 0 ? cf.sk2 : cf.sw2;
+    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+        const int o = M.own[f], n = M.nbr[f];
+        const double Sf = M.area[f], w = M.w[f], wn = M.wn[f];
+        const double sg = blend(s1, s2, w * LD(I.f1 + o) + wn * LD(I.f1 + n));
+        const double nuEff_f = w * (nu + sg * LD(I.nut + o)) + wn * (nu + sg * LD(I.nut + n));
+        const double Df = div_by(nuEff_f * Sf, M.deltaC[f], M.rdelta[f]);
+        double mFlux;
+        if (flux) {
+            double m = (LD(I.ux + o) * w + LD(I.ux + n) * wn) * M.nx[f] + (LD(I.uy + o) * w + LD(I.uy + n) * wn) * M.ny[f];
+            if (!D2) m = m + (LD(I.uz + o) * w + LD(I.uz + n) * wn) * M.nz[f];
+            mFlux = m * Sf;
+            I.fflux[f] = mFlux;
+        } else {
+            mFlux = I.fflux[f];   // written by this thread
+        }
+        I.upper[f] = -(Df + pos_part(-mFlux));
+        I.lower[f] = -(Df + pos_part(mFlux));
+    }
+}
+template <class T>
+__device__ __noinline__ void phase_turbq_cells(T &tm, const DevMesh &M, DevInst &I, int which) {
+    const Coef cf = load_coef(I);
+    const double nu = I.nu;
+    const double s1 = which == 0 ? cf.sk1 : cf.sw1, s2 = which == 0 ? cf.sk2 : cf.sw2;
+    const double *phib = which == 0 ? I.kb : I.omb;
+    const double *phi = which == 0 ? I.k : I.om;
+    const double alpha = which == 0 ? I.S.alphaK : I.S.alphaW;
+    const double relax = which == 0 ? I.S.relaxK : I.S.relaxW, rAlpha = which == 0 ? I.S.rAlphaK : I.S.rAlphaW;
+    const double ten = 10.0 * cf.bstar;
+    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+        double diag = 0.0, src = 0.0;
+        cell_faces(M, c, [&](int f, int, bool own) { diag = diag + flip(LD((own ? I.lower : I.upper) + f), true); });
+        const double F1c = LD(I.f1 + c), nutc = LD(I.nut + c);
+        for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
+            const int b = M.cbFace[e];
+            const double Sf = M.barea[b];
+            const double sg = blend(s1, s2, F1c);
+            const double Db = div_by((nu + sg * nutc) * Sf, M.bdeltaC[b], M.brdelta[b]);
+            const double vb = LD(phib + b);
+            const double mFlux = (LD(I.ubx + b) * M.bnx[b] + LD(I.uby + b) * M.bny[b] + LD(I.ubz + b) * M.bnz[b]) * Sf;
+            if (mFlux >= 0) {
+                diag = diag + (mFlux + Db);
+                src = src + Db * vb;
+            } else {
+                diag = diag + Db;
+                src = src + (Db - mFlux) * vb;
+            }
+        }
+        const double vol = M.vol[c];
+        const double omc = LD(I.om + c), omC = smax(omc, 1e-20);
+        if (which == 0) {
+            src = src + LD(I.pk + c) * vol;
+            diag = diag + cf.bstar * omC * vol;
+        } else {
+            const double S = LD(I.smag + c), F2c = 1.0 - F1c;
+            const double lim = ten * pos_part(LD(I.k + c)) * omC / smax(nutc, 1e-30);
+            src = src + (F1c * cf.al1 + F2c * cf.al2) * smin(S * S, lim) * vol;
+            diag = diag + (F1c * cf.b1 + F2c * cf.b2) * omC * vol;
+            src = src + F2c * LD(I.cdkw + c) * vol;
+        }
+        src = src + relax * diag * LD(phi + c);
+        I.diag[c] = div_by(diag, alpha, rAlpha);
+        I.src[c] = src;
+    }
+}
+
 // gradient of one scalar into (gx, gy, gz)
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_grad1(T &tm, const DevMesh &M, const double *phi, const double *phib,
                             double *ox, double *oy, double *oz) {
     const double *P[1] = {phi};
     const double *PB[1] = {phib};
     for (int c = tm.rank(); c < M.nC; c += tm.size()) {
         double gx[1], gy[1], gz[1];
-        gg_cell<T, 1, Fast>(M, c, P, PB, gx, gy, gz);
+        gg_cell<T, 1>(M, c, P, PB, gx, gy, gz);
         ox[c] = gx[0]; oy[c] = gy[0]; oz[c] = gz[0];
     }
 }
 
 // velocity gradients (Field.hpp:232-246): g[3*i+j] = dU_i/dx_j; `which` selects
 // components (bit i) so a partially updated U only recomputes what changed
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_velgrad(T &tm, const DevMesh &M, DevInst &I, int which) {
     const double *U[3] = {I.ux, I.uy, I.uz};
     const double *UB[3] = {I.ubx, I.uby, I.ubz};
     for (int c = tm.rank(); c < M.nC; c += tm.size()) {
         if (which == 7) {
             double gx[3], gy[3], gz[3];
-            gg_cell<T, 3, Fast>(M, c, U, UB, gx, gy, gz);
+            gg_cell<T, 3>(M, c, U, UB, gx, gy, gz);
 #pragma unroll
             for (int i = 0; i < 3; ++i) { I.g[3 * i][c] = gx[i]; I.g[3 * i + 1][c] = gy[i]; I.g[3 * i + 2][c] = gz[i]; }
         } else {
@@ -191,7 +554,7 @@ __device__ __noinline__ void phase_velgrad(T &tm, const DevMesh &M, DevInst &I, 
                 const double *P[1] = {U[i]};
                 const double *PB[1] = {UB[i]};
                 double gx[1], gy[1], gz[1];
-                gg_cell<T, 1, Fast>(M, c, P, PB, gx, gy, gz);
+                gg_cell<T, 1>(M, c, P, PB, gx, gy, gz);
                 I.g[3 * i][c] = gx[0]; I.g[3 * i + 1][c] = gy[0]; I.g[3 * i + 2][c] = gz[0];
             }
         }
@@ -200,7 +563,7 @@ __device__ __noinline__ void phase_velgrad(T &tm, const DevMesh &M, DevInst &I, 
 
 // SSTModel::computeFields + frozen |S| + startup floor (SIMPLESolver.cpp:736-768).
 // Requires velocity gradients in I.g.  nutMin < 0 skips the floor.
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_sst(T &tm, const DevMesh &M, DevInst &I, double nutMin) {
     const Coef cf = load_coef(I);
     const double nu = I.nu;
@@ -213,33 +576,17 @@ __device__ __noinline__ void phase_sst(T &tm, const DevMesh &M, DevInst &I, doub
         double S23 = 0.5 * (LD(I.g[5] + c) + LD(I.g[7] + c));
         double Sc = sqrt(2.0 * (S11 * S11 + S22 * S22 + S33 * S33 + 2.0 * (S12 * S12 + S13 * S13 + S23 * S23)));
         double gx[2], gy[2], gz[2];
-        gg_cell<T, 2, Fast>(M, c, P, PB, gx, gy, gz);
+        gg_cell<T, 2>(M, c, P, PB, gx, gy, gz);
         double kc = smax(LD(I.k + c), 0.0);
         double wc = smax(LD(I.om + c), 1e-20);
         double y = smax(M.wd[c], 1e-20);
-        if (Fast) {
-            const SstCell r = sst_cell_fast(cf, kc, wc, y, nu, Sc, gx[0] * gx[1] + gy[0] * gy[1] + gz[0] * gz[1]);
-            I.smag[c] = Sc;
-            I.cdkw[c] = r.CDkw;
-            I.f1[c] = r.F1;
-            I.f2[c] = r.F2;
-            I.pk[c] = r.Pk;
-            I.nut[c] = (nutMin < 0.0) ? r.nuT : smax(r.nuT, nutMin);
-            continue;
-        }
-        double omSafe = smax(wc, 1e-20);
-        double CDkw = 2.0 * cf.sw2 / omSafe * (gx[0] * gx[1] + gy[0] * gy[1] + gz[0] * gz[1]);
-        double CDpos = smax(CDkw, 1e-20);
-        double F1 = (cf.variant == 2) ? 1.0 : sst_F1(cf, kc, wc, y, nu, CDpos);
-        double F2 = sst_F2(cf, kc, wc, y, nu);
-        double nuT = sst_nut(cf, kc, wc, Sc, F2);
-        double Pk = sst_Pk(cf, nuT, Sc, kc, wc);
+        const SstCell r = sst_cell_fast(cf, kc, wc, y, nu, Sc, gx[0] * gx[1] + gy[0] * gy[1] + gz[0] * gz[1]);
         I.smag[c] = Sc;
-        I.cdkw[c] = CDkw;
-        I.f1[c] = F1;
-        I.f2[c] = F2;
-        I.pk[c] = Pk;
-        I.nut[c] = (nutMin < 0.0) ? nuT : smax(nuT, nutMin);
+        I.cdkw[c] = r.CDkw;
+        I.f1[c] = r.F1;
+        I.f2[c] = r.F2;
+        I.pk[c] = r.Pk;
+        I.nut[c] = (nutMin < 0.0) ? r.nuT : smax(r.nuT, nutMin);
     }
 }
 
@@ -248,18 +595,18 @@ __device__ __noinline__ void phase_sst(T &tm, const DevMesh &M, DevInst &I, doub
 // ---------------------------------------------------------------------------
 // Face pass of the momentum system: upper/lower coefficients and the
 // transpose-stress flux of component `comp` (StressOperators.hpp:331-340).
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_mom_faces(T &tm, const DevMesh &M, DevInst &I, int comp) {
     const double nu = I.nu;
     const double *gc0 = I.g[comp], *gc1 = I.g[3 + comp], *gc2 = I.g[6 + comp];
     for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
-        const double Sf = M.area[f], delta = M.deltaC[f], w = M.w[f];
+        const double Sf = M.area[f], w = M.w[f];
         const double nuo = LD(I.nut + o), nun = LD(I.nut + n);
         double nuEff_o = nu + nuo;
         double nuEff_n = nu + nun;
         double nuEff_f = w * nuEff_o + (1.0 - w) * nuEff_n;
-        double Df = Fast ? nuEff_f * M.aOverD[f] : nuEff_f * Sf / delta;
+        double Df = nuEff_f * M.aOverD[f];
         double Ufx = LD(I.ux + o) * w + LD(I.ux + n) * (1.0 - w);
         double Ufy = LD(I.uy + o) * w + LD(I.uy + n) * (1.0 - w);
         double Ufz = LD(I.uz + o) * w + LD(I.uz + n) * (1.0 - w);
@@ -356,7 +703,7 @@ __device__ __noinline__ void phase_inj(T &tm, const DevMesh &M, DevInst &I, cons
 }
 
 // Cell pass of the momentum system (diag, source, relaxation).
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_mom_cells(T &tm, const DevMesh &M, DevInst &I, int comp) {
     const double nu = I.nu;
     const double alphaU = I.S.alphaU;
@@ -383,9 +730,9 @@ __device__ __noinline__ void phase_mom_cells(T &tm, const DevMesh &M, DevInst &I
         const double nutc = LD(I.nut + c);
         for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
             const int b = M.cbFace[e];
-            const double Sf = M.barea[b], delta = M.bdeltaC[b];
+            const double Sf = M.barea[b];
             double nuEff = (M.bwall[b] && !wallFn) ? nu : nu + nutc;
-            double Db = Fast ? nuEff * M.baOverD[b] : nuEff * Sf / delta;
+            double Db = nuEff * M.baOverD[b];
             double Ub = LD(Ubc + b);
             double mFlux = (LD(I.ubx + b) * M.bnx[b] + LD(I.uby + b) * M.bny[b] + LD(I.ubz + b) * M.bnz[b]) * Sf;
             if (mFlux >= 0) {
@@ -410,13 +757,8 @@ __device__ __noinline__ void phase_mom_cells(T &tm, const DevMesh &M, DevInst &I
         src = src + ts;
         if (I.inj) src = src + LD(I.inj + (size_t)comp * M.nC + c);
         const double phi_old = LD(Uc + c);
-        if (Fast) {
-            src = src + relaxSrc * diag * phi_old;
-            diag = diag * relaxDiag;
-        } else {
-            src = src + (1.0 - alphaU) / alphaU * diag * phi_old;
-            diag = diag / alphaU;
-        }
+        src = src + relaxSrc * diag * phi_old;
+        diag = diag * relaxDiag;
         I.diag[c] = diag;
         I.src[c] = src;
         if (comp == 0) I.aPx[c] = diag;
@@ -482,20 +824,20 @@ __device__ __noinline__ void phase_p_cells(T &tm, const DevMesh &M, DevInst &I) 
 }
 
 // k (which = 0) or omega (which = 1) face pass
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_turb_faces(T &tm, const DevMesh &M, DevInst &I, int which) {
     const Coef cf = load_coef(I);
     const double nu = I.nu;
     const double s1 = which == 0 ? cf.sk1 : cf.sw1, s2 = which == 0 ? cf.sk2 : cf.sw2;
     for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
-        const double Sf = M.area[f], delta = M.deltaC[f], w = M.w[f];
+        const double Sf = M.area[f], w = M.w[f];
         double F1_f = w * LD(I.f1 + o) + (1.0 - w) * LD(I.f1 + n);
         double sg = blend(s1, s2, F1_f);
         double nuEff_o = nu + sg * LD(I.nut + o);
         double nuEff_n = nu + sg * LD(I.nut + n);
         double nuEff_f = w * nuEff_o + (1.0 - w) * nuEff_n;
-        double Df = Fast ? nuEff_f * M.aOverD[f] : nuEff_f * Sf / delta;
+        double Df = nuEff_f * M.aOverD[f];
         double Ufx = LD(I.ux + o) * w + LD(I.ux + n) * (1.0 - w);
         double Ufy = LD(I.uy + o) * w + LD(I.uy + n) * (1.0 - w);
         double Ufz = LD(I.uz + o) * w + LD(I.uz + n) * (1.0 - w);
@@ -507,7 +849,7 @@ __device__ __noinline__ void phase_turb_faces(T &tm, const DevMesh &M, DevInst &
     }
 }
 
-template <class T, bool Fast = false>
+template <class T>
 __device__ __noinline__ void phase_turb_cells(T &tm, const DevMesh &M, DevInst &I, int which) {
     const Coef cf = load_coef(I);
     const double nu = I.nu;
@@ -526,10 +868,10 @@ __device__ __noinline__ void phase_turb_cells(T &tm, const DevMesh &M, DevInst &
         const double F1c = LD(I.f1 + c), nutc = LD(I.nut + c);
         for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
             const int b = M.cbFace[e];
-            const double Sf = M.barea[b], delta = M.bdeltaC[b];
+            const double Sf = M.barea[b];
             double sg = blend(s1, s2, F1c);
             double nuEff = nu + sg * nutc;
-            double Db = Fast ? nuEff * M.baOverD[b] : nuEff * Sf / delta;
+            double Db = nuEff * M.baOverD[b];
             double vb = LD(phib + b);
             double mFlux = (LD(I.ubx + b) * M.bnx[b] + LD(I.uby + b) * M.bny[b] + LD(I.ubz + b) * M.bnz[b]) * Sf;
             if (mFlux >= 0) {
@@ -555,13 +897,8 @@ __device__ __noinline__ void phase_turb_cells(T &tm, const DevMesh &M, DevInst &
             diag = diag + betaB * omC * vol;
             src = src + (1.0 - F1c) * LD(I.cdkw + c) * vol;
         }
-        if (Fast) {
-            src = src + relaxSrc * diag * LD(phi + c);
-            diag = diag * relaxDiag;
-        } else {
-            src = src + (1.0 - alpha) / alpha * diag * LD(phi + c);
-            diag = diag / alpha;
-        }
+        src = src + relaxSrc * diag * LD(phi + c);
+        diag = diag * relaxDiag;
         I.diag[c] = diag;
         I.src[c] = src;
     }
