@@ -120,7 +120,7 @@ __device__ __noinline__ bool dense_inverse_panels(T &tm, double *A, double *mult
         // panel columns; then the pivot rows' columns outside the panel, 16
         // lanes hold a column's panel rows.  Two of each to a warp.
         const int nOut = n - b, units = (nOut + 1) >> 1;
-        for (int u = tm.rank() >> 5; u < 2 * units; u += tm.size() >> 5) {
+        for (int u = tm.spread() >> 5; u < 2 * units; u += tm.size() >> 5) {
             const bool rows = u < units;
             const int q = 2 * (rows ? u : u - units) + half;
             const bool on = q < nOut && l < b;

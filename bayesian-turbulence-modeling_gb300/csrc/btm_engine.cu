@@ -56,7 +56,7 @@ __device__ void amg_galerkin(T &tm, const DevMesh &M, DevInst &I, int l) {
     const AmgLevelDev &L = M.lev[l];
     const double *fine = lev_vals(I, M, l - 1);
     double *val = lev_vals(I, M, l);
-    for (int k = tm.rank(); k < L.nnz; k += tm.size()) {
+    for (int k = tm.spread(); k < L.nnz; k += tm.size()) {
         double s = 0.0;
         for (int q = L.gOff[k]; q < L.gOff[k + 1]; ++q) s += LD(fine + L.gIdx[q]);
         val[k] = s;
@@ -69,7 +69,7 @@ __device__ void amg_level_rd(T &tm, const DevMesh &M, DevInst &I, int l) {
     const AmgLevelDev &L = M.lev[l];
     double *rd = lev_rd(I, M, l);
     const double *val = lev_vals(I, M, l);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) {
+    for (int i = tm.spread(); i < L.n; i += tm.size()) {
         double d;
         if (l == 0) d = LD(I.diag + i);
         else d = L.diagPos[i] >= 0 ? LD(val + L.diagPos[i]) : 0.0;
@@ -88,7 +88,7 @@ __device__ __noinline__ void amg_coarse_inverse_sweep(T &tm, const DevMesh &M, D
     const int n = L.n, w2 = 2 * n;
     double *A = I.gj, *B = I.gj + (size_t)n * w2;
     const double *val = lev_vals(I, M, l);
-    for (int i = tm.rank(); i < n; i += tm.size()) {
+    for (int i = tm.spread(); i < n; i += tm.size()) {
         double *row = A + (size_t)i * w2;
         for (int j = 0; j < w2; ++j) row[j] = 0.0;
         if (l == 0) {
@@ -108,7 +108,7 @@ __device__ __noinline__ void amg_coarse_inverse_sweep(T &tm, const DevMesh &M, D
         const double piv = LD(A + (size_t)k * w2 + k);
         const bool skip = !(fabs(piv) > 1e-300);
         const double rp = skip ? 0.0 : 1.0 / piv;
-        for (int idx = tm.rank(); idx < n * w2; idx += tm.size()) {
+        for (int idx = tm.spread(); idx < n * w2; idx += tm.size()) {
             const int i = idx / w2, j = idx - i * w2;
             const double akj = LD(A + (size_t)k * w2 + j) * rp;
             double v = LD(A + idx);
@@ -121,7 +121,7 @@ __device__ __noinline__ void amg_coarse_inverse_sweep(T &tm, const DevMesh &M, D
         tm.sync();
         double *tmp = A; A = B; B = tmp;
     }
-    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) {
+    for (int idx = tm.spread(); idx < n * n; idx += tm.size()) {
         const int i = idx / n, j = idx - i * n;
         I.ainv[idx] = LD(A + (size_t)i * w2 + n + j);
     }
@@ -134,9 +134,9 @@ __device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst
     const AmgLevelDev &L = M.lev[l];
     double *A = I.ainv;
     const double *val = lev_vals(I, M, l);
-    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
+    for (int idx = tm.spread(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
     tm.sync();
-    for (int i = tm.rank(); i < n; i += tm.size()) {
+    for (int i = tm.spread(); i < n; i += tm.size()) {
         double *row = A + (size_t)i * n;
         if (l == 0) {
             row[i] = LD(I.diag + i);  // level 0 as coarsest: LDU rows
@@ -166,7 +166,7 @@ __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, i
     const double *rd = lev_rd(I, M, l);
     for (int cc = 0; cc < L.nColors; ++cc) {
         const int col = reverse ? L.nColors - 1 - cc : cc;
-        for (int q = L.colorOff[col] + tm.rank(); q < L.colorOff[col + 1]; q += tm.size()) {
+        for (int q = L.colorOff[col] + tm.spread(); q < L.colorOff[col + 1]; q += tm.size()) {
             const int i = L.colorRows[q];
             const double ri = LD(rd + i);
             if (ri == 0.0) continue;
@@ -179,13 +179,19 @@ __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, i
     }
 }
 
-// residual of level l and restriction into level l+1 (x_{l+1} = 0)
+// Residual of level l and restriction into level l+1 (x_{l+1} = 0); with `smooth`
+// also the first damped-Jacobi sweep of level l + 1, which starts from zero and
+// needs no neighbours, into that level's r (its x is not read before the second
+// sweep writes it).  Two passes: one over the coarse rows, each forming its
+// members' residuals in turn, leaves most lanes waiting for the row with the
+// most members (123k-cell step: 10 % slower).
+constexpr double kJacobiWeight64 = 0.7;
 template <class T>
-__device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, int l) {
+__device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, int l, bool smooth = false) {
     const AmgLevelDev &L = M.lev[l];
     const double *x = lev_x(I, M, l), *b = lev_b(I, M, l), *val = lev_vals(I, M, l);
     double *r = lev_r(I, M, l);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) {
+    for (int i = tm.spread(); i < L.n; i += tm.size()) {
         double s;
         if (l == 0) {
             s = ldu_row<T>(M, I, x, i);
@@ -196,12 +202,14 @@ __device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, i
     }
     tm.sync();
     const AmgLevelDev &C = M.lev[l + 1];
-    double *bc = lev_b(I, M, l + 1), *xc = lev_x(I, M, l + 1);
-    for (int J = tm.rank(); J < C.n; J += tm.size()) {
+    double *bc = lev_b(I, M, l + 1), *xc = lev_x(I, M, l + 1), *rc = lev_r(I, M, l + 1);
+    const double *rd = lev_rd(I, M, l + 1);
+    for (int J = tm.spread(); J < C.n; J += tm.size()) {
         double s = 0.0;
         for (int q = L.aggOff[J]; q < L.aggOff[J + 1]; ++q) s += LD(r + L.aggMem[q]);
         bc[J] = s;
-        xc[J] = 0.0;
+        if (smooth) rc[J] = fma(kJacobiWeight64 * LD(rd + J), s, 0.0);
+        else xc[J] = 0.0;
     }
     tm.sync();
 }
@@ -211,25 +219,38 @@ __device__ void amg_prolong(T &tm, const DevMesh &M, DevInst &I, int l) {
     const AmgLevelDev &L = M.lev[l];
     double *x = lev_x(I, M, l);
     const double *xc = lev_x(I, M, l + 1);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) x[i] = LD(x + i) + LD(xc + L.map[i]);
+    for (int i = tm.spread(); i < L.n; i += tm.size()) x[i] = LD(x + i) + LD(xc + L.map[i]);
     tm.sync();
+}
+
+// The correction v of row J of level l to the members of its aggregate on the
+// finer level: the prolongation of that row (every finer row has one aggregate).
+__device__ __forceinline__ void amg_add_up(const DevMesh &M, DevInst &I, int l, int J, double v, int first, int step) {
+    const AmgLevelDev &F = M.lev[l - 1];
+    double *x = lev_x(I, M, l - 1);
+    for (int q = F.aggOff[J] + first; q < F.aggOff[J + 1]; q += step) {
+        const int m = F.aggMem[q];
+        x[m] = __ldcg(x + m) + v;
+    }
 }
 
 // grid-size dense coarsest inverse (up to kCoarseDirectGrid rows): one warp
 // per row, lane-strided partial sums folded by a butterfly
+// (with `up`, the row's correction goes straight to the members of its aggregate)
 template <class T>
-__device__ __noinline__ void amg_coarse_dense_warp(T &tm, const DevMesh &M, DevInst &I) {
+__device__ __noinline__ void amg_coarse_dense_warp(T &tm, const DevMesh &M, DevInst &I, bool up) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
     const double *b = lev_b(I, M, l);
     double *x = lev_x(I, M, l);
-    const int lane = tm.rank() & 31;
-    for (int i = tm.rank() >> 5; i < n; i += tm.size() >> 5) {
+    const int lane = tm.spread() & 31;
+    for (int i = tm.spread() >> 5; i < n; i += tm.size() >> 5) {
         const double *row = I.ainv + (size_t)i * n;
         double s = 0.0;
         for (int j = lane; j < n; j += 32) s = fma(LD(row + j), LD(b + j), s);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) x[i] = s;
+        if (up) amg_add_up(M, I, l, i, s, lane, 32);
+        else if (lane == 0) x[i] = s;
     }
     tm.sync();
 }
@@ -239,11 +260,11 @@ __device__ void amg_coarse_solve(T &tm, const DevMesh &M, DevInst &I) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
     if (M.coarseDirect && n > kCoarseDirect) {
-        amg_coarse_dense_warp(tm, M, I);
+        amg_coarse_dense_warp(tm, M, I, false);
     } else if (M.coarseDirect) {
         const double *b = lev_b(I, M, l);
         double *x = lev_x(I, M, l);
-        for (int i = tm.rank(); i < n; i += tm.size()) {
+        for (int i = tm.spread(); i < n; i += tm.size()) {
             double s = 0.0;
             for (int j = 0; j < n; ++j) s = fma(LD(I.ainv + (size_t)i * n + j), LD(b + j), s);
             x[i] = s;
@@ -255,51 +276,74 @@ __device__ void amg_coarse_solve(T &tm, const DevMesh &M, DevInst &I) {
 }
 
 // one damped-Jacobi sweep on a coarse level (l >= 1): reads x, writes `out`
-constexpr double kJacobiWeight64 = 0.7;
 template <class T>
-__device__ __noinline__ void amg_jacobi(T &tm, const DevMesh &M, DevInst &I, int l, const double *x, double *out) {
+__device__ __noinline__ void amg_jacobi(T &tm, const DevMesh &M, DevInst &I, int l, const double *x, double *out,
+                                        bool up = false) {
     const AmgLevelDev &L = M.lev[l];
     const double *b = lev_b(I, M, l), *val = lev_vals(I, M, l), *rd = lev_rd(I, M, l);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) {
+    for (int i = tm.spread(); i < L.n; i += tm.size()) {
         const double s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
-        out[i] = fma(kJacobiWeight64 * LD(rd + i), s, LD(x + i));
+        const double v = fma(kJacobiWeight64 * LD(rd + i), s, LD(x + i));
+        if (up) amg_add_up(M, I, l, i, v, 0, 1);
+        else out[i] = v;
     }
     tm.sync();
 }
 
-// Two smoothing sweeps of level l: multicolour Gauss-Seidel (colours
-// ascending before the coarse correction, descending after).  On the
-// cooperative grid the coarse levels take a pair of damped-Jacobi sweeps
-// (x -> r -> x) instead: one grid barrier per sweep rather than one per
-// colour (6-11 colours on Galerkin levels), for ~15-20 % more PCG iterations.
+// On the cooperative grid the coarse levels take a pair of damped-Jacobi
+// sweeps (x -> r -> x) instead of two multicolour Gauss-Seidel sweeps: one grid
+// barrier per sweep rather than one per colour (6-11 colours on Galerkin
+// levels), for ~15-20 % more PCG iterations.
 template <class T> struct GridSmoothing { static constexpr bool jacobi = false; };
 template <> struct GridSmoothing<GridTeam> { static constexpr bool jacobi = true; };
 
+// V-cycle on all levels: 2 pre-sweeps (colours ascending), 2 post sweeps
+// (colours descending), symmetric so the preconditioner suits CG.
 template <class T>
-__device__ void amg_smooth2(T &tm, const DevMesh &M, DevInst &I, int l, bool post) {
-    if (l == 0 || !GridSmoothing<T>::jacobi) {
-        amg_gs_sweep(tm, M, I, l, post);
-        amg_gs_sweep(tm, M, I, l, post);
-    } else {
-        double *x = lev_x(I, M, l), *tmp = lev_r(I, M, l);
-        amg_jacobi(tm, M, I, l, x, tmp);
-        amg_jacobi(tm, M, I, l, tmp, x);
-    }
-}
-
-// V-cycle on levels [l0, nLevels): 2 pre-sweeps, 2 post sweeps, symmetric so
-// the preconditioner suits CG.
-template <class T>
-__device__ void amg_vcycle_from(T &tm, const DevMesh &M, DevInst &I, int l0) {
+__device__ void amg_vcycle_gs(T &tm, const DevMesh &M, DevInst &I) {
     const int nl = M.nLevels;
-    for (int l = l0; l < nl - 1; ++l) {
-        amg_smooth2(tm, M, I, l, false);
+    for (int l = 0; l < nl - 1; ++l) {
+        amg_gs_sweep(tm, M, I, l, false);
+        amg_gs_sweep(tm, M, I, l, false);
         amg_restrict(tm, M, I, l);
     }
     amg_coarse_solve(tm, M, I);
-    for (int l = nl - 2; l >= l0; --l) {
+    for (int l = nl - 2; l >= 0; --l) {
         amg_prolong(tm, M, I, l);
-        amg_smooth2(tm, M, I, l, true);
+        amg_gs_sweep(tm, M, I, l, true);
+        amg_gs_sweep(tm, M, I, l, true);
+    }
+}
+
+// The same with Jacobi pairs on the coarse levels, five barriers a level
+// instead of seven: the first pre-sweep is part of the finer level's
+// restriction, the prolongation part of the second post-sweep (or of the
+// coarsest solve).
+template <class T>
+__device__ void amg_vcycle_jacobi(T &tm, const DevMesh &M, DevInst &I) {
+    const int nl = M.nLevels;
+    if (nl > 1) {
+        amg_gs_sweep(tm, M, I, 0, false);
+        amg_gs_sweep(tm, M, I, 0, false);
+        amg_restrict(tm, M, I, 0, nl > 2);
+    }
+    for (int l = 1; l < nl - 1; ++l) {
+        amg_jacobi(tm, M, I, l, lev_r(I, M, l), lev_x(I, M, l));
+        amg_restrict(tm, M, I, l, l + 1 < nl - 1);
+    }
+    if (nl > 1 && M.coarseDirect && M.lev[nl - 1].n > kCoarseDirect) {
+        amg_coarse_dense_warp(tm, M, I, true);
+    } else {
+        amg_coarse_solve(tm, M, I);
+        if (nl > 1) amg_prolong(tm, M, I, nl - 2);
+    }
+    for (int l = nl - 2; l > 0; --l) {
+        amg_jacobi(tm, M, I, l, lev_x(I, M, l), lev_r(I, M, l));
+        amg_jacobi(tm, M, I, l, lev_r(I, M, l), lev_x(I, M, l), true);
+    }
+    if (nl > 1) {
+        amg_gs_sweep(tm, M, I, 0, true);
+        amg_gs_sweep(tm, M, I, 0, true);
     }
 }
 
@@ -318,7 +362,8 @@ template <class T> struct AmgDriver {
         if (M.coarseDirect) amg_coarse_inverse(tm, M, I);
     }
     __device__ static void vcycle(T &tm, const DevMesh &M, DevInst &I) {
-        amg_vcycle_from(tm, M, I, 0);
+        if constexpr (GridSmoothing<T>::jacobi) amg_vcycle_jacobi(tm, M, I);
+        else amg_vcycle_gs(tm, M, I);
     }
 };
 
@@ -922,7 +967,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block(DevInst *insts, i
         sM = *sI.M;
     }
     __syncthreads();
-    BlockTeam tm{red, 0, tot, 0};
+    BlockTeam tm{red, 0, tot, 0, live_warps(sM.nC)};
     simple_solve(tm, sM, sI);
 }
 template __global__ void k_simple_block<256>(DevInst *, int);
@@ -949,6 +994,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_simple_block_ref(DevInst *inst
     tm.buf = 0;
     tm.tot = tot;
     tm.turn = 0;
+    tm.live = live_warps(sM.nC);
     simple_solve(tm, sM, sI);
 }
 template __global__ void k_simple_block_ref<256>(DevInst *, int, int);
@@ -985,6 +1031,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_debug(DevInst *inst) {
     tm.buf = 0;
     tm.tot = tot;
     tm.turn = 0;
+    tm.live = live_warps(sM.nC);
     const DevMesh &M = sM;
     DevInst &I = sI;
     const int ph = I.dbgPhase, arg = I.dbgArg;

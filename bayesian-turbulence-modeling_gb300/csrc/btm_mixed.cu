@@ -144,7 +144,7 @@ __device__ __noinline__ void mx_velgrad(T &tm, const DevMesh &M, DevInst &I, int
     DevWork32 &F = I.f;
     const double *U[3] = {I.ux, I.uy, I.uz};
     const double *UB[3] = {I.ubx, I.uby, I.ubz};
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         if (which == 7) {
             float gx[3], gy[3], gz[3];
             ggd_cell<T, 3, double>(M, c, U, UB, gx, gy, gz);
@@ -173,7 +173,7 @@ __device__ __noinline__ void mx_pgrad(T &tm, const DevMesh &M, DevInst &I) {
     DevWork32 &F = I.f;
     const double *P[1] = {I.p};
     const double *PB[1] = {I.pb};
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         float gx[1], gy[1], gz[1];
         ggd_cell<T, 1, double>(M, c, P, PB, gx, gy, gz);
         F.gp[0][c] = gx[0]; F.gp[1][c] = gy[0]; F.gp[2][c] = gz[0];
@@ -188,7 +188,7 @@ __device__ __noinline__ void mx_sst(T &tm, const DevMesh &M, DevInst &I, float n
     DevWork32 &F = I.f;
     const double *P[2] = {I.k, I.om};
     const double *PB[2] = {I.kb, I.omb};
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         float S11 = F.g[0][c], S22 = F.g[4][c], S33 = F.g[8][c];
         float S12 = 0.5f * (F.g[1][c] + F.g[3][c]);
         float S13 = 0.5f * (F.g[2][c] + F.g[6][c]);
@@ -276,7 +276,7 @@ __device__ __noinline__ void mx_mom_faces(T &tm, const DevMesh &M, DevInst &I, i
     const float nu = (float)I.nu;
     const bool z = I.solveZ != 0;
     const float *gc0 = F.g[comp], *gc1 = F.g[3 + comp], *gc2 = F.g[6 + comp];
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         float w, wn;
         int o, n;
         cd_face<T>(M, I, f, nu, -1.0f, 0.0f, true, z, w, wn, o, n);
@@ -380,7 +380,7 @@ __device__ __noinline__ void mx_p_faces(T &tm, const DevMesh &M, DevInst &I) {
     DevWork32 &F = I.f;
     const bool rc = M.rhieChow != 0;
     const bool z = I.solveZ != 0;
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
         const float Sf = G.area[f], w = G.w[f], wn = 1.0f - w;
         const float aPo = LD(F.aPx + o), aPn = LD(F.aPx + n);
@@ -446,7 +446,7 @@ __device__ __noinline__ void mx_turb_faces(T &tm, const DevMesh &M, DevInst &I, 
     const float nu = (float)I.nu;
     const float s1 = which == 0 ? cf.sk1 : cf.sw1, s2 = which == 0 ? cf.sk2 : cf.sw2;
     const bool z = I.solveZ != 0;
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         float w, wn;
         int o, n;
         cd_face<T>(M, I, f, nu, s1, s2, which == 0, z, w, wn, o, n);
@@ -527,11 +527,14 @@ __device__ __noinline__ SolveResF mx_bicgstab(T &tm, const DevMesh &M, DevWork32
                                               int maxIter, float tol) {
     SolveResF res = {0, 0.0f, 0};
     const int nC = M.nC;
+    const RowTab rows(M);
+    const float *sys = F.diag, *src = F.src;
+    float *r = F.r, *rh = F.rh, *pv = F.pv, *v = F.v, *s = F.s, *t = F.t, *ph = F.ph, *sh = F.sh, *rd = F.rd;
     float a0[1] = {0.0f};
     for (int c = tm.rank(); c < nC; c += tm.size()) {
-        const float rc = LD(F.src + c) * scale;
-        F.r[c] = rc; F.rh[c] = rc; F.pv[c] = 0.0f; F.v[c] = 0.0f;
-        F.rd[c] = jac_rdf(LD(F.diag + c));
+        const float rc = LD(src + c) * scale;
+        r[c] = rc; rh[c] = rc; pv[c] = 0.0f; v[c] = 0.0f;
+        rd[c] = jac_rdf(LD(sys + c));
         x[c] = 0.0f;
         a0[0] = fmaf(rc, rc, a0[0]);
     }
@@ -545,16 +548,16 @@ __device__ __noinline__ SolveResF mx_bicgstab(T &tm, const DevMesh &M, DevWork32
         if (fabsf(rhoN) < 1e-30f) break;
         const float beta = (rhoN / (rho + 1e-30f)) * (alpha / (omega + 1e-30f));
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            const float p = fmaf(beta, fmaf(-omega, LD(F.v + c), LD(F.pv + c)), LD(F.r + c));
-            F.pv[c] = p;
-            F.ph[c] = p * LD(F.rd + c);
+            const float p = fmaf(beta, fmaf(-omega, LD(v + c), LD(pv + c)), LD(r + c));
+            pv[c] = p;
+            ph[c] = p * LD(rd + c);
         }
         tm.sync();
         float a1[1] = {0.0f};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            const float vc = ldu_rowf<T>(M, F, F.ph, c);
-            F.v[c] = vc;
-            a1[0] = fmaf(LD(F.rh + c), vc, a1[0]);
+            const float vc = ldu_off<T, false>(rows, sys, (const float *)ph, c, LD(sys + c) * LD(ph + c));
+            v[c] = vc;
+            a1[0] = fmaf(LD(rh + c), vc, a1[0]);
         }
         tm.template sumf<1>(a1);
         const float rv = a1[0];
@@ -562,35 +565,35 @@ __device__ __noinline__ SolveResF mx_bicgstab(T &tm, const DevMesh &M, DevWork32
         alpha = rhoN / rv;
         float a2[1] = {0.0f};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            const float sc = fmaf(-alpha, LD(F.v + c), LD(F.r + c));
-            F.s[c] = sc;
-            F.sh[c] = sc * LD(F.rd + c);
+            const float sc = fmaf(-alpha, LD(v + c), LD(r + c));
+            s[c] = sc;
+            sh[c] = sc * LD(rd + c);
             a2[0] = fmaf(sc, sc, a2[0]);
         }
         tm.template sumf<1>(a2);
         const float sn = sqrtf(a2[0]);
         if (sn / r0 < tol) {
-            for (int c = tm.rank(); c < nC; c += tm.size()) x[c] = fmaf(alpha, LD(F.ph + c), x[c]);
+            for (int c = tm.rank(); c < nC; c += tm.size()) x[c] = fmaf(alpha, LD(ph + c), x[c]);
             res.iterations = it + 1; res.finalRes = sn / r0; res.converged = 1;
             return res;
         }
         float a3[2] = {0.0f, 0.0f};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            const float tc = ldu_rowf<T>(M, F, F.sh, c);
-            F.t[c] = tc;
+            const float tc = ldu_off<T, false>(rows, sys, (const float *)sh, c, LD(sys + c) * LD(sh + c));
+            t[c] = tc;
             a3[0] = fmaf(tc, tc, a3[0]);
-            a3[1] = fmaf(tc, LD(F.s + c), a3[1]);
+            a3[1] = fmaf(tc, LD(s + c), a3[1]);
         }
         tm.template sumf<2>(a3);
         const float tt = a3[0];
         omega = (tt > 1e-30f) ? a3[1] / tt : 0.0f;
         float a4[2] = {0.0f, 0.0f};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            x[c] = x[c] + fmaf(alpha, LD(F.ph + c), omega * LD(F.sh + c));
-            const float rc = fmaf(-omega, LD(F.t + c), LD(F.s + c));
-            F.r[c] = rc;
+            x[c] = x[c] + fmaf(alpha, LD(ph + c), omega * LD(sh + c));
+            const float rc = fmaf(-omega, LD(t + c), LD(s + c));
+            r[c] = rc;
             a4[0] = fmaf(rc, rc, a4[0]);
-            a4[1] = fmaf(LD(F.rh + c), rc, a4[1]);
+            a4[1] = fmaf(LD(rh + c), rc, a4[1]);
         }
         tm.template sumf<2>(a4);
         const float rn = sqrtf(a4[0]);
@@ -626,7 +629,7 @@ __device__ void mx_amg_galerkin(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     const AmgLevelDev &L = M.lev[l];
     const float *fine = lev_valsf(F, M, l - 1);
     float *val = lev_valsf(F, M, l);
-    for (int k = tm.rank(); k < L.nnz; k += tm.size()) {
+    for (int k = tm.spread(); k < L.nnz; k += tm.size()) {
         float s = 0.0f;
         for (int q = L.gOff[k]; q < L.gOff[k + 1]; ++q) s += LD(fine + L.gIdx[q]);
         val[k] = s;
@@ -638,7 +641,7 @@ __device__ void mx_amg_level_rd(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     const AmgLevelDev &L = M.lev[l];
     float *rd = lev_rdf(F, M, l);
     const float *val = lev_valsf(F, M, l);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) {
+    for (int i = tm.spread(); i < L.n; i += tm.size()) {
         float d;
         if (l == 0) d = LD(F.diag + i);
         else d = L.diagPos[i] >= 0 ? LD(val + L.diagPos[i]) : 0.0f;
@@ -659,7 +662,7 @@ __device__ __noinline__ void mx_amg_coarse_inverse_sweep(T &tm, const DevMesh &M
     const int n = L.n, w2 = 2 * n;
     double *A = F.gj, *B = F.gj + (size_t)n * w2;
     const float *val = lev_valsf(F, M, l);
-    for (int i = tm.rank(); i < n; i += tm.size()) {
+    for (int i = tm.spread(); i < n; i += tm.size()) {
         double *row = A + (size_t)i * w2;
         for (int j = 0; j < w2; ++j) row[j] = 0.0;
         if (l == 0) {
@@ -679,7 +682,7 @@ __device__ __noinline__ void mx_amg_coarse_inverse_sweep(T &tm, const DevMesh &M
         const double piv = LD(A + (size_t)k * w2 + k);
         const bool skip = !(fabs(piv) > 1e-300);
         const double rp = skip ? 0.0 : 1.0 / piv;
-        for (int idx = tm.rank(); idx < n * w2; idx += tm.size()) {
+        for (int idx = tm.spread(); idx < n * w2; idx += tm.size()) {
             const int i = idx / w2, j = idx - i * w2;
             const double akj = LD(A + (size_t)k * w2 + j) * rp;
             double v = LD(A + idx);
@@ -692,7 +695,7 @@ __device__ __noinline__ void mx_amg_coarse_inverse_sweep(T &tm, const DevMesh &M
         tm.sync();
         double *tmp = A; A = B; B = tmp;
     }
-    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) {
+    for (int idx = tm.spread(); idx < n * n; idx += tm.size()) {
         const int i = idx / n, j = idx - i * n;
         F.ainv[idx] = LD(A + (size_t)i * w2 + n + j);
     }
@@ -705,9 +708,9 @@ __device__ __noinline__ void mx_amg_coarse_inverse(T &tm, const DevMesh &M, DevW
     const AmgLevelDev &L = M.lev[l];
     double *A = F.ainv;
     const float *val = lev_valsf(F, M, l);
-    for (int idx = tm.rank(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
+    for (int idx = tm.spread(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
     tm.sync();
-    for (int i = tm.rank(); i < n; i += tm.size()) {
+    for (int i = tm.spread(); i < n; i += tm.size()) {
         double *row = A + (size_t)i * n;
         if (l == 0) {
             row[i] = LD(F.diag + i);
@@ -736,7 +739,7 @@ __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 
     const float *rd = lev_rdf(F, M, l);
     for (int cc = 0; cc < L.nColors; ++cc) {
         const int col = reverse ? L.nColors - 1 - cc : cc;
-        for (int q = L.colorOff[col] + tm.rank(); q < L.colorOff[col + 1]; q += tm.size()) {
+        for (int q = L.colorOff[col] + tm.spread(); q < L.colorOff[col + 1]; q += tm.size()) {
             const int i = L.colorRows[q];
             const float ri = LD(rd + i);
             if (ri == 0.0f) continue;
@@ -749,32 +752,52 @@ __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 
     }
 }
 
-// residual of level l restricted into level l+1 in one pass (x_{l+1} = 0):
-// each coarse row sums b - A x over its aggregate's members, and every fine
-// row belongs to exactly one aggregate
+// The correction v of row J of level l to the members of its aggregate on the
+// finer level: the prolongation of that row.
+template <class T>
+__device__ __forceinline__ void mx_amg_add_up(const DevMesh &M, DevWork32 &F, int l, int J, float v, int first,
+                                              int step) {
+    const AmgLevelDev &L = M.lev[l - 1];
+    float *x = lev_xf(F, M, l - 1);
+    for (int q = L.aggOff[J] + first; q < L.aggOff[J + 1]; q += step) {
+        const int m = L.aggMem[q];
+        x[m] = LD(x + m) + v;
+    }
+}
+
 // one damped-Jacobi sweep on a coarse level (l >= 1): reads x, writes `out`
 // (the V-cycle ping-pongs between the level's x and r arrays)
 constexpr float kJacobiWeight = 0.7f;
+// (`up`: the result is the level's last, and goes to the finer level instead)
 template <class T>
-__device__ __noinline__ void mx_amg_jacobi(T &tm, const DevMesh &M, DevWork32 &F, int l, const float *x, float *out) {
+__device__ __noinline__ void mx_amg_jacobi(T &tm, const DevMesh &M, DevWork32 &F, int l, const float *x, float *out,
+                                           bool up = false) {
     const AmgLevelDev &L = M.lev[l];
     const float *b = lev_bf(F, M, l);
     const float *val = lev_valsf(F, M, l);
     const float *rd = lev_rdf(F, M, l);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) {
+    for (int i = tm.spread(); i < L.n; i += tm.size()) {
         const float s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
-        out[i] = fmaf(kJacobiWeight * LD(rd + i), s, LD(x + i));
+        const float v = fmaf(kJacobiWeight * LD(rd + i), s, LD(x + i));
+        if (up) mx_amg_add_up<T>(M, F, l, i, v, 0, 1);
+        else out[i] = v;
     }
     tm.sync();
 }
 
+// residual of level l restricted into level l+1 in one pass: each coarse row
+// sums b - A x over its aggregate's members, and every fine row belongs to
+// exactly one aggregate; with `smooth` also the first damped-Jacobi sweep of
+// level l + 1, which starts from zero and needs no neighbours, into that
+// level's r (x is not read before the second sweep writes it)
 template <class T>
-__device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 &F, int l) {
+__device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 &F, int l, bool smooth) {
     const AmgLevelDev &L = M.lev[l];
     const float *x = lev_xf(F, M, l), *b = lev_bf(F, M, l), *val = lev_valsf(F, M, l);
     const AmgLevelDev &C = M.lev[l + 1];
-    float *bc = lev_bf(F, M, l + 1), *xc = lev_xf(F, M, l + 1);
-    for (int J = tm.rank(); J < C.n; J += tm.size()) {
+    float *bc = lev_bf(F, M, l + 1), *xc = lev_xf(F, M, l + 1), *rc = lev_rf(F, M, l + 1);
+    const float *rdc = lev_rdf(F, M, l + 1);
+    for (int J = tm.spread(); J < C.n; J += tm.size()) {
         float acc = 0.0f;
         for (int q = L.aggOff[J]; q < L.aggOff[J + 1]; ++q) {
             const int i = L.aggMem[q];
@@ -787,7 +810,8 @@ __device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 
             acc += LD(b + i) - s;
         }
         bc[J] = acc;
-        xc[J] = 0.0f;
+        if (smooth) rc[J] = fmaf(kJacobiWeight * LD(rdc + J), acc, 0.0f);
+        else xc[J] = 0.0f;
     }
     tm.sync();
 }
@@ -797,25 +821,27 @@ __device__ void mx_amg_prolong(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     const AmgLevelDev &L = M.lev[l];
     float *x = lev_xf(F, M, l);
     const float *xc = lev_xf(F, M, l + 1);
-    for (int i = tm.rank(); i < L.n; i += tm.size()) x[i] = LD(x + i) + LD(xc + L.map[i]);
+    for (int i = tm.spread(); i < L.n; i += tm.size()) x[i] = LD(x + i) + LD(xc + L.map[i]);
     tm.sync();
 }
 
 // grid-size dense coarsest inverse (up to kCoarseDirectGrid rows): one warp
 // per row, lane-strided partial sums folded by a butterfly
+// (with `up`, the row's correction goes straight to the members of its aggregate)
 template <class T>
-__device__ __noinline__ void mx_amg_coarse_dense_warp(T &tm, const DevMesh &M, DevWork32 &F) {
+__device__ __noinline__ void mx_amg_coarse_dense_warp(T &tm, const DevMesh &M, DevWork32 &F, bool up) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
     const float *b = lev_bf(F, M, l);
     float *x = lev_xf(F, M, l);
-    const int lane = tm.rank() & 31;
-    for (int i = tm.rank() >> 5; i < n; i += tm.size() >> 5) {
+    const int lane = tm.spread() & 31;
+    for (int i = tm.spread() >> 5; i < n; i += tm.size() >> 5) {
         const double *row = F.ainv + (size_t)i * n;
         double s = 0.0;
         for (int j = lane; j < n; j += 32) s = fma(LD(row + j), (double)LD(b + j), s);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) x[i] = (float)s;
+        if (up) mx_amg_add_up<T>(M, F, l, i, (float)s, lane, 32);
+        else if (lane == 0) x[i] = (float)s;
     }
     tm.sync();
 }
@@ -825,11 +851,11 @@ __device__ void mx_amg_coarse_solve(T &tm, const DevMesh &M, DevWork32 &F) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
     if (M.coarseDirect && n > kCoarseDirect) {
-        mx_amg_coarse_dense_warp(tm, M, F);
+        mx_amg_coarse_dense_warp(tm, M, F, false);
     } else if (M.coarseDirect) {
         const float *b = lev_bf(F, M, l);
         float *x = lev_xf(F, M, l);
-        for (int i = tm.rank(); i < n; i += tm.size()) {
+        for (int i = tm.spread(); i < n; i += tm.size()) {
             double s = 0.0;
             for (int j = 0; j < n; ++j) s = fma(LD(F.ainv + (size_t)i * n + j), (double)LD(b + j), s);
             x[i] = (float)s;
@@ -853,40 +879,39 @@ __device__ void mx_amg_values_from(T &tm, const DevMesh &M, DevWork32 &F, int l0
     tm.sync();
 }
 
-// symmetric V-cycle on levels [l0, nLevels): 2 pre-sweeps (colours
-// ascending), 2 post-sweeps (colours descending)
-// two smoothing sweeps of level l: multicolour Gauss-Seidel (colours
-// ascending before the coarse correction, descending after); on the coarse
-// levels a pair of damped-Jacobi sweeps (x -> r -> x) instead, which needs
-// one barrier per sweep rather than one per colour (6-11 colours on Galerkin
-// levels) and costs ~15-20 % more PCG iterations
-template <class T> struct CoarseJacobi { static constexpr bool value = false; };
-template <> struct CoarseJacobi<BlockTeam> { static constexpr bool value = true; };
-template <> struct CoarseJacobi<GridTeam> { static constexpr bool value = true; };
-
+// Symmetric V-cycle: two smoothing sweeps of level l before and after the coarse
+// correction, on level 0 multicolour Gauss-Seidel (colours ascending before,
+// descending after), on the coarse levels a pair of damped-Jacobi sweeps
+// (x -> r -> x) instead, which needs one barrier per sweep rather than one per
+// colour (6-11 colours on Galerkin levels) and costs ~15-20 % more PCG
+// iterations.  Four barriers a coarse level: the first pre-sweep is part of the
+// finer level's restriction, the prolongation part of the second post-sweep (or
+// of the coarsest solve).
 template <class T>
-__device__ void mx_amg_smooth2(T &tm, const DevMesh &M, DevWork32 &F, int l, bool post) {
-    if (l == 0 || !CoarseJacobi<T>::value) {
-        mx_amg_gs_sweep(tm, M, F, l, post);
-        mx_amg_gs_sweep(tm, M, F, l, post);
-    } else {
-        float *x = lev_xf(F, M, l), *tmp = lev_rf(F, M, l);
-        mx_amg_jacobi(tm, M, F, l, x, tmp);
-        mx_amg_jacobi(tm, M, F, l, tmp, x);
-    }
-}
-
-template <class T>
-__device__ void mx_amg_vcycle_from(T &tm, const DevMesh &M, DevWork32 &F, int l0) {
+__device__ void mx_amg_vcycle(T &tm, const DevMesh &M, DevWork32 &F) {
     const int nl = M.nLevels;
-    for (int l = l0; l < nl - 1; ++l) {
-        mx_amg_smooth2(tm, M, F, l, false);
-        mx_amg_restrict(tm, M, F, l);
+    if (nl > 1) {
+        mx_amg_gs_sweep(tm, M, F, 0, false);
+        mx_amg_gs_sweep(tm, M, F, 0, false);
+        mx_amg_restrict(tm, M, F, 0, nl > 2);
     }
-    mx_amg_coarse_solve(tm, M, F);
-    for (int l = nl - 2; l >= l0; --l) {
-        mx_amg_prolong(tm, M, F, l);
-        mx_amg_smooth2(tm, M, F, l, true);
+    for (int l = 1; l < nl - 1; ++l) {
+        mx_amg_jacobi(tm, M, F, l, lev_rf(F, M, l), lev_xf(F, M, l));
+        mx_amg_restrict(tm, M, F, l, l + 1 < nl - 1);
+    }
+    if (nl > 1 && M.coarseDirect && M.lev[nl - 1].n > kCoarseDirect) {
+        mx_amg_coarse_dense_warp(tm, M, F, true);
+    } else {
+        mx_amg_coarse_solve(tm, M, F);
+        if (nl > 1) mx_amg_prolong(tm, M, F, nl - 2);
+    }
+    for (int l = nl - 2; l > 0; --l) {
+        mx_amg_jacobi(tm, M, F, l, lev_xf(F, M, l), lev_rf(F, M, l));
+        mx_amg_jacobi(tm, M, F, l, lev_rf(F, M, l), lev_xf(F, M, l), true);
+    }
+    if (nl > 1) {
+        mx_amg_gs_sweep(tm, M, F, 0, true);
+        mx_amg_gs_sweep(tm, M, F, 0, true);
     }
 }
 
@@ -905,11 +930,6 @@ __device__ void mx_amg_setup(T &tm, const DevMesh &M, DevWork32 &F, bool coarse 
     if (!coarse) return;
     mx_amg_values_from(tm, M, F, 1);
     if (M.coarseDirect) mx_amg_coarse_inverse(tm, M, F);
-}
-
-template <class T>
-__device__ void mx_amg_vcycle(T &tm, const DevMesh &M, DevWork32 &F) {
-    mx_amg_vcycle_from(tm, M, F, 0);
 }
 
 // AMG-preconditioned CG (AMGSolver::solve, LinearSolver.hpp:602-653):
@@ -2135,7 +2155,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mixed_block(DevInst *insts, in
         for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     }
     __syncthreads();
-    BlockTeam tm{red, 0, tot, 0};
+    BlockTeam tm{red, 0, tot, 0, live_warps(sM.nC)};
     mixed_solve(tm, sM, sI);
 }
 template __global__ void k_mixed_block<256>(DevInst *, int, int);

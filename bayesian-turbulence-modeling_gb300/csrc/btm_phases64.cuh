@@ -230,7 +230,7 @@ __device__ __noinline__ void phase_grads(T &tm, const DevMesh &M, DevInst &I, in
         I.g[3 * i + 1][c] = y;
         if (!D2) I.g[3 * i + 2][c] = z;
     };
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         if ((which & 7) == 7) {
             constexpr int NU = D2 ? 2 : 3;
             const double *P[4] = {U[0], U[1], D2 ? I.p : U[2], I.p};
@@ -271,7 +271,7 @@ __device__ __noinline__ void phase_closure(T &tm, const DevMesh &M, DevInst &I, 
     const double *P[2] = {I.k, I.om};
     const double *PB[2] = {I.kb, I.omb};
     const double nu500 = 500.0 * nu, sw2x2 = 2.0 * cf.sw2, sw2x4 = 4.0 * cf.sw2, ten = 10.0 * cf.bstar;
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         const double S11 = LD(I.g[0] + c), S22 = LD(I.g[4] + c);
         const double S12 = 0.5 * (LD(I.g[1] + c) + LD(I.g[3] + c));
         double Sc;
@@ -321,7 +321,7 @@ __device__ __noinline__ void phase_momq_faces(T &tm, const DevMesh &M, DevInst &
                                               double *keepD) {
     const double nu = I.nu;
     const double *gc0 = I.g[comp], *gc1 = I.g[3 + comp], *gc2 = I.g[6 + comp];
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
         const double Sf = M.area[f], w = M.w[f], wn = M.wn[f];
         const double nuo = LD(I.nut + o), nun = LD(I.nut + n);
@@ -352,7 +352,7 @@ __device__ __noinline__ void phase_momq_cells(T &tm, const DevMesh &M, DevInst &
     const double *gp = comp == 0 ? I.gpx : (comp == 1 ? I.gpy : I.gpz);
     const double *gc0 = I.g[comp], *gc1 = I.g[3 + comp], *gc2 = I.g[6 + comp];
     const bool wallFn = I.S.useWallFn != 0;
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         double diag = 0.0, ts = 0.0, src = 0.0;
         cell_faces(M, c, [&](int f, int, bool own) {
             diag = diag + flip(LD((own ? I.lower : I.upper) + f), true);
@@ -409,7 +409,7 @@ __device__ __forceinline__ void phase_dp(T &tm, const DevMesh &M, DevInst &I) {
 template <class T, bool D2>
 __device__ __noinline__ void phase_pq_faces(T &tm, const DevMesh &M, DevInst &I) {
     const bool rc = M.rhieChow != 0;
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
         const double Sf = M.area[f], delta = M.deltaC[f], rdelta = M.rdelta[f], w = M.w[f], wn = M.wn[f];
         const double dP_f = w * LD(I.ph + o) + wn * LD(I.ph + n);
@@ -430,7 +430,7 @@ __device__ __noinline__ void phase_pq_faces(T &tm, const DevMesh &M, DevInst &I)
 }
 template <class T>
 __device__ __noinline__ void phase_pq_cells(T &tm, const DevMesh &M, DevInst &I) {
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         double diag = 0.0, src = 0.0;
         cell_faces(M, c, [&](int f, int, bool own) {
             diag = diag + flip(LD(I.upper + f), true);
@@ -457,7 +457,7 @@ __device__ __noinline__ void phase_turbq_faces(T &tm, const DevMesh &M, DevInst 
     const Coef cf = load_coef(I);
     const double nu = I.nu;
     const double s1 = which == 0 ? cf.sk1 : cf.sw1, s2 = which == 0 ? cf.sk2 : cf.sw2;
-    for (int f = tm.rank(); f < M.nIF; f += tm.size()) {
+    for (int f = tm.spread(); f < M.nIF; f += tm.size()) {
         const int o = M.own[f], n = M.nbr[f];
         const double Sf = M.area[f], w = M.w[f], wn = M.wn[f];
         const double sg = blend(s1, s2, w * LD(I.f1 + o) + wn * LD(I.f1 + n));
@@ -486,7 +486,7 @@ __device__ __noinline__ void phase_turbq_cells(T &tm, const DevMesh &M, DevInst 
     const double alpha = which == 0 ? I.S.alphaK : I.S.alphaW;
     const double relax = which == 0 ? I.S.relaxK : I.S.relaxW, rAlpha = which == 0 ? I.S.rAlphaK : I.S.rAlphaW;
     const double ten = 10.0 * cf.bstar;
-    for (int c = tm.rank(); c < M.nC; c += tm.size()) {
+    for (int c = tm.spread(); c < M.nC; c += tm.size()) {
         double diag = 0.0, src = 0.0;
         cell_faces(M, c, [&](int f, int, bool own) { diag = diag + flip(LD((own ? I.lower : I.upper) + f), true); });
         const double F1c = LD(I.f1 + c), nutc = LD(I.nut + c);
@@ -973,11 +973,14 @@ template <class T>
 __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevInst &I, double *x, int maxIter, double tol) {
     SolveResult res = {0, 0.0, 0.0, 0};
     const int nC = M.nC;
+    const RowTab rows(M);
+    const double *sys = I.diag, *src = I.src;
+    double *r = I.r, *rh = I.rh, *pv = I.pv, *v = I.v, *s = I.s, *t = I.t, *ph = I.ph, *sh = I.sh, *rd = I.rd;
     double acc[1] = {0.0};
     for (int c = tm.rank(); c < nC; c += tm.size()) {
-        double rc = LD(I.src + c) - ldu_row<T>(M, I, x, c);
-        I.r[c] = rc; I.rh[c] = rc; I.pv[c] = 0.0; I.v[c] = 0.0;
-        I.rd[c] = jac_rd(LD(I.diag + c));
+        double rc = LD(src + c) - ldu_off<T, false>(rows, sys, (const double *)x, c, LD(sys + c) * LD(x + c));
+        r[c] = rc; rh[c] = rc; pv[c] = 0.0; v[c] = 0.0;
+        rd[c] = jac_rd(LD(sys + c));
         acc[0] = fma(rc, rc, acc[0]);
     }
     double o[4];
@@ -998,16 +1001,16 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
         if (!tm.ok()) break;
         if (small) break;
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            double p = fma(beta, fma(-omega, LD(I.v + c), LD(I.pv + c)), LD(I.r + c));
-            I.pv[c] = p;
-            I.ph[c] = p * LD(I.rd + c);
+            double p = fma(beta, fma(-omega, LD(v + c), LD(pv + c)), LD(r + c));
+            pv[c] = p;
+            ph[c] = p * LD(rd + c);
         }
         tm.sync();
         double a1[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            double vc = ldu_row<T>(M, I, I.ph, c);
-            I.v[c] = vc;
-            a1[0] = fma(LD(I.rh + c), vc, a1[0]);
+            double vc = ldu_off<T, false>(rows, sys, (const double *)ph, c, LD(sys + c) * LD(ph + c));
+            v[c] = vc;
+            a1[0] = fma(LD(rh + c), vc, a1[0]);
         }
         tm.template sum_then<1, 2>(a1, o, [rhoN](int lane, double rv, double) {
             return pick(lane, flag64(fabs(rv) < 1e-30), rhoN / rv);
@@ -1016,36 +1019,36 @@ __device__ __noinline__ SolveResult team_bicgstab(T &tm, const DevMesh &M, DevIn
         const double alpha = o[1];
         double a2[1] = {0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            double sc = fma(-alpha, LD(I.v + c), LD(I.r + c));
-            I.s[c] = sc;
-            I.sh[c] = sc * LD(I.rd + c);
+            double sc = fma(-alpha, LD(v + c), LD(r + c));
+            s[c] = sc;
+            sh[c] = sc * LD(rd + c);
             a2[0] = fma(sc, sc, a2[0]);
         }
         tm.template sum_then<1, 2>(a2, o, [=](int lane, double ss, double) {
             return pick(lane, ss, flag64(residual_below(ss, limit, r0, tol)));
         });
         if (is_set(o[1])) {
-            for (int c = tm.rank(); c < nC; c += tm.size()) x[c] = fma(alpha, LD(I.ph + c), LD(x + c));
+            for (int c = tm.rank(); c < nC; c += tm.size()) x[c] = fma(alpha, LD(ph + c), LD(x + c));
             res.iterations = it + 1; res.finalSq = o[0]; res.converged = 1;
             tm.sync();
             return res;
         }
         double a3[2] = {0.0, 0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            double tc = ldu_row<T>(M, I, I.sh, c);
-            I.t[c] = tc;
+            double tc = ldu_off<T, false>(rows, sys, (const double *)sh, c, LD(sys + c) * LD(sh + c));
+            t[c] = tc;
             a3[0] = fma(tc, tc, a3[0]);
-            a3[1] = fma(tc, LD(I.s + c), a3[1]);
+            a3[1] = fma(tc, LD(s + c), a3[1]);
         }
         tm.template sum_then<2, 1>(a3, o, [](int, double tt, double ts) { return (tt > 1e-30) ? ts / tt : 0.0; });
         omega = o[0];
         double a4[2] = {0.0, 0.0};
         for (int c = tm.rank(); c < nC; c += tm.size()) {
-            x[c] = LD(x + c) + fma(alpha, LD(I.ph + c), omega * LD(I.sh + c));
-            double rc = fma(-omega, LD(I.t + c), LD(I.s + c));
-            I.r[c] = rc;
+            x[c] = LD(x + c) + fma(alpha, LD(ph + c), omega * LD(sh + c));
+            double rc = fma(-omega, LD(t + c), LD(s + c));
+            r[c] = rc;
             a4[0] = fma(rc, rc, a4[0]);
-            a4[1] = fma(LD(I.rh + c), rc, a4[1]);
+            a4[1] = fma(LD(rh + c), rc, a4[1]);
         }
         // how the iteration ends (0: on to the next, 1: converged, 2:
         // breakdown), and the next beta = (rho' / rho) (alpha / omega): the two

@@ -60,7 +60,7 @@ struct RedMax {   // smax: the first operand survives ties and NaN
 // CTA they took as long as the matrix products of a BiCGSTAB iteration.
 constexpr int kRedResults = 6;
 template <int N, class Op, int NOUT, class F>
-__device__ __forceinline__ void block_reduce(double *red, double *tot, double *v, int turn, double *out, F f) {
+__device__ __forceinline__ void block_reduce(double *red, double *tot, double *v, int turn, int live, double *out, F f) {
     static_assert((N == 1 || N == 2) && NOUT <= kRedResults, "one or two values at a time");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     double *res = tot + 2 * nw;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void block_reduce(double *red, double *tot, double *v
         if (warp == (turn & 3)) {
             const double *t = tot + (lane < N ? lane * nw : 0);
             double s = t[0];
-            for (int q = 1; q < nw; ++q) s = Op::op(s, t[q]);
+            for (int q = 1; q < live; ++q) s = Op::op(s, t[q]);
             const double t0 = __shfl_sync(0xffffffffu, s, 0), t1 = N == 2 ? __shfl_sync(0xffffffffu, s, 1) : 0.0;
             const double r = f(lane, t0, t1);
             if (lane < NOUT) res[lane] = r;
@@ -107,43 +107,47 @@ __device__ __forceinline__ void block_reduce(double *red, double *tot, double *v
     for (int j = 0; j < NOUT; ++j) out[j] = res[j];
 }
 template <int N, class Op>
-__device__ __noinline__ void block_totals(double *red, double *tot, double *v, int turn) {
-    block_reduce<N, Op, N>(red, tot, v, turn, v, [](int lane, double t0, double t1) { return lane == 0 ? t0 : t1; });
+__device__ __noinline__ void block_totals(double *red, double *tot, double *v, int turn, int live) {
+    block_reduce<N, Op, N>(red, tot, v, turn, live, v, [](int lane, double t0, double t1) { return lane == 0 ? t0 : t1; });
 }
 
+
+__device__ __forceinline__ int live_warps(int nC) { return max(1, min((int)(blockDim.x >> 5), (nC + 31) >> 5)); }
 
 struct BlockTeam {
     double *red;   // shared [max(threads, 2 * 32 * kRedSlots)]
     int buf;
     double *tot;   // shared [2 * warps + kRedResults]
     int turn;
+    int live;      // warps that own cells: the others only ever add zeros to a sum
     __device__ __forceinline__ int rank() const { return threadIdx.x; }
+    __device__ __forceinline__ int spread() const { return threadIdx.x; }
     __device__ __forceinline__ int size() const { return blockDim.x; }
     __device__ __forceinline__ bool leader() const { return threadIdx.x == 0; }
     __device__ __forceinline__ bool sync() { __syncthreads(); return true; }
     __device__ __forceinline__ bool ok() const { return true; }
 
     template <int N, class Op>
-    __device__ __forceinline__ void reduce(double *v) {
+    __device__ __forceinline__ void reduce(double *v, int warps) {
         if constexpr (N > 2) {
-            reduce<2, Op>(v);
-            reduce<N - 2, Op>(v + 2);
+            reduce<2, Op>(v, warps);
+            reduce<N - 2, Op>(v + 2, warps);
         } else {
-            block_totals<N, Op>(red, tot, v, turn++);
+            block_totals<N, Op>(red, tot, v, turn++, warps);
         }
     }
     // Sum N values over the team; every thread receives the identical totals.
     template <int N>
-    __device__ __forceinline__ void sum(double *v) { reduce<N, RedAdd>(v); }
+    __device__ __forceinline__ void sum(double *v) { reduce<N, RedAdd>(v, live); }
     template <int N>
-    __device__ __forceinline__ void maxr(double *v) { reduce<N, RedMax>(v); }
+    __device__ __forceinline__ void maxr(double *v) { reduce<N, RedMax>(v, blockDim.x >> 5); }
     template <int N>
-    __device__ __forceinline__ void sumd(double *v) { reduce<N, RedAdd>(v); }
+    __device__ __forceinline__ void sumd(double *v) { reduce<N, RedAdd>(v, live); }
     // Sums N values and leaves f(q, t0, t1) of the totals in out[q], q < NOUT,
     // in every thread; one warp evaluates f.
     template <int N, int NOUT, class F>
     __device__ __forceinline__ void sum_then(double *v, double *out, F f) {
-        block_reduce<N, RedAdd, NOUT>(red, tot, v, turn++, out, f);
+        block_reduce<N, RedAdd, NOUT>(red, tot, v, turn++, live, out, f);
     }
     // The same for warp 0's values f(lane) that need no reduction
     template <int NOUT, class F>
@@ -227,6 +231,13 @@ struct GridTeam {
     int *shAbort;           // shared flag
     unsigned int target;    // thread 0: arrivals that complete the next barrier
     __device__ __forceinline__ int rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
+    // The same ranks dealt out warp by warp over the CTAs, for passes that end
+    // in no reduction (a sum's bits depend on who owns what): with rank() a
+    // 1,257-row level runs on 3 SMs, 16 warps deep in their FP64 units, and the
+    // last pass over any array fills some SMs and leaves the others idle.
+    __device__ __forceinline__ int spread() const {
+        return (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5 | (threadIdx.x & 31));
+    }
     __device__ __forceinline__ int size() const { return gridDim.x * blockDim.x; }
     __device__ __forceinline__ bool leader() const { return blockIdx.x == 0 && threadIdx.x == 0; }
     __device__ __forceinline__ bool ok() const { return *shAbort == 0; }
@@ -429,22 +440,30 @@ template <> struct Ld<GridTeam> {
 __device__ __forceinline__ double fma_any(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fma_any(float a, float b, float c) { return fmaf(a, b, c); }
 
+// The row tables of a mesh as locals: DevMesh and DevInst live in shared memory,
+// where every store through a pointer has their fields read again.
+struct RowTab {
+    const int32_t *ent, *col;
+    int nC, width;
+    __device__ __forceinline__ explicit RowTab(const DevMesh &M)
+        : ent(M.rowEnt), col(M.rowCol), nC(M.nC), width(M.rowW) {}
+};
+
 // Off-diagonal part of row c of an LDU system `sys` = diag | upper | lower, in
 // ascending face order (entries and columns of all rows by position in the
 // row, [rowW][nC], so neighbouring threads read neighbouring words; -1: no
 // entry).
 template <class T, bool Neg, int W, class V>
-__device__ __forceinline__ V ldu_off_w(const DevMesh &M, const V *sys, const V *x, int c, V y) {
-    const int nC = M.nC, width = M.rowW;
-    for (int w0 = 0; w0 < width; w0 += W) {
+__device__ __forceinline__ V ldu_off_w(const RowTab &R, const V *sys, const V *x, int c, V y) {
+    for (int w0 = 0; w0 < R.width; w0 += W) {
         int col[W], ent[W];
         V a[W], v[W];
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            const bool in = w0 + k < width;
-            const size_t at = (size_t)(in ? w0 + k : 0) * nC + c;
-            col[k] = in ? M.rowCol[at] : -1;
-            ent[k] = M.rowEnt[at];
+            const bool in = w0 + k < R.width;
+            const size_t at = (size_t)(in ? w0 + k : 0) * R.nC + c;
+            col[k] = in ? R.col[at] : -1;
+            ent[k] = R.ent[at];
         }
 #pragma unroll
         for (int k = 0; k < W; ++k) {
@@ -458,9 +477,13 @@ __device__ __forceinline__ V ldu_off_w(const DevMesh &M, const V *sys, const V *
     return y;
 }
 template <class T, bool Neg, class V>
-__device__ __forceinline__ V ldu_off(const DevMesh &M, const V *sys, const V *x, int c, V y) {
+__device__ __forceinline__ V ldu_off(const RowTab &R, const V *sys, const V *x, int c, V y) {
     // quadrilaterals have up to 4 faces, hexahedra 6
-    return M.rowW <= 4 ? ldu_off_w<T, Neg, 4>(M, sys, x, c, y) : ldu_off_w<T, Neg, 6>(M, sys, x, c, y);
+    return R.width <= 4 ? ldu_off_w<T, Neg, 4>(R, sys, x, c, y) : ldu_off_w<T, Neg, 6>(R, sys, x, c, y);
+}
+template <class T, bool Neg, class V>
+__device__ __forceinline__ V ldu_off(const DevMesh &M, const V *sys, const V *x, int c, V y) {
+    return ldu_off<T, Neg>(RowTab(M), sys, x, c, y);
 }
 
 // Row i of a CSR level without its column `skip` (-1: all of it).
