@@ -24,6 +24,7 @@
 #include "btm_observe.cuh"
 #include "btm_ramg.cuh"
 #include "btm_dense.cuh"
+#include "btm_cycle.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -156,6 +157,25 @@ __device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst
     }
 }
 
+// the arrays of an instance for the V-cycle (btm_cycle.cuh)
+struct Cycle64 {
+    using V = double;
+    static constexpr double kWeight = 0.7;
+    const DevMesh &M;
+    DevInst &I;
+    __device__ __forceinline__ int levels() const { return M.nLevels; }
+    __device__ __forceinline__ bool direct() const { return M.coarseDirect != 0; }
+    __device__ __forceinline__ const AmgLevelDev &lev(int l) const { return M.lev[l]; }
+    __device__ __forceinline__ RowTab rows() const { return RowTab(M); }
+    __device__ __forceinline__ double *x(int l) const { return lev_x(I, M, l); }
+    __device__ __forceinline__ double *b(int l) const { return lev_b(I, M, l); }
+    __device__ __forceinline__ double *r(int l) const { return lev_r(I, M, l); }
+    __device__ __forceinline__ double *rd(int l) const { return lev_rd(I, M, l); }
+    __device__ __forceinline__ double *val(int l) const { return lev_vals(I, M, l); }
+    __device__ __forceinline__ const double *sys() const { return I.diag; }
+    __device__ __forceinline__ const double *ainv() const { return I.ainv; }
+};
+
 // one colour-ordered Gauss-Seidel sweep (forward or reverse colour order)
 template <class T>
 __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
@@ -179,15 +199,9 @@ __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, i
     }
 }
 
-// Residual of level l and restriction into level l+1 (x_{l+1} = 0); with `smooth`
-// also the first damped-Jacobi sweep of level l + 1, which starts from zero and
-// needs no neighbours, into that level's r (its x is not read before the second
-// sweep writes it).  Two passes: one over the coarse rows, each forming its
-// members' residuals in turn, leaves most lanes waiting for the row with the
-// most members (123k-cell step: 10 % slower).
-constexpr double kJacobiWeight64 = 0.7;
+// residual of level l and restriction into level l+1 (x_{l+1} = 0)
 template <class T>
-__device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, int l, bool smooth = false) {
+__device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, int l) {
     const AmgLevelDev &L = M.lev[l];
     const double *x = lev_x(I, M, l), *b = lev_b(I, M, l), *val = lev_vals(I, M, l);
     double *r = lev_r(I, M, l);
@@ -202,14 +216,12 @@ __device__ __noinline__ void amg_restrict(T &tm, const DevMesh &M, DevInst &I, i
     }
     tm.sync();
     const AmgLevelDev &C = M.lev[l + 1];
-    double *bc = lev_b(I, M, l + 1), *xc = lev_x(I, M, l + 1), *rc = lev_r(I, M, l + 1);
-    const double *rd = lev_rd(I, M, l + 1);
+    double *bc = lev_b(I, M, l + 1), *xc = lev_x(I, M, l + 1);
     for (int J = tm.spread(); J < C.n; J += tm.size()) {
         double s = 0.0;
         for (int q = L.aggOff[J]; q < L.aggOff[J + 1]; ++q) s += LD(r + L.aggMem[q]);
         bc[J] = s;
-        if (smooth) rc[J] = fma(kJacobiWeight64 * LD(rd + J), s, 0.0);
-        else xc[J] = 0.0;
+        xc[J] = 0.0;
     }
     tm.sync();
 }
@@ -223,48 +235,14 @@ __device__ void amg_prolong(T &tm, const DevMesh &M, DevInst &I, int l) {
     tm.sync();
 }
 
-// The correction v of row J of level l to the members of its aggregate on the
-// finer level: the prolongation of that row (every finer row has one aggregate).
-__device__ __forceinline__ void amg_add_up(const DevMesh &M, DevInst &I, int l, int J, double v, int first, int step) {
-    const AmgLevelDev &F = M.lev[l - 1];
-    double *x = lev_x(I, M, l - 1);
-    for (int q = F.aggOff[J] + first; q < F.aggOff[J + 1]; q += step) {
-        const int m = F.aggMem[q];
-        x[m] = __ldcg(x + m) + v;
-    }
-}
-
-// grid-size dense coarsest inverse (up to kCoarseDirectGrid rows): one warp
-// per row, lane-strided partial sums folded by a butterfly
-// (with `up`, the row's correction goes straight to the members of its aggregate)
-template <class T>
-__device__ __noinline__ void amg_coarse_dense_warp(T &tm, const DevMesh &M, DevInst &I, bool up) {
-    const int l = M.nLevels - 1;
-    const int n = M.lev[l].n;
-    const double *b = lev_b(I, M, l);
-    double *x = lev_x(I, M, l);
-    const int lane = tm.spread() & 31;
-    for (int i = tm.spread() >> 5; i < n; i += tm.size() >> 5) {
-        const double *row = I.ainv + (size_t)i * n;
-        double s = 0.0;
-        for (int j = lane; j < n; j += 32) s = fma(LD(row + j), LD(b + j), s);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (up) amg_add_up(M, I, l, i, s, lane, 32);
-        else if (lane == 0) x[i] = s;
-    }
-    tm.sync();
-}
-
 template <class T>
 __device__ void amg_coarse_solve(T &tm, const DevMesh &M, DevInst &I) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
-    if (M.coarseDirect && n > kCoarseDirect) {
-        amg_coarse_dense_warp(tm, M, I, false);
-    } else if (M.coarseDirect) {
+    if (M.coarseDirect) {
         const double *b = lev_b(I, M, l);
         double *x = lev_x(I, M, l);
-        for (int i = tm.spread(); i < n; i += tm.size()) {
+        for (int i = tm.rank(); i < n; i += tm.size()) {
             double s = 0.0;
             for (int j = 0; j < n; ++j) s = fma(LD(I.ainv + (size_t)i * n + j), LD(b + j), s);
             x[i] = s;
@@ -275,29 +253,9 @@ __device__ void amg_coarse_solve(T &tm, const DevMesh &M, DevInst &I) {
     }
 }
 
-// one damped-Jacobi sweep on a coarse level (l >= 1): reads x, writes `out`
-template <class T>
-__device__ __noinline__ void amg_jacobi(T &tm, const DevMesh &M, DevInst &I, int l, const double *x, double *out,
-                                        bool up = false) {
-    const AmgLevelDev &L = M.lev[l];
-    const double *b = lev_b(I, M, l), *val = lev_vals(I, M, l), *rd = lev_rd(I, M, l);
-    for (int i = tm.spread(); i < L.n; i += tm.size()) {
-        const double s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
-        const double v = fma(kJacobiWeight64 * LD(rd + i), s, LD(x + i));
-        if (up) amg_add_up(M, I, l, i, v, 0, 1);
-        else out[i] = v;
-    }
-    tm.sync();
-}
-
-// On the cooperative grid the coarse levels take a pair of damped-Jacobi
-// sweeps (x -> r -> x) instead of two multicolour Gauss-Seidel sweeps: one grid
-// barrier per sweep rather than one per colour (6-11 colours on Galerkin
-// levels), for ~15-20 % more PCG iterations.
-template <class T> struct GridSmoothing { static constexpr bool jacobi = false; };
-template <> struct GridSmoothing<GridTeam> { static constexpr bool jacobi = true; };
-
-// V-cycle on all levels: 2 pre-sweeps (colours ascending), 2 post sweeps
+// V-cycle on all levels, on one CTA (L1 keeps the rows there, and passes that
+// fetch ahead of their barrier measured 20 % slower: the grid's are in
+// btm_cycle.cuh): 2 pre-sweeps (colours ascending), 2 post sweeps
 // (colours descending), symmetric so the preconditioner suits CG.
 template <class T>
 __device__ void amg_vcycle_gs(T &tm, const DevMesh &M, DevInst &I) {
@@ -312,38 +270,6 @@ __device__ void amg_vcycle_gs(T &tm, const DevMesh &M, DevInst &I) {
         amg_prolong(tm, M, I, l);
         amg_gs_sweep(tm, M, I, l, true);
         amg_gs_sweep(tm, M, I, l, true);
-    }
-}
-
-// The same with Jacobi pairs on the coarse levels, five barriers a level
-// instead of seven: the first pre-sweep is part of the finer level's
-// restriction, the prolongation part of the second post-sweep (or of the
-// coarsest solve).
-template <class T>
-__device__ void amg_vcycle_jacobi(T &tm, const DevMesh &M, DevInst &I) {
-    const int nl = M.nLevels;
-    if (nl > 1) {
-        amg_gs_sweep(tm, M, I, 0, false);
-        amg_gs_sweep(tm, M, I, 0, false);
-        amg_restrict(tm, M, I, 0, nl > 2);
-    }
-    for (int l = 1; l < nl - 1; ++l) {
-        amg_jacobi(tm, M, I, l, lev_r(I, M, l), lev_x(I, M, l));
-        amg_restrict(tm, M, I, l, l + 1 < nl - 1);
-    }
-    if (nl > 1 && M.coarseDirect && M.lev[nl - 1].n > kCoarseDirect) {
-        amg_coarse_dense_warp(tm, M, I, true);
-    } else {
-        amg_coarse_solve(tm, M, I);
-        if (nl > 1) amg_prolong(tm, M, I, nl - 2);
-    }
-    for (int l = nl - 2; l > 0; --l) {
-        amg_jacobi(tm, M, I, l, lev_x(I, M, l), lev_r(I, M, l));
-        amg_jacobi(tm, M, I, l, lev_r(I, M, l), lev_x(I, M, l), true);
-    }
-    if (nl > 1) {
-        amg_gs_sweep(tm, M, I, 0, true);
-        amg_gs_sweep(tm, M, I, 0, true);
     }
 }
 
@@ -362,7 +288,7 @@ template <class T> struct AmgDriver {
         if (M.coarseDirect) amg_coarse_inverse(tm, M, I);
     }
     __device__ static void vcycle(T &tm, const DevMesh &M, DevInst &I) {
-        if constexpr (GridSmoothing<T>::jacobi) amg_vcycle_jacobi(tm, M, I);
+        if constexpr (std::is_same<T, GridTeam>::value) Cycle<T, Cycle64>::run(tm, Cycle64{M, I});
         else amg_vcycle_gs(tm, M, I);
     }
 };

@@ -31,6 +31,7 @@
 #include "btm_phases64.cuh"
 #include "btm_observe.cuh"
 #include "btm_dense.cuh"
+#include "btm_cycle.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -730,6 +731,25 @@ __device__ __noinline__ void mx_amg_coarse_inverse(T &tm, const DevMesh &M, DevW
     }
 }
 
+// the arrays of an instance for the V-cycle (btm_cycle.cuh)
+struct Cycle32 {
+    using V = float;
+    static constexpr float kWeight = 0.7f;
+    const DevMesh &M;
+    DevWork32 &F;
+    __device__ __forceinline__ int levels() const { return M.nLevels; }
+    __device__ __forceinline__ bool direct() const { return M.coarseDirect != 0; }
+    __device__ __forceinline__ const AmgLevelDev &lev(int l) const { return M.lev[l]; }
+    __device__ __forceinline__ RowTab rows() const { return RowTab(M); }
+    __device__ __forceinline__ float *x(int l) const { return lev_xf(F, M, l); }
+    __device__ __forceinline__ float *b(int l) const { return lev_bf(F, M, l); }
+    __device__ __forceinline__ float *r(int l) const { return lev_rf(F, M, l); }
+    __device__ __forceinline__ float *rd(int l) const { return lev_rdf(F, M, l); }
+    __device__ __forceinline__ float *val(int l) const { return lev_valsf(F, M, l); }
+    __device__ __forceinline__ const float *sys() const { return F.diag; }
+    __device__ __forceinline__ const double *ainv() const { return F.ainv; }
+};
+
 template <class T>
 __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 &F, int l, bool reverse) {
     const AmgLevelDev &L = M.lev[l];
@@ -752,51 +772,31 @@ __device__ __noinline__ void mx_amg_gs_sweep(T &tm, const DevMesh &M, DevWork32 
     }
 }
 
-// The correction v of row J of level l to the members of its aggregate on the
-// finer level: the prolongation of that row.
-template <class T>
-__device__ __forceinline__ void mx_amg_add_up(const DevMesh &M, DevWork32 &F, int l, int J, float v, int first,
-                                              int step) {
-    const AmgLevelDev &L = M.lev[l - 1];
-    float *x = lev_xf(F, M, l - 1);
-    for (int q = L.aggOff[J] + first; q < L.aggOff[J + 1]; q += step) {
-        const int m = L.aggMem[q];
-        x[m] = LD(x + m) + v;
-    }
-}
-
 // one damped-Jacobi sweep on a coarse level (l >= 1): reads x, writes `out`
 // (the V-cycle ping-pongs between the level's x and r arrays)
 constexpr float kJacobiWeight = 0.7f;
-// (`up`: the result is the level's last, and goes to the finer level instead)
 template <class T>
-__device__ __noinline__ void mx_amg_jacobi(T &tm, const DevMesh &M, DevWork32 &F, int l, const float *x, float *out,
-                                           bool up = false) {
+__device__ __noinline__ void mx_amg_jacobi(T &tm, const DevMesh &M, DevWork32 &F, int l, const float *x, float *out) {
     const AmgLevelDev &L = M.lev[l];
     const float *b = lev_bf(F, M, l);
     const float *val = lev_valsf(F, M, l);
     const float *rd = lev_rdf(F, M, l);
     for (int i = tm.spread(); i < L.n; i += tm.size()) {
         const float s = csr_off<T, true>(L, val, x, i, -1, LD(b + i));
-        const float v = fmaf(kJacobiWeight * LD(rd + i), s, LD(x + i));
-        if (up) mx_amg_add_up<T>(M, F, l, i, v, 0, 1);
-        else out[i] = v;
+        out[i] = fmaf(kJacobiWeight * LD(rd + i), s, LD(x + i));
     }
     tm.sync();
 }
 
 // residual of level l restricted into level l+1 in one pass: each coarse row
 // sums b - A x over its aggregate's members, and every fine row belongs to
-// exactly one aggregate; with `smooth` also the first damped-Jacobi sweep of
-// level l + 1, which starts from zero and needs no neighbours, into that
-// level's r (x is not read before the second sweep writes it)
+// exactly one aggregate (x_{l+1} = 0)
 template <class T>
-__device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 &F, int l, bool smooth) {
+__device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     const AmgLevelDev &L = M.lev[l];
     const float *x = lev_xf(F, M, l), *b = lev_bf(F, M, l), *val = lev_valsf(F, M, l);
     const AmgLevelDev &C = M.lev[l + 1];
-    float *bc = lev_bf(F, M, l + 1), *xc = lev_xf(F, M, l + 1), *rc = lev_rf(F, M, l + 1);
-    const float *rdc = lev_rdf(F, M, l + 1);
+    float *bc = lev_bf(F, M, l + 1), *xc = lev_xf(F, M, l + 1);
     for (int J = tm.spread(); J < C.n; J += tm.size()) {
         float acc = 0.0f;
         for (int q = L.aggOff[J]; q < L.aggOff[J + 1]; ++q) {
@@ -810,8 +810,7 @@ __device__ __noinline__ void mx_amg_restrict(T &tm, const DevMesh &M, DevWork32 
             acc += LD(b + i) - s;
         }
         bc[J] = acc;
-        if (smooth) rc[J] = fmaf(kJacobiWeight * LD(rdc + J), acc, 0.0f);
-        else xc[J] = 0.0f;
+        xc[J] = 0.0f;
     }
     tm.sync();
 }
@@ -825,37 +824,14 @@ __device__ void mx_amg_prolong(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     tm.sync();
 }
 
-// grid-size dense coarsest inverse (up to kCoarseDirectGrid rows): one warp
-// per row, lane-strided partial sums folded by a butterfly
-// (with `up`, the row's correction goes straight to the members of its aggregate)
-template <class T>
-__device__ __noinline__ void mx_amg_coarse_dense_warp(T &tm, const DevMesh &M, DevWork32 &F, bool up) {
-    const int l = M.nLevels - 1;
-    const int n = M.lev[l].n;
-    const float *b = lev_bf(F, M, l);
-    float *x = lev_xf(F, M, l);
-    const int lane = tm.spread() & 31;
-    for (int i = tm.spread() >> 5; i < n; i += tm.size() >> 5) {
-        const double *row = F.ainv + (size_t)i * n;
-        double s = 0.0;
-        for (int j = lane; j < n; j += 32) s = fma(LD(row + j), (double)LD(b + j), s);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (up) mx_amg_add_up<T>(M, F, l, i, (float)s, lane, 32);
-        else if (lane == 0) x[i] = (float)s;
-    }
-    tm.sync();
-}
-
 template <class T>
 __device__ void mx_amg_coarse_solve(T &tm, const DevMesh &M, DevWork32 &F) {
     const int l = M.nLevels - 1;
     const int n = M.lev[l].n;
-    if (M.coarseDirect && n > kCoarseDirect) {
-        mx_amg_coarse_dense_warp(tm, M, F, false);
-    } else if (M.coarseDirect) {
+    if (M.coarseDirect) {
         const float *b = lev_bf(F, M, l);
         float *x = lev_xf(F, M, l);
-        for (int i = tm.spread(); i < n; i += tm.size()) {
+        for (int i = tm.rank(); i < n; i += tm.size()) {
             double s = 0.0;
             for (int j = 0; j < n; ++j) s = fma(LD(F.ainv + (size_t)i * n + j), (double)LD(b + j), s);
             x[i] = (float)s;
@@ -879,39 +855,36 @@ __device__ void mx_amg_values_from(T &tm, const DevMesh &M, DevWork32 &F, int l0
     tm.sync();
 }
 
-// Symmetric V-cycle: two smoothing sweeps of level l before and after the coarse
+// Symmetric V-cycle: two smoothing sweeps of a level before and after the coarse
 // correction, on level 0 multicolour Gauss-Seidel (colours ascending before,
 // descending after), on the coarse levels a pair of damped-Jacobi sweeps
 // (x -> r -> x) instead, which needs one barrier per sweep rather than one per
-// colour (6-11 colours on Galerkin levels) and costs ~15-20 % more PCG
-// iterations.  Four barriers a coarse level: the first pre-sweep is part of the
-// finer level's restriction, the prolongation part of the second post-sweep (or
-// of the coarsest solve).
+// colour (6-11 colours on Galerkin levels) and costs ~15-20 % more PCG iterations.
 template <class T>
 __device__ void mx_amg_vcycle(T &tm, const DevMesh &M, DevWork32 &F) {
-    const int nl = M.nLevels;
-    if (nl > 1) {
-        mx_amg_gs_sweep(tm, M, F, 0, false);
-        mx_amg_gs_sweep(tm, M, F, 0, false);
-        mx_amg_restrict(tm, M, F, 0, nl > 2);
-    }
-    for (int l = 1; l < nl - 1; ++l) {
-        mx_amg_jacobi(tm, M, F, l, lev_rf(F, M, l), lev_xf(F, M, l));
-        mx_amg_restrict(tm, M, F, l, l + 1 < nl - 1);
-    }
-    if (nl > 1 && M.coarseDirect && M.lev[nl - 1].n > kCoarseDirect) {
-        mx_amg_coarse_dense_warp(tm, M, F, true);
+    if constexpr (std::is_same<T, GridTeam>::value) {
+        Cycle<T, Cycle32>::run(tm, Cycle32{M, F});
     } else {
+        const int nl = M.nLevels;
+        auto smooth = [&](int l, bool post) {
+            if (l == 0) {
+                mx_amg_gs_sweep(tm, M, F, 0, post);
+                mx_amg_gs_sweep(tm, M, F, 0, post);
+            } else {
+                float *x = lev_xf(F, M, l), *tmp = lev_rf(F, M, l);
+                mx_amg_jacobi(tm, M, F, l, x, tmp);
+                mx_amg_jacobi(tm, M, F, l, tmp, x);
+            }
+        };
+        for (int l = 0; l < nl - 1; ++l) {
+            smooth(l, false);
+            mx_amg_restrict(tm, M, F, l);
+        }
         mx_amg_coarse_solve(tm, M, F);
-        if (nl > 1) mx_amg_prolong(tm, M, F, nl - 2);
-    }
-    for (int l = nl - 2; l > 0; --l) {
-        mx_amg_jacobi(tm, M, F, l, lev_xf(F, M, l), lev_rf(F, M, l));
-        mx_amg_jacobi(tm, M, F, l, lev_rf(F, M, l), lev_xf(F, M, l), true);
-    }
-    if (nl > 1) {
-        mx_amg_gs_sweep(tm, M, F, 0, true);
-        mx_amg_gs_sweep(tm, M, F, 0, true);
+        for (int l = nl - 2; l >= 0; --l) {
+            mx_amg_prolong(tm, M, F, l);
+            smooth(l, true);
+        }
     }
 }
 

@@ -26,7 +26,8 @@ LIB_NAME = "libbtm_gb300.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["btm_engine.cu", "btm_mixed.cu", "btm_host.cpp", "btm_server.cpp", "btm_noalloc.cu"]
 HEADERS = ["btm_common.h", "btm_host_internal.h", "btm_team.cuh", "btm_bc.cuh", "btm_phases64.cuh",
-           "btm_observe.cuh", "btm_ramg.cuh", "btm_dense.cuh"]
+           "btm_observe.cuh", "btm_ramg.cuh", "btm_dense.cuh",
+           "btm_cycle.cuh"]
 
 
 def nvcc() -> str:
