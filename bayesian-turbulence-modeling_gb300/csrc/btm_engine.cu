@@ -179,20 +179,25 @@ struct Cycle64 {
 // one colour-ordered Gauss-Seidel sweep (forward or reverse colour order)
 template <class T>
 __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
-    const AmgLevelDev &L = M.lev[l];
+    // (locals: the descriptors are in shared memory, and every store has them read again)
+    const CsrTab L(M.lev[l]);
+    const RowTab R(M);
     double *x = lev_x(I, M, l);
     const double *b = lev_b(I, M, l);
     const double *val = lev_vals(I, M, l);
     const double *rd = lev_rd(I, M, l);
-    for (int cc = 0; cc < L.nColors; ++cc) {
-        const int col = reverse ? L.nColors - 1 - cc : cc;
-        for (int q = L.colorOff[col] + tm.spread(); q < L.colorOff[col + 1]; q += tm.size()) {
-            const int i = L.colorRows[q];
+    const int32_t *off = M.lev[l].colorOff, *rows = M.lev[l].colorRows;
+    const int nColors = M.lev[l].nColors;
+    for (int cc = 0; cc < nColors; ++cc) {
+        const int col = reverse ? nColors - 1 - cc : cc;
+        const int q1 = off[col + 1];
+        for (int q = off[col] + tm.rank(); q < q1; q += tm.size()) {
+            const int i = rows[q];
             const double ri = LD(rd + i);
-            if (ri == 0.0) continue;
+            if (!nonzero64(ri)) continue;
             double s = LD(b + i);
-            if (l == 0) s = ldu_off<T, true>(M, I.diag, x, i, s);
-            else s = csr_off<T, true>(L, val, x, i, i, s);
+            if (l == 0) s = ldu_off<T, true>(R, val, (const double *)x, i, s);
+            else s = csr_off<T, true>(L, val, (const double *)x, i, i, s);
             x[i] = s * ri;
         }
         tm.sync();

@@ -106,15 +106,9 @@ __device__ __forceinline__ void ggd_cell(const DevMesh &M, int c, const V *const
     float ax[NF], ay[NF], az[NF];
 #pragma unroll
     for (int q = 0; q < NF; ++q) { ax[q] = 0.0f; ay[q] = 0.0f; az[q] = 0.0f; pc[q] = LD(phi[q] + c); }
-    const int e0 = M.cfOff[c], e1 = M.cfOff[c + 1];
-    for (int e = e0; e < e1; ++e) {
-        const int f = M.cfFace[e];
-        const int oth = M.cfOther[e];
-        const float nx = G.nx[f], ny = G.ny[f], nz = G.nz[f];
-        float fac;
-        int other;
-        if (oth >= 0) { fac = (1.0f - G.w[f]) * G.area[f]; other = oth; }
-        else { fac = -G.w[f] * G.area[f]; other = -(oth + 1); }
+    cell_faces(M, c, [&](int f, int other, bool own) {
+        const float nx = G.nx[f], ny = G.ny[f], nz = G.nz[f], w = G.w[f];
+        const float fac = (own ? 1.0f - w : -w) * G.area[f];
 #pragma unroll
         for (int q = 0; q < NF; ++q) {
             const float d = (float)(LD(phi[q] + other) - pc[q]) * fac;
@@ -122,7 +116,7 @@ __device__ __forceinline__ void ggd_cell(const DevMesh &M, int c, const V *const
             ay[q] = fmaf(d, ny, ay[q]);
             az[q] = fmaf(d, nz, az[q]);
         }
-    }
+    });
     for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
         const int b = M.cbFace[e];
         const float fac = G.barea[b], nx = G.bnx[b], ny = G.bny[b], nz = G.bnz[b];
@@ -220,7 +214,7 @@ __device__ __noinline__ void mx_sst(T &tm, const DevMesh &M, DevInst &I, float n
 // normals and areas in FP64); the z term is skipped when U_z is identically 0
 template <class T>
 __device__ __forceinline__ double mflux64(const DevMesh &M, const DevInst &I, int f, int o, int n, bool z) {
-    const double w = M.w[f], wn = 1.0 - w;
+    const double w = M.w[f], wn = M.wn[f];
     double m = (LD(I.ux + o) * w + LD(I.ux + n) * wn) * M.nx[f];
     m = fma(LD(I.uy + o) * w + LD(I.uy + n) * wn, M.ny[f], m);
     if (z) m = fma(LD(I.uz + o) * w + LD(I.uz + n) * wn, M.nz[f], m);
@@ -298,23 +292,15 @@ __device__ __forceinline__ double cd_cell_flux(const DevMesh &M, const DevInst &
                                                double phiP, float &diag) {
     const DevWork32 &F = I.f;
     double r = 0.0;
-    for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-        const int f = M.cfFace[e], oth = M.cfOther[e];
-        int other;
-        double mo;
-        if (oth >= 0) {
-            diag -= LD(F.lower + f);
-            other = oth;
-            mo = LD(F.mflux + f);
-        } else {
-            diag -= LD(F.upper + f);
-            other = -(oth + 1);
-            mo = -LD(F.mflux + f);
-        }
+    const float *upper = F.upper, *lower = F.lower, *dcoef = F.dcoef;
+    const double *mflux = F.mflux;
+    cell_faces(M, c, [&](int f, int other, bool own) {
+        diag -= LD((own ? lower : upper) + f);
+        const double mo = flip(LD(mflux + f), !own);
         const double phiN = LD(phi + other);
-        r = fma((double)LD(F.dcoef + f), phiP - phiN, r);
-        r = fma(mo, mo >= 0.0 ? phiP : phiN, r);
-    }
+        r = fma((double)LD(dcoef + f), phiP - phiN, r);
+        r = fma(mo, is_negative(mo) ? phiN : phiP, r);
+    });
     return r;
 }
 
@@ -338,10 +324,8 @@ __device__ __noinline__ double mx_mom_cells(T &tm, const DevMesh &M, DevInst &I,
         const double uP = LD(Uc + c);
         float diag = 0.0f, ts = 0.0f;
         double flux = cd_cell_flux<T>(M, I, c, Uc, uP, diag);
-        for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-            const int f = M.cfFace[e];
-            ts += M.cfOther[e] >= 0 ? LD(F.tflux + f) : -LD(F.tflux + f);
-        }
+        const float *tflux = F.tflux;
+        cell_faces(M, c, [&](int f, int, bool own) { ts += own ? LD(tflux + f) : -LD(tflux + f); });
         const float nutc = F.nut[c];
         for (int e = M.cbOff[c]; e < M.cbOff[c + 1]; ++e) {
             const int b = M.cbFace[e];
@@ -414,12 +398,12 @@ __device__ __noinline__ double mx_p_cells(T &tm, const DevMesh &M, DevInst &I) {
     for (int c = tm.rank(); c < M.nC; c += tm.size()) {
         float diag = 0.0f;
         double src = 0.0;
-        for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-            const int f = M.cfFace[e];
-            diag -= LD(F.upper + f);
-            if (M.cfOther[e] >= 0) src -= LD(F.mflux + f);
-            else src += LD(F.mflux + f);
-        }
+        const float *upper = F.upper;
+        const double *mflux = F.mflux;
+        cell_faces(M, c, [&](int f, int, bool own) {
+            diag -= LD(upper + f);
+            src += flip(LD(mflux + f), own);
+        });
         const float aPc = F.aPx[c];
         for (int e = M.cbpOff[c]; e < M.cbpOff[c + 1]; ++e) {
             const int b = M.cbpFace[e];
@@ -1217,11 +1201,10 @@ __device__ __noinline__ double mx_p_defect(T &tm, const DevMesh &M, DevWork32 &F
     double rr = 0.0;
     for (int c = tm.rank(); c < M.nC; c += tm.size()) {
         double ay = (double)LD(F.diag + c) * (double)LD(F.pp + c);
-        for (int e = M.cfOff[c]; e < M.cfOff[c + 1]; ++e) {
-            const int f = M.cfFace[e], oth = M.cfOther[e];
-            if (oth >= 0) ay = fma((double)LD(F.upper + f), (double)LD(F.pp + oth), ay);
-            else ay = fma((double)LD(F.lower + f), (double)LD(F.pp + (-(oth + 1))), ay);
-        }
+        const float *upper = F.upper, *lower = F.lower, *pp = F.pp;
+        cell_faces(M, c, [&](int f, int other, bool own) {
+            ay = fma((double)LD((own ? upper : lower) + f), (double)LD(pp + other), ay);
+        });
         const double d = LD(F.src64 + c) * s - ay;
         F.src[c] = (float)d;
         rr = fma(d, d, rr);
@@ -2031,13 +2014,13 @@ __device__ __host__ inline size_t smem_round(size_t b) { return (b + kSmemAlign 
 // not fit, or that the instance does not use, stays in global memory.
 enum SmemItem : int {
     SI_SYS = 0, SI_BAND, SI_BANDRD, SI_R, SI_S, SI_T, SI_PV, SI_V, SI_PP, SI_X, SI_AMGRD, SI_AMGX, SI_AMGB, SI_AMGR,
-    SI_AMGVAL, SI_RH, SI_PH, SI_SH, SI_RD, SI_SRC, SI_AINV, SI_ROWCOL, SI_ROWENT, SI_CFOFF, SI_CFFACE, SI_CFOTHER, SI_COUNT
+    SI_AMGVAL, SI_RH, SI_PH, SI_SH, SI_RD, SI_SRC, SI_AINV, SI_ROWCOL, SI_ROWENT, SI_COUNT
 };
 
 // sizes in placement order (bytes, 0: not staged); returns the count.  With
 // a band factor (band > 0) the pressure correction does not use the AMG
 // arrays, which stay in global memory for the fallback solve.
-__device__ __host__ inline int smem_items(int nC, int nIF, int64_t vec, int64_t val, int nc, int nGather, int band,
+__device__ __host__ inline int smem_items(int nC, int nIF, int64_t vec, int64_t val, int nc, int band,
                                           int rowW, size_t *sz) {
     const bool amg = band == 0;
     sz[SI_SYS] = 4 * ((size_t)nC + 2 * (size_t)nIF);                  // diag | upper | lower
@@ -2050,9 +2033,6 @@ __device__ __host__ inline int smem_items(int nC, int nIF, int64_t vec, int64_t 
     for (int q = SI_RH; q <= SI_SRC; ++q) sz[q] = 4 * (size_t)nC;      // rh ph sh rd src
     sz[SI_AINV] = amg ? 8 * (size_t)nc * nc : 0;                       // coarse inverse (FP64)
     sz[SI_ROWCOL] = sz[SI_ROWENT] = 4 * (size_t)nC * rowW;
-    sz[SI_CFOFF] = 4 * ((size_t)nC + 1);
-    sz[SI_CFFACE] = 4 * (size_t)nGather;
-    sz[SI_CFOTHER] = 4 * (size_t)nGather;
     return SI_COUNT;
 }
 
@@ -2060,9 +2040,8 @@ __device__ void stage_smem(DevMesh &M, DevInst &I, unsigned char *dsm, size_t ca
     DevWork32 &F = I.f;
     const int nC = M.nC, nIF = M.nIF;
     const int nc = M.coarseDirect ? M.lev[M.nLevels - 1].n : 1;
-    const int nGather = 2 * nIF;
     size_t sz[SI_COUNT];
-    const int nItems = smem_items(nC, nIF, M.amgVecTotal, M.amgValTotal, nc, nGather, M.band, M.rowW, sz);
+    const int nItems = smem_items(nC, nIF, M.amgVecTotal, M.amgValTotal, nc, M.band, M.rowW, sz);
     size_t off = 0;
     int nc_ = 0;
     for (int q = 0; q < nItems; ++q) {
@@ -2095,9 +2074,6 @@ __device__ void stage_smem(DevMesh &M, DevInst &I, unsigned char *dsm, size_t ca
             case SI_AINV: F.ainv = (double *)p; break;
             case SI_ROWCOL: copies[nc_++] = {p, M.rowCol, (int)sz[q]}; M.rowCol = (const int32_t *)p; break;
             case SI_ROWENT: copies[nc_++] = {p, M.rowEnt, (int)sz[q]}; M.rowEnt = (const int32_t *)p; break;
-            case SI_CFOFF: copies[nc_++] = {p, M.cfOff, (int)sz[q]}; M.cfOff = (const int32_t *)p; break;
-            case SI_CFFACE: copies[nc_++] = {p, M.cfFace, (int)sz[q]}; M.cfFace = (const int32_t *)p; break;
-            case SI_CFOTHER: copies[nc_++] = {p, M.cfOther, (int)sz[q]}; M.cfOther = (const int32_t *)p; break;
         }
     }
     *nCopies = nc_;
@@ -2111,7 +2087,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mixed_block(DevInst *insts, in
     __shared__ double tot[2 * (NT / 32) + kRedResults];
     __shared__ DevMesh sM;
     __shared__ DevInst sI;
-    __shared__ SmemCopy copies[5];
+    __shared__ SmemCopy copies[2];
     __shared__ int nCopies;
     if (blockIdx.x >= n) return;
     if (threadIdx.x == 0) {
@@ -2170,7 +2146,7 @@ int mixed_launch_grid(DevInst *dInst, int blocks, void *stream) {
 // dynamic shared memory that would hold an instance's whole solver working set
 size_t mixed_smem_bytes(int nC, int nIF, int64_t vecTotal, int64_t valTotal, int coarseN, int band, int rowW) {
     size_t sz[SI_COUNT];
-    const int n = smem_items(nC, nIF, vecTotal, valTotal, coarseN, 2 * nIF, band, rowW, sz);
+    const int n = smem_items(nC, nIF, vecTotal, valTotal, coarseN, band, rowW, sz);
     size_t t = 0;
     for (int q = 0; q < n; ++q) t += smem_round(sz[q]);
     return t;

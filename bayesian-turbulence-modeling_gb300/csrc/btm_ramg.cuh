@@ -162,7 +162,6 @@ struct RGroup {
 // eighth, and rows past the CTA's size, are read in place.
 constexpr int kRowRegs = 8;
 constexpr int kRec = 10, kRec0 = 6;   // doubles per record: values, columns (level 0: and 1/diag), by 16-byte parts
-__device__ __forceinline__ bool nonzero64(double v) { return (__double_as_longlong(v) << 1) != 0; }
 // x of a level, in shared memory (addresses of 32 bits) or global memory
 template <bool SM> struct RX;
 template <> struct RX<true> {

@@ -437,6 +437,8 @@ template <> struct Ld<GridTeam> {
 // 6-entry level on the grid 7 us long where its barrier takes 1.6 us; fetched
 // together it is 2.6 us.
 // ---------------------------------------------------------------------------
+// v != 0 (and not -0) without an FP64 comparison
+__device__ __forceinline__ bool nonzero64(double v) { return (__double_as_longlong(v) << 1) != 0; }
 __device__ __forceinline__ double fma_any(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fma_any(float a, float b, float c) { return fmaf(a, b, c); }
 
@@ -486,9 +488,13 @@ __device__ __forceinline__ V ldu_off(const DevMesh &M, const V *sys, const V *x,
     return ldu_off<T, Neg>(RowTab(M), sys, x, c, y);
 }
 
+struct CsrTab {
+    const int32_t *rowPtr, *colIdx;
+    __device__ __forceinline__ CsrTab(const AmgLevelDev &L) : rowPtr(L.rowPtr), colIdx(L.colIdx) {}
+};
 // Row i of a CSR level without its column `skip` (-1: all of it).
 template <class T, bool Neg, class V>
-__device__ __forceinline__ V csr_off(const AmgLevelDev &L, const V *val, const V *x, int i, int skip, V y) {
+__device__ __forceinline__ V csr_off(const CsrTab &L, const V *val, const V *x, int i, int skip, V y) {
     constexpr int W = 8;
     const int q1 = L.rowPtr[i + 1];
     for (int q = L.rowPtr[i]; q < q1; q += W) {
