@@ -221,16 +221,20 @@ __device__ __forceinline__ double ramg_rest(const RLevel &L, int i, double s) {
     }
     return s;
 }
-// b minus the products of the row's first W entries
-template <int W, bool SM>
-__device__ __forceinline__ double ramg_sum(const RRow<W, SM> &R) {
-    double x[W];
+// b minus the products of the row's first N entries
+template <int N, int W, bool SM>
+__device__ __forceinline__ double ramg_sum_first(const RRow<W, SM> &R) {
+    double x[N];
 #pragma unroll
-    for (int k = 0; k < W; ++k) x[k] = RX<SM>::get(R.from[k]);
+    for (int k = 0; k < N; ++k) x[k] = RX<SM>::get(R.from[k]);
     double s = R.b;
 #pragma unroll
-    for (int k = 0; k < W; ++k) s = fma(-R.val[k], x[k], s);
+    for (int k = 0; k < N; ++k) s = fma(-R.val[k], x[k], s);
     return s;
+}
+template <int W, bool SM>
+__device__ __forceinline__ double ramg_sum(const RRow<W, SM> &R) {
+    return ramg_sum_first<W>(R);
 }
 template <int W, bool SM>
 __device__ __forceinline__ void ramg_relax(const RLevel &L, const RRow<W, SM> &R) {
@@ -265,6 +269,7 @@ __device__ __noinline__ bool ramg_gs_resident(const RLevel &L, int sweeps) {
     int wave[2] = {-1, -1};
     unsigned int used[2] = {0, 0};   // wavefronts with rows in slots 0-31 / 32-63
     unsigned int wide[2] = {0, 0};   // ... and wide rows among them
+    unsigned int past4[2] = {0, 0}, past6[2] = {0, 0};   // ... and rows of more than 4, 6 entries
     bool fits = true;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -296,6 +301,10 @@ __device__ __noinline__ bool ramg_gs_resident(const RLevel &L, int sweeps) {
             const bool mine = slot >= o && slot < o + num;
             if (mine && nonzero64(R[h].rd)) wave[h] = w;
             if (__any_sync(0xffffffffu, mine && R[h].wide)) wide[h] |= 1u << w;
+            const bool four = nonzero64(R[h].val[4]) || nonzero64(R[h].val[5]);
+            const bool six = nonzero64(R[h].val[6]) || nonzero64(R[h].val[7]);
+            if (__any_sync(0xffffffffu, mine && (four || six))) past4[h] |= 1u << w;
+            if (__any_sync(0xffffffffu, mine && six)) past6[h] |= 1u << w;
         }
     }
     for (int t = 0; t < sweeps; ++t) {
@@ -303,7 +312,10 @@ __device__ __noinline__ bool ramg_gs_resident(const RLevel &L, int sweeps) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (used[h] >> w & 1) {
-                    double s = ramg_sum(R[h]);
+                    // (a position whose entries are all zero leaves the sums as they are)
+                    double s = past6[h] >> w & 1   ? ramg_sum_first<8>(R[h])
+                               : past4[h] >> w & 1 ? ramg_sum_first<6>(R[h])
+                                                   : ramg_sum_first<4>(R[h]);
                     if (wide[h] >> w & 1) {
 #pragma unroll
                         for (int k = 0; k < kRowMore; ++k) s = fma(-more[h][k], RX<SM>::get(moreAt[h][k]), s);
@@ -472,7 +484,7 @@ __device__ int ramg_wavefronts(T &tm, const RamgWork &W, const int32_t *ptr, con
     for (int i = tm.rank(); i < n; i += tm.size()) a[i] = 0;
     tm.sync();
     for (int it = 0; it <= n; ++it) {
-        double ch[1] = {0.0};
+        bool changed = false;
         for (int i = tm.rank(); i < n; i += tm.size()) {
             int dd = 0;
             for (int j = ptr[i]; j < ptr[i + 1]; ++j) {
@@ -480,17 +492,22 @@ __device__ int ramg_wavefronts(T &tm, const RamgWork &W, const int32_t *ptr, con
                 if (c < i) dd = max(dd, a[c] + 1);
             }
             b[i] = dd;
-            if (dd != a[i]) ch[0] = 1.0;
+            changed = changed || dd != a[i];
         }
-        tm.template maxr<1>(ch);
+        const bool again = __syncthreads_or(changed);
         int32_t *tmp = a; a = b; b = tmp;
-        if (ch[0] == 0.0) break;
+        if (!again) break;
     }
     // a holds the depths; count, scan and place
-    double mx[1] = {0.0};
-    for (int i = tm.rank(); i < n; i += tm.size()) mx[0] = smax(mx[0], (double)a[i]);
-    tm.template maxr<1>(mx);
-    const int nWf = (int)mx[0] + 1;
+    __shared__ int deepest;
+    if (tm.leader()) deepest = 0;
+    tm.sync();
+    int mx = 0;
+    for (int i = tm.rank(); i < n; i += tm.size()) mx = max(mx, a[i]);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) atomicMax(&deepest, mx);
+    tm.sync();
+    const int nWf = deepest + 1;
     for (int q = tm.rank(); q <= nWf; q += tm.size()) wfOff[q] = 0;
     tm.sync();
     for (int i = tm.rank(); i < n; i += tm.size()) atomicAdd(&wfOff[a[i]], 1);
