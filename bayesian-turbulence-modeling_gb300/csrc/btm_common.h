@@ -40,6 +40,7 @@ enum : int32_t {
 struct AmgLevelDev {
     int32_t n;            // rows of this level
     int32_t nnz;          // CSR entries (levels >= 1)
+    int32_t widest;       // entries of the longest row (levels >= 1)
     const int32_t *rowPtr, *colIdx, *diagPos;     // CSR (levels >= 1)
     const int32_t *gOff, *gIdx;                   // Galerkin gather into the finer level's values
     const int32_t *map;                           // this level's rows -> next level's rows

@@ -32,10 +32,11 @@ struct CycRow {
 template <class T, class A>
 struct Cycle {
     using V = typename A::V;
-    static constexpr int W0 = 6, WC = 8;   // entries held: level 0 (hexahedra have 6 neighbours), coarse levels
+    static constexpr int WC = 8;   // entries held of a coarse row; of level 0: 4 (quadrilaterals) or 6 (hexahedra)
 
     // ---- rows: level 0 from the position-major tables (off-diagonal part),
     // coarse levels from their CSR (all of it)
+    template <int W0>
     __device__ __forceinline__ static void fetch(const A &a, const RowTab &R, int i, CycRow<V, W0> &r) {
         const V *sys = a.sys();
         r.n = R.width;
@@ -60,7 +61,7 @@ struct Cycle {
         }
     }
     // y + row x (Neg: y - row x), without column `skip`, in the row's order
-    template <bool Neg>
+    template <bool Neg, int W0>
     __device__ __forceinline__ static V apply(const A &a, const RowTab &R, const CycRow<V, W0> &r, const V *x, int i,
                                               V y) {
         V v[W0];
@@ -104,14 +105,14 @@ struct Cycle {
         const V *b = a.b(l), *rd = a.rd(l), *val = a.val(l);
         const int32_t *off = L.colorOff, *rowsOf = L.colorRows;
         const int nColors = L.nColors;
-        if (l == 0) gs_level<true>(tm, a, L, R, x, b, rd, val, off, rowsOf, nColors, reverse, zero);
-        else gs_level<false>(tm, a, L, R, x, b, rd, val, off, rowsOf, nColors, reverse, zero);
+        if (l > 0) gs_level<false, WC>(tm, a, L, R, x, b, rd, val, off, rowsOf, nColors, reverse, zero);
+        else if (R.width <= 4) gs_level<true, 4>(tm, a, L, R, x, b, rd, val, off, rowsOf, nColors, reverse, zero);
+        else gs_level<true, 6>(tm, a, L, R, x, b, rd, val, off, rowsOf, nColors, reverse, zero);
     }
-    template <bool L0>
+    template <bool L0, int W>
     __device__ __forceinline__ static void gs_level(T &tm, const A &a, const AmgLevelDev &L, const RowTab &R, V *x,
                                                     const V *b, const V *rd, const V *val, const int32_t *off,
                                                     const int32_t *rowsOf, int nColors, bool reverse, bool zero) {
-        constexpr int W = L0 ? W0 : WC;
         for (int cc = 0; cc < nColors; ++cc) {
             const int col = reverse ? nColors - 1 - cc : cc;
             const int q1 = off[col + 1];
@@ -155,6 +156,25 @@ struct Cycle {
         }
     }
 
+    template <int W0>
+    __device__ __forceinline__ static void residual0(T &tm, const A &a, const RowTab &R, const V *x, const V *b, V *res,
+                                                     int n) {
+        const V *sys = a.sys();
+        int i = tm.spread();
+        CycRow<V, W0> r;
+        V d = 0, bi = 0;
+        auto get = [&](int j) {
+            fetch(a, R, j, r);
+            d = LD(sys + j);
+            bi = LD(b + j);
+        };
+        if (i < n) get(i);
+        tm.sync();
+        for (; i < n; i += tm.size()) {
+            res[i] = bi - apply<false>(a, R, r, x, i, d * LD(x + i));
+            if (i + tm.size() < n) get(i + tm.size());
+        }
+    }
     // ---- residual of level l and its restriction, b of level l + 1 (members in
     // order); with `smooth` also the first damped-Jacobi sweep of level l + 1,
     // which starts from zero and needs no neighbours, into that level's r (its
@@ -169,23 +189,8 @@ struct Cycle {
             V *res = a.r(l);
             const int n = L.n;
             if (l == 0) {
-                int i = tm.spread();
-                CycRow<V, W0> r;
-                V d = 0, bi = 0;
-                if (i < n) {
-                    fetch(a, R, i, r);
-                    d = LD(a.sys() + i);
-                    bi = LD(b + i);
-                }
-                tm.sync();
-                for (; i < n; i += tm.size()) {
-                    res[i] = bi - apply<false>(a, R, r, x, i, d * LD(x + i));
-                    if (i + tm.size() < n) {
-                        fetch(a, R, i + tm.size(), r);
-                        d = LD(a.sys() + i + tm.size());
-                        bi = LD(b + i + tm.size());
-                    }
-                }
+                if (R.width <= 4) residual0<4>(tm, a, R, x, b, res, n);
+                else residual0<6>(tm, a, R, x, b, res, n);
             } else {
                 int i = tm.spread();
                 CycRow<V, WC> r;

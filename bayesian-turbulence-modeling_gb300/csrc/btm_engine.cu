@@ -177,8 +177,8 @@ struct Cycle64 {
 };
 
 // one colour-ordered Gauss-Seidel sweep (forward or reverse colour order)
-template <class T>
-__device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
+template <class T, int W>
+__device__ __noinline__ void amg_gs_rows(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
     // (locals: the descriptors are in shared memory, and every store has them read again)
     const CsrTab L(M.lev[l]);
     const RowTab R(M);
@@ -196,12 +196,23 @@ __device__ __noinline__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, i
             const double ri = LD(rd + i);
             if (!nonzero64(ri)) continue;
             double s = LD(b + i);
-            if (l == 0) s = ldu_off<T, true>(R, val, (const double *)x, i, s);
-            else s = csr_off<T, true>(L, val, (const double *)x, i, i, s);
+            if constexpr (W == 0) s = ldu_off<T, true>(R, val, (const double *)x, i, s);
+            else s = csr_off<T, true, W>(L, val, (const double *)x, i, i, s);
             x[i] = s * ri;
         }
         tm.sync();
     }
+}
+
+// (W entries of a row at a time, as the level's longest row needs: levels of
+// structured meshes have rows of 5, whose sweeps are a tenth faster than with 8)
+template <class T>
+__device__ void amg_gs_sweep(T &tm, const DevMesh &M, DevInst &I, int l, bool reverse) {
+    const int widest = M.lev[l].widest;
+    if (l == 0) amg_gs_rows<T, 0>(tm, M, I, l, reverse);
+    else if (widest <= 5) amg_gs_rows<T, 5>(tm, M, I, l, reverse);
+    else if (widest <= 6) amg_gs_rows<T, 6>(tm, M, I, l, reverse);
+    else amg_gs_rows<T, 8>(tm, M, I, l, reverse);
 }
 
 // residual of level l and restriction into level l+1 (x_{l+1} = 0)

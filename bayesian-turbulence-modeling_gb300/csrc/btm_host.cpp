@@ -705,6 +705,8 @@ void build_case(btm_case *C, const btm_mesh *m, const btm_patch_bc *bcs, std::ve
         dl.n = L.n;
         dl.nnz = l == 0 ? 0 : (int)L.colIdx.size();
         dl.nColors = L.nColors;
+        dl.widest = 0;
+        for (int i = 0; i < L.n; ++i) dl.widest = std::max(dl.widest, L.rowPtr[i + 1] - L.rowPtr[i]);
         if (l >= 1) {
             dl.valOff = valTot; valTot += (L.colIdx.size() + 31) & ~size_t(31);
             dl.vecOff = vecTot; vecTot += (L.n + 31) & ~31;

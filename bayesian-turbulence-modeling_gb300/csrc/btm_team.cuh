@@ -492,10 +492,11 @@ struct CsrTab {
     const int32_t *rowPtr, *colIdx;
     __device__ __forceinline__ CsrTab(const AmgLevelDev &L) : rowPtr(L.rowPtr), colIdx(L.colIdx) {}
 };
-// Row i of a CSR level without its column `skip` (-1: all of it).
-template <class T, bool Neg, class V>
+// Row i of a CSR level without its column `skip` (-1: all of it), W entries at a
+// time (an FP64 multiply-add that no lane needs takes its 64 clocks all the
+// same: W should fit the level's longest row).
+template <class T, bool Neg, int W = 8, class V>
 __device__ __forceinline__ V csr_off(const CsrTab &L, const V *val, const V *x, int i, int skip, V y) {
-    constexpr int W = 8;
     const int q1 = L.rowPtr[i + 1];
     for (int q = L.rowPtr[i]; q < q1; q += W) {
         int col[W];
