@@ -7,11 +7,11 @@
 // multiply-adds take 0.3; the rest were dependent loads (row pointer, columns, x,
 // then 1 / diagonal and the aggregate's members), all from L2, as a barrier's
 // acquire empties L1.  But only x (or the residual) changes from pass to pass.
-// Every pass here therefore begins with its loads of everything else, has its
-// barrier after them instead of at its end, and then needs x only: the barrier's
-// latency and those of the loads overlap.  74k-cell duct, FP32: pressure solve
-// 1.66 -> 1.14 ms an outer iteration; 123k-cell step, FP64: 22.4 -> 20.8 ms
-// (there the FP64 multiply-adds weigh more).
+// Every pass here therefore begins with its loads of everything else, runs them
+// inside its barrier (between arrival and wait), and then needs x only: the
+// barrier's latency and those of the loads overlap.  74k-cell duct, FP32:
+// pressure solve 1.66 -> 1.05 ms an outer iteration; 123k-cell step, FP64: 22.4
+// -> 19.4 ms (there the FP64 multiply-adds weigh more).
 //
 // `A` presents the arrays of an engine: V (value type), lev(l), x(l), b(l),
 // r(l), val(l), rd(l), sys() (diag | upper | lower of level 0), ainv().
@@ -121,6 +121,7 @@ struct Cycle {
             int i = 0;
             CycRow<V, W> r;
             V ri = 0, bi = 0;
+            tm.arrive();
             if (on) {
                 i = rowsOf[q];
                 ri = LD(rd + i);
@@ -130,7 +131,7 @@ struct Cycle {
                     else fetch(L, val, i, r);
                 }
             }
-            tm.sync();
+            tm.wait();
             if (on && ri != (V)0) {
                 if (alone) bi = LD(b + i);
                 else if constexpr (L0) bi = apply<true>(a, R, r, x, i, bi);
@@ -168,8 +169,9 @@ struct Cycle {
             d = LD(sys + j);
             bi = LD(b + j);
         };
+        tm.arrive();
         if (i < n) get(i);
-        tm.sync();
+        tm.wait();
         for (; i < n; i += tm.size()) {
             res[i] = bi - apply<false>(a, R, r, x, i, d * LD(x + i));
             if (i + tm.size() < n) get(i + tm.size());
@@ -195,11 +197,12 @@ struct Cycle {
                 int i = tm.spread();
                 CycRow<V, WC> r;
                 V bi = 0;
+                tm.arrive();
                 if (i < n) {
                     fetch(L, val, i, r);
                     bi = LD(b + i);
                 }
-                tm.sync();
+                tm.wait();
                 for (; i < n; i += tm.size()) {
                     res[i] = bi - apply<false>(L, val, r, x, -1, (V)0);
                     if (i + tm.size() < n) {
@@ -226,8 +229,9 @@ struct Cycle {
             for (int k = 0; k < K; ++k) at[k] = mem[o + min(k, m - 1)];
             if (smooth) w = A::kWeight * LD(rd + J);
         };
+        tm.arrive();
         if (ready) members();
-        tm.sync();
+        tm.wait();
         for (; J < n; J += tm.size()) {
             if (!ready) members();
             ready = false;
@@ -289,8 +293,9 @@ struct Cycle {
             w = A::kWeight * LD(rd + j);
             if (UP) u.fetch(a, l, j);
         };
+        tm.arrive();
         if (i < n) get(i);
-        tm.sync();
+        tm.wait();
         for (; i < n; i += tm.size()) {
             const V xi = LD(x + i);
             if (fresh) bi = LD(b + i);
@@ -326,8 +331,9 @@ struct Cycle {
             for (int k = 0; k < K; ++k) m[k] = LD(row + min(lane + 32 * k, n - 1));
             u.fetch(a, l, j);
         };
+        tm.arrive();
         if (i < n) get(i);
-        tm.sync();
+        tm.wait();
         for (; i < n; i += tm.size() >> 5) {
             const double *row = a.ainv() + (size_t)i * n;
             double s = 0.0;

@@ -252,11 +252,18 @@ struct GridTeam {
     // error flag and the clock, and after kBarrierTimeoutNs it flags the error
     // and the whole team abandons the solve.  A CTA that has abandoned it no
     // longer arrives.
-    __device__ __noinline__ bool sync() {
+    //
+    // arrive() and wait() are its two halves: loads that do not depend on what
+    // the other CTAs are still writing go between them.
+    __device__ __noinline__ void arrive() {
         __syncthreads();
         if (threadIdx.x == 0 && *shAbort == 0) {
             target += gridDim.x;
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        }
+    }
+    __device__ __noinline__ bool wait() {
+        if (threadIdx.x == 0 && *shAbort == 0) {
             uint64_t t0 = 0;
             for (unsigned int polls = 1;; ++polls) {
                 unsigned int now;
@@ -277,6 +284,10 @@ struct GridTeam {
         }
         __syncthreads();
         return *shAbort == 0;
+    }
+    __device__ __forceinline__ bool sync() {
+        arrive();
+        return wait();
     }
     static constexpr unsigned int kPollsPerCheck = 256;
 
