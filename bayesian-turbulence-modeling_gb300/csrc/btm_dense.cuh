@@ -71,7 +71,7 @@ __device__ __noinline__ bool dense_inverse_small(T &tm, double *A, int n) {
 // matrix takes the kPanel updates of an element from registers in one pass:
 // two grid barriers and one pass over the matrix per 16 pivots instead of one
 // each per pivot, and half of the fused multiply-adds.  972 rows: 15.1 ms ->
-// 3.1 ms (FP64 issue alone: 1.6 ms).
+// 2.6 ms (FP64 issue alone: 1.6 ms).
 template <class T>
 __device__ __noinline__ bool dense_inverse_panels(T &tm, double *A, double *mult, double *prow, int n) {
     __shared__ double D[kPanel][kPanel];     // diagonal block as it evolves
