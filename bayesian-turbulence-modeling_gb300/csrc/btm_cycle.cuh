@@ -98,6 +98,7 @@ struct Cycle {
     // ---- one colour-ordered Gauss-Seidel sweep (colours ascending, or
     // descending).  `zero`: x is zero, and the first colour needs no x at all;
     // b may have been written in the pass before, so it waits for the barrier.
+    // Without `zero` b is older than the last barrier.
     __device__ __noinline__ static void gs(T &tm, const A &a, int l, bool reverse, bool zero) {
         const AmgLevelDev &L = a.lev(l);
         const RowTab R = a.rows();
@@ -380,6 +381,10 @@ struct Cycle {
                 x[i] = (V)s;
             }
         } else {
+            // the sweeps fetch b inside their first barrier, and the restriction
+            // (or the residual of a mesh without coarse levels) has just written
+            // it: a barrier of its own, once a cycle of kCoarseSweeps sweeps
+            tm.sync();
             for (int s = 0; s < kCoarseSweeps; ++s) gs(tm, a, l, (s & 1) != 0, false);
         }
     }
