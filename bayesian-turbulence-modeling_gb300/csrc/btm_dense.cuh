@@ -18,13 +18,14 @@ namespace btm {
 
 __device__ __forceinline__ bool bad_pivot(double piv) { return !(fabs(piv) > 1e-300); }
 
-// n <= 32 on one CTA, A [n][n] (shared or global).  The reciprocal of a pivot
-// (8-9 dependent FP64 instructions, 550 clocks) is the longest part of a step:
-// warp 0 forms the next pivot first and its reciprocal while the other warps
-// update the matrix.  Returns false, with A half done, at a vanishing pivot.
+// n <= kCoarseDirect on one CTA, A [n][n] (shared or global).  The reciprocal of
+// a pivot (8-9 dependent FP64 instructions, 550 clocks) is the longest part of a
+// step: warp 0 forms the next pivot first and its reciprocal while the other
+// warps update the matrix.  Returns false, with A half done, at a vanishing pivot.
 template <class T>
 __device__ __noinline__ bool dense_inverse_small(T &tm, double *A, int n) {
-    __shared__ double row[32], col[32], next;
+    static_assert(kCoarseDirect == 32, "a row to a warp");
+    __shared__ double row[kCoarseDirect], col[kCoarseDirect], next;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
     if (t == 0) next = A[0];
     __syncthreads();
@@ -182,7 +183,8 @@ __device__ __noinline__ bool dense_inverse_panels(T &tm, double *A, double *mult
 }
 
 // Inverse of the n x n matrix in A (filled by the caller, every thread past a
-// barrier); work [2 kPanel n] doubles.  False: a pivot vanished.
+// barrier); work [2 kPanel n] doubles; n <= kCoarseDirect on one CTA.  False: a
+// pivot vanished.
 template <class T>
 __device__ __forceinline__ bool dense_inverse(T &tm, double *A, double *work, int n) {
     if constexpr (std::is_same<T, GridTeam>::value) {

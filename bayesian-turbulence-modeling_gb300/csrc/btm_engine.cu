@@ -135,6 +135,11 @@ __device__ __noinline__ void amg_coarse_inverse(T &tm, const DevMesh &M, DevInst
     const AmgLevelDev &L = M.lev[l];
     double *A = I.ainv;
     const double *val = lev_vals(I, M, l);
+    // a large mesh's level on one CTA (the phase test hook)
+    if (!std::is_same<T, GridTeam>::value && n > kCoarseDirect) {
+        amg_coarse_inverse_sweep(tm, M, I);
+        return;
+    }
     for (int idx = tm.spread(); idx < n * n; idx += tm.size()) A[idx] = 0.0;
     tm.sync();
     for (int i = tm.spread(); i < n; i += tm.size()) {
