@@ -1025,6 +1025,14 @@ void fill_inst(btm_case *C, btm::DevInst &I, const double *coeffs, int variant, 
     I.normFixed = 0;
 }
 
+// A warm start must have the fields that the engine starts from; the closure
+// fields may be missing (the slab's own then stay).
+void check_warm(const btm_case *C, const btm_state *ws) {
+    if (!ws) throw BtmError(BTM_ERR_ARG, "warm init without a state");
+    if (!ws->U || !ws->p || !ws->k || !ws->omega || (C->nB > 0 && (!ws->Ub || !ws->pb || !ws->kb || !ws->omegab)))
+        throw BtmError(BTM_ERR_ARG, "warm state without U, p, k, omega or their boundary values");
+}
+
 // host staging for SoA <-> AoS conversion
 void upload_state(btm_case *C, const btm::DevInst &I, const btm_state *ws, cudaStream_t st,
                   std::vector<double> &stage) {
@@ -1107,8 +1115,12 @@ struct StageUpload {
     StageMem &M;
     cudaStream_t st;
     std::vector<btm::StageItem> items;
-    std::vector<const btm_state *> from;
-    std::vector<int64_t> where;      // first word of from[q]
+    struct Packed {
+        const btm_state *state;
+        int nC, nB;                  // the layout
+        int64_t at;                  // first word
+    };
+    std::vector<Packed> packed;
     int64_t words = 0;
     int maxCells = 0;
     bool inFlight = false;
@@ -1119,8 +1131,8 @@ struct StageUpload {
         if ((size_t)(need + 2 * itemWords) * 8 > kStageBytes) return false;
         ensure_first(batchWords);
         int64_t at = -1;
-        for (size_t q = from.size(); q-- > 0 && at < 0;)
-            if (from[q] == ws) at = where[q];
+        for (size_t q = packed.size(); q-- > 0 && at < 0;)
+            if (packed[q].state == ws && packed[q].nC == C->nC && packed[q].nB == C->nB) at = packed[q].at;
         const int64_t extra = at < 0 ? need : 0;
         if (items.size() == kStageItems || (size_t)(words + extra + (int64_t)(items.size() + 1) * itemWords) * 8 > M.bytes) {
             flush();
@@ -1128,8 +1140,7 @@ struct StageUpload {
         }
         if (at < 0) {
             at = words;
-            from.push_back(ws);
-            where.push_back(at);
+            packed.push_back({ws, C->nC, C->nB, at});
             words += need;
             double *o = (double *)M.pin + at;
             const size_t nC = C->nC, nB = C->nB;
@@ -1165,8 +1176,7 @@ struct StageUpload {
         // the pinned memory is written again by the next part, or by the results
         ck(cudaStreamSynchronize(st), "upload sync");
         items.clear();
-        from.clear();
-        where.clear();
+        packed.clear();
         words = 0;
         inFlight = true;
     }
@@ -1719,9 +1729,10 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
             } else {
                 if (ini && ini->mode != BTM_INIT_COLD && ini->mode != BTM_INIT_WARM)
                     throw BtmError(BTM_ERR_ARG, "unknown init mode");
+                const bool warm = ini && ini->mode == BTM_INIT_WARM;
+                if (warm) check_warm(J.C, ini->warm);
                 fill_inst(J.C, I, coeffs + 11 * (size_t)i, variants ? variants[i] : 0, ini);
-                if (ini && ini->mode == BTM_INIT_WARM) {
-                    if (!ini->warm) throw BtmError(BTM_ERR_ARG, "warm init without a state");
+                if (warm) {
                     if (!up.add(J.C, I, ini->warm, batchWords)) upload_state(J.C, I, ini->warm, st, stage);
                 }
             }
