@@ -23,7 +23,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 
 from . import _lib
-from ._lib import BtmHistory, BtmInit, Case, check, dptr, lib, new_states, state_struct
+from ._lib import STATE_ORDER, BtmHistory, BtmInit, Case, check, dptr, lib, new_states, state_struct
 from ._types import (EvaluationResult, EvaluationStatus, InferenceParameterSet, SolverSettings,
                      Vec3, _vec)
 
@@ -56,7 +56,11 @@ class SolveOutput:
         self.residuals = residuals
 
 
-def _init_struct(init, keep):
+def _init_struct(init, keep, shared=None):
+    """The BtmInit of one start; `keep` holds what it points to.  States of the same
+    arrays share one BtmState (`shared`, of one call), which the library then
+    moves to the device once.  The key is the arrays, kept alive here: a state
+    object may be made on access, or be filled anew for every instance."""
     ini = BtmInit()
     if isinstance(init, str):
         if init != "device":
@@ -67,8 +71,15 @@ def _init_struct(init, keep):
         init = {}
     if isinstance(init, dict) and "U" in init:
         ini.mode = 1
-        st = state_struct(init)
-        keep.append(st)
+        state = {f: init[f] for f in STATE_ORDER}
+        state["turb_established"] = int(init.get("turb_established", 0))
+        key = tuple(v if f == "turb_established" else id(v) for f, v in state.items())
+        st = None if shared is None else shared.get(key)
+        if st is None:
+            st = state_struct(state)
+            keep.append((state, st))
+            if shared is not None:
+                shared[key] = st
         ini.warm = C.pointer(st)
     else:
         u = _vec(init.get("u", (1.0, 0.0, 0.0)))
@@ -95,13 +106,17 @@ def solve_batch(cases: Sequence[Case], coeffs, variants=None, inits=None, want_s
     n = len(cases)
     coeffs = np.ascontiguousarray(np.asarray(coeffs, np.float64).reshape(n, 11))
     var = np.ascontiguousarray(np.zeros(n, np.int32) if variants is None else np.asarray(variants, np.int32))
-    keep, seen = [], {}
+    keep, shared = [], {}
     ini_arr = (BtmInit * n)()
+    last = made = None
+    plain = type(inits) in (list, tuple)
     for i in range(n):
         ini = None if inits is None else inits[i]
-        if id(ini) not in seen:   # instances that start alike share one struct
-            seen[id(ini)] = _init_struct(ini, keep)
-        ini_arr[i] = seen[id(ini)]
+        # a plain dict of a plain sequence once more: no code ran since that could
+        # have changed it (219 instances of one start: 0.6 ms less)
+        if made is None or not (plain and ini is last and type(ini) is dict):
+            last, made = ini, _init_struct(ini, keep, shared)
+        ini_arr[i] = made
     if want_state:
         states, st_arr = new_states(cases)
     else:
