@@ -136,17 +136,20 @@ __device__ __forceinline__ void gg_cell(const DevMesh &M, int c, const double *c
 // x / d, correctly rounded, from r = 1 / d correctly rounded: one
 // multiplication and two fused multiply-adds (P. Markstein, IBM J. Res. Dev. 34
 // (1990) 111; N. Brisebarre, J.-M. Muller, S. K. Raina, IEEE Trans. Comput. 53
-// (2004) 1069: exact when nothing over- or underflows on the way).  Exponents
-// outside 2^-620 .. 2^620 of x, d or r take the division itself.
-__device__ __forceinline__ bool mid_range(double v) {
-    return ((unsigned int)__double2hiint(v) & 0x7fffffffu) - 0x19300000u < 0x4d800000u;
+// (2004) 1069: exact when nothing over- or underflows on the way).  That is so
+// for x within 2^-620 .. 2^620 and d within 2^-300 .. 2^300: the quotient stays
+// within 2^-921 .. 2^921, and the remainder is a multiple of 2^-726.  Everything
+// else takes the division itself.
+template <int E>
+__device__ __forceinline__ bool within(double v) {   // |v| in 2^-E .. 2^E
+    return ((unsigned int)__double2hiint(v) & 0x7fffffffu) - ((1023u - E) << 20) < (2u * E) << 20;
 }
 __device__ __forceinline__ double div_by(double x, double d, double r) {
-    if (mid_range(x) && mid_range(d)) {
+    if (within<620>(x) && within<300>(d)) {
         const double q = x * r;
         return fma(fma(-q, d, x), r, q);
     }
-    if (x == 0.0 && mid_range(d)) return x * r;
+    if (x == 0.0 && within<300>(d)) return x * r;
     return x / d;
 }
 // smax(v, 0) and smax(-v, 0) without an FP64 comparison (the sign of zero aside)
