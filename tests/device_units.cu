@@ -3,6 +3,7 @@
 #include "../bayesian-turbulence-modeling_gb300/csrc/btm_common.h"
 #include "../bayesian-turbulence-modeling_gb300/csrc/btm_team.cuh"
 #include "../bayesian-turbulence-modeling_gb300/csrc/btm_phases64.cuh"
+#include "../bayesian-turbulence-modeling_gb300/csrc/btm_dense.cuh"
 
 #include <cuda_runtime.h>
 #include <vector>
@@ -12,6 +13,39 @@ using namespace btm;
 __global__ void k_div(const double *x, const double *d, const double *r, double *q, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) q[i] = div_by(x[i], d[i], r[i]);
+}
+
+// below[i][j] = residual_below(sq[i][j], limit(r0[i], tol[i]), ...): one warp per i
+__global__ void k_limit(const double *r0, const double *tol, const double *sq, int m, int *below, double *limit) {
+    const int i = blockIdx.x, lane = threadIdx.x;
+    const double l = residual_limit(r0[i], tol[i]);
+    if (lane == 0) limit[i] = l;
+    for (int j = lane; j < m; j += 32)
+        below[(size_t)i * m + j] = residual_below(sq[(size_t)i * m + j], l, r0[i], tol[i]);
+}
+
+constexpr int kThreads = 512;
+struct GridMem {
+    double *gpart;
+    unsigned int *bar;
+    int32_t *err;
+};
+__global__ void __launch_bounds__(kThreads, 1) k_inverse_grid(double *A, double *work, int n, GridMem g, int *ok) {
+    __shared__ double red[2 * 32 * kRedSlots];
+    __shared__ int shAbort;
+    if (threadIdx.x == 0) shAbort = 0;
+    __syncthreads();
+    GridTeam tm{red, 0, g.gpart, g.bar, g.err, &shAbort, 0u};
+    const bool good = dense_inverse(tm, A, work, n);
+    if (threadIdx.x == 0) ok[blockIdx.x] = good;
+}
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_inverse_block(double *A, int n, int *ok) {
+    __shared__ double red[NT > 2 * 32 * kRedSlots ? NT : 2 * 32 * kRedSlots];
+    __shared__ double tot[2 * (NT / 32) + kRedResults];
+    BlockTeam tm{red, 0, tot, 0, live_warps(n)};
+    const bool good = dense_inverse(tm, A, nullptr, n);
+    if (threadIdx.x == 0) ok[0] = good;
 }
 
 namespace {
@@ -52,6 +86,47 @@ int unit_div_by(int n, const double *x, const double *d, const double *r, double
     M.launched();
     M.back(q, dq, n);
     return (int)M.e;
+}
+
+int unit_residual_limit(int n, int m, const double *r0, const double *tol, const double *sq, int *below,
+                        double *limit) {
+    Mem M;
+    double *dr = M.get(n, r0), *dt = M.get(n, tol), *ds = M.get((size_t)n * m, sq), *dl = M.get<double>(n);
+    int *db = M.get<int>((size_t)n * m);
+    if (M.e != cudaSuccess) return (int)M.e;
+    k_limit<<<n, 32>>>(dr, dt, ds, m, db, dl);
+    M.launched();
+    M.back(below, db, (size_t)n * m);
+    M.back(limit, dl, n);
+    return (int)M.e;
+}
+
+// A [n][n] to its inverse, in place.  blocks > 0: on a cooperative grid of that
+// many CTAs (all co-resident: one to an SM); 0: on one CTA of `threads`.
+// ok: the outcome of every CTA.
+int unit_dense_inverse(int blocks, int threads, int n, double *A, int *ok) {
+    Mem M;
+    double *dA = M.get((size_t)n * n, A), *work = M.get<double>((size_t)2 * kPanel * n);
+    int *dOk = M.get<int>(blocks > 0 ? blocks : 1);
+    GridMem g{M.get<double>((size_t)2 * (blocks > 0 ? blocks : 1) * kRedSlots), M.get<unsigned int>(1),
+              M.get<int32_t>(1)};
+    if (M.e != cudaSuccess) return (int)M.e;
+    if (blocks > 0) {
+        void *args[] = {&dA, &work, &n, &g, &dOk};
+        M.e = cudaLaunchCooperativeKernel((const void *)k_inverse_grid, dim3(blocks), dim3(kThreads), args, 0, 0);
+    } else if (n > kCoarseDirect) {
+        return -1;
+    } else if (threads == 256) {
+        k_inverse_block<256><<<1, 256>>>(dA, n, dOk);
+    } else {
+        k_inverse_block<512><<<1, 512>>>(dA, n, dOk);
+    }
+    M.launched();
+    M.back(A, dA, (size_t)n * n);
+    M.back(ok, dOk, blocks > 0 ? blocks : 1);
+    int32_t err = 0;
+    M.back(&err, g.err, 1);
+    return M.e != cudaSuccess ? (int)M.e : err ? -2 : 0;
 }
 
 }  // extern "C"
