@@ -1858,7 +1858,9 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
                 Job &J = jobs[i1];
                 btm::StageItem S = stage_item(J.C, J.S->inst);
                 const bool wantObs = J.S->inst.obsOut && hists && hists[i1].predictions;
+                // observation outputs or a state that do not fit are fetched below
                 S.nObs = wantObs ? J.C->dmesh.obs.n + 1 : 0;
+                if (8 * (btm::kStageHead + (size_t)S.nObs + itemWords) > kStageBytes) S.nObs = 0;
                 const size_t head = btm::kStageHead + S.nObs, state = btm::stage_state_words(S.nC, S.nB);
                 S.state = outs && 8 * (head + state + itemWords) <= kStageBytes;
                 const size_t need = head + (S.state ? state : 0);
@@ -1913,6 +1915,8 @@ int btm_solve_batch(int32_t n, btm_case *const *cases, const double *coeffs, con
                         const double *o = w + btm::kStageHead;
                         for (int k = 0; k + 1 < S.nObs; ++k) h.predictions[k] = o[k];
                         h.log_lik = o[S.nObs - 1];
+                    } else {
+                        download_obs(J.C, I, &h, st);
                     }
                 }
                 if (outs) {
