@@ -1622,7 +1622,6 @@ int btm_case_set_observations(btm_case *C, const btm_mesh *m, int32_t n, const b
             throw BtmError(BTM_ERR_CUDA, cudaGetErrorString(e));
         }
         if (C->obsArena) cudaFree(C->obsArena);
-    if (C->injTarget) cudaFree(C->injTarget);
         C->obsArena = arena;
         C->dmesh = D;
     } catch (const BtmError &e) {
