@@ -19,13 +19,18 @@ def _d(a):
     return a.ctypes.data_as(_dp)
 
 
+_built = []   # once per process: test_gpu_vcycle.py uses it too
+
+
 @pytest.fixture(scope="module")
 def units(tmp_path_factory):
-    so = str(tmp_path_factory.mktemp("units") / "device_units.so")
-    subprocess.run([_build.nvcc()] + _build.ARCH + ["-O3", "-std=c++17", "-fmad=false", "-shared", "-Xcompiler", "-fPIC",
-                                                    "-I", _build.INCLUDE, cases.HERE + "/device_units.cu", "-o", so,
-                                                    "-cudart", "static"], check=True)
-    return C.CDLL(so)
+    if not _built:
+        so = str(tmp_path_factory.mktemp("units") / "device_units.so")
+        subprocess.run([_build.nvcc()] + _build.ARCH + ["-O3", "-std=c++17", "-fmad=false", "-shared", "-Xcompiler",
+                                                        "-fPIC", "-I", _build.INCLUDE, cases.HERE + "/device_units.cu",
+                                                        "-o", so, "-cudart", "static"], check=True)
+        _built.append(C.CDLL(so))
+    return _built[0]
 
 
 def _same(a, b):
