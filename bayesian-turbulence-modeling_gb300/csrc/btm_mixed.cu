@@ -634,12 +634,13 @@ __device__ void mx_amg_level_rd(T &tm, const DevMesh &M, DevWork32 &F, int l) {
     }
 }
 
-// Dense inverse of the coarsest level in FP64: the coarsest Galerkin matrix of a pinned pure-Neumann pressure system
-// is nearly singular (its condition grows with the mesh), and an FP32 inverse
-// of it wrecked the preconditioner on a 2M-cell duct (39 PCG iterations per
-// solve instead of about one).  At most 32 rows, refreshed every
-// kAmgRefresh outer iterations.  The sweep with ping-pong buffers is for a
-// matrix with a vanishing pivot, whose rows are passed over.
+// Dense inverse of the coarsest level in FP64: the coarsest Galerkin matrix of a
+// pinned pure-Neumann pressure system is nearly singular (its condition grows
+// with the mesh), and an FP32 inverse of it wrecked the preconditioner on a
+// 2M-cell duct (39 PCG iterations per solve instead of about one).  At most 32
+// rows on one CTA and kCoarseDirectGrid on the grid, refreshed every kAmgRefresh
+// outer iterations.  The sweep with ping-pong buffers is for a matrix with a
+// vanishing pivot, whose rows are passed over.
 template <class T>
 __device__ __noinline__ void mx_amg_coarse_inverse_sweep(T &tm, const DevMesh &M, DevWork32 &F) {
     const int l = M.nLevels - 1;

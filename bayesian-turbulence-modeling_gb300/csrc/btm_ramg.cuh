@@ -161,7 +161,7 @@ struct RGroup {
 // registers of warp 0 for all its sweeps.  The entries of a row past the
 // eighth, and rows past the CTA's size, are read in place.
 constexpr int kRowRegs = 8;
-constexpr int kRec = 10, kRec0 = 6;   // doubles per record: values, columns (level 0: and 1/diag), by 16-byte parts
+constexpr int kRec = 10;   // doubles per record of a coarse level: 8 values, 8 columns, by 16-byte parts
 // x of a level, in shared memory (addresses of 32 bits) or global memory
 template <bool SM> struct RX;
 template <> struct RX<true> {
@@ -522,12 +522,14 @@ __device__ int ramg_wavefronts(T &tm, const RamgWork &W, const int32_t *ptr, con
 
 // Packs the rows of every level as records in wavefront order (the coarsest
 // level first: its 50 sweeps are the longest chain).  Nothing is allocated for
-// them: the coarse levels take the place of the other AMG form's arrays, which
+// them.  The coarse levels take the place of the other AMG form's arrays, which
 // an instance with this one does not use (amgVal up to gpart is one stretch of
-// the slab), with their 1/diag in that of the Galerkin contributions, level 0 of a mesh of quadrilaterals that of the velocity
-// gradients, which the pressure correction leaves free (formed anew at the
-// start of every outer iteration; `vel`: they are still needed).  A level that
-// does not fit, or has more than 32 wavefronts, is swept from its CSR rows.
+// the slab), with their 1/diag in that of the Galerkin contributions.  Level 0 of
+// a mesh of quadrilaterals (records of 6 doubles: 4 values, 4 columns, 1/diag)
+// takes that of the velocity gradients, which the pressure correction leaves free
+// (formed anew at the start of every outer iteration; `vel`: they are still
+// needed).  A level that does not fit, or has more than 32 wavefronts, is swept
+// from its CSR rows.
 template <class T>
 __device__ void ramg_pack(T &tm, const DevMesh &M, DevInst &I, int nLev, bool vel) {
     const RamgWork &W = I.rg;
