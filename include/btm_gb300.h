@@ -208,7 +208,10 @@ typedef struct btm_init {
 
 /* Full flow state: FlowFields (core/include/FlowFields.hpp:9-33).  Cell arrays
  * have n_cells entries (U: n_cells*3), boundary arrays n_faces-n_internal
- * entries (Ub: *3).  Any pointer may be NULL on output to skip that field. */
+ * entries (Ub: *3).  Any pointer may be NULL on output to skip that field.  A
+ * warm start of btm_solve / btm_solve_batch needs U, p, k, omega and, where the
+ * mesh has boundary faces, Ub, pb, kb and omegab (BTM_ERR_ARG without them); the
+ * closure fields nuT, F1, F2, Pk and CDkw may be NULL. */
 struct btm_state {
     double *U, *p, *k, *omega, *nuT, *F1, *F2, *Pk, *CDkw;
     double *Ub, *pb, *kb, *omegab;
